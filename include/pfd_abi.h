@@ -200,11 +200,12 @@ pfd_status pfd_pm_sweep(pfd_ctx* ctx, int frame_id, const pfd_pm_params* params,
  * For callers that cannot allocate device memory once frames are streaming: an
  * application whose memory pool claimed all free HBM at start-up, or a
  * real-time loop that forbids cudaMalloc/cudaFree because they can synchronise
- * the whole device.  The cost-vector scratch is a fixed 8 MiB array in the
+ * the whole device.  The sweep itself needs no scratch; under tap counting or
+ * texture fetches its cost-vector scratch is a fixed 8 MiB array in the
  * library's device image (held by every GPU that loads the library, until
- * exit) instead of a cudaMalloc'd buffer; inputs and outputs are the frame's
+ * exit) instead of a cudaMalloc'd buffer.  Inputs and outputs are the frame's
  * state exactly as for pfd_pm_sweep, and the results are the same bit for bit.
- * Limit: the array must hold one CTA's scratch (seven warps, each the cost
+ * Limit (tap counting, texture fetches): the array must hold one CTA's scratch (seven warps, each the cost
  * vectors of one pixel) for every SM: every max_nb up to 32 fits on a 148-SM
  * B200; a device with more SMs than the array holds CTAs gets PFD_EINVAL.
  * Every call looks up the array's device address (cudaGetSymbolAddress, a
@@ -255,7 +256,8 @@ pfd_status pfd_set_matcher(pfd_ctx* ctx, int matcher);
  * pfd_patchmatch_batch; no counterpart in the reference, whose sweep is one
  * thread per pixel in 16x16 blocks).  A shape is a number of warps per CTA and
  * the CTAs per SM its registers are sized for; every shape computes the same
- * state bit for bit.  Shape 0 (7 warps, 4 CTAs) is the default.
+ * state bit for bit.  Shape 0 (16 warps, 2 CTAs) is the default.  Texture fetches
+ * and tap counting have one shape of their own.
  * PFD_SHAPE_AUTOTUNE: the engine's autotuner picks the shape per key (window,
  * neighbour count, patch size and tap stride, blur channel, moment mode,
  * matcher) and device: the first half-sweep of a new key runs once in every
@@ -263,7 +265,7 @@ pfd_status pfd_set_matcher(pfd_ctx* ctx, int matcher);
  * (the stored cost vectors are neither read nor written by these trials, so
  * each writes the half-sweep's result), and the fastest is kept for the rest
  * of the process.  pfd_patchmatch_batch uses the shape of each launch's
- * largest frame.  Tap counting and pfd_pm_sweep_noalloc always run shape 0. */
+ * largest frame.  pfd_pm_sweep_noalloc always runs shape 0. */
 #define PFD_SWEEP_SHAPES 4
 #define PFD_SHAPE_AUTOTUNE -1
 pfd_status pfd_set_sweep_shape(pfd_ctx* ctx, int shape);

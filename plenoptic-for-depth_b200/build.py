@@ -24,7 +24,7 @@ NVCC_FLAGS = [
     "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC,-O2,-ffp-contract=off", "-ccbin", "/usr/bin/g++",
 ]
 
-CU_SOURCES = ["pm_kernels.cu", "pm_sweep.cu", "check_kernels.cu", "refocus_kernels.cu", "vdrd_kernels.cu", "fuse_kernels.cu", "mla_kernels.cu", "select_kernels.cu", "blur_kernels.cu", "pfd_abi.cu"]
+CU_SOURCES = ["pm_kernels.cu", "pm_slots.cu", "pm_sweep.cu", "check_kernels.cu", "refocus_kernels.cu", "vdrd_kernels.cu", "fuse_kernels.cu", "mla_kernels.cu", "select_kernels.cu", "blur_kernels.cu", "pfd_abi.cu"]
 CPP_SOURCES = ["neighbors.cpp", "server.cpp", "calib_xml.cpp"]
 SYNTH_LIB = os.path.join(OUT, "libpfd_synth.so")
 HOST_DIR = os.path.join(PKG_DIR, "host")
@@ -80,7 +80,7 @@ def build_lib(force: bool = False, verbose: bool = False) -> str:
     # the translation units are independent: compile them side by side, the
     # largest (the sweep's kernel variants) first
     with concurrent.futures.ThreadPoolExecutor(max_workers=max(1, min(8, os.cpu_count() or 1))) as ex:
-        for f in [ex.submit(_run, c) for c in sorted(cmds, key=lambda c: "pm_sweep" not in c[-3])]:
+        for f in [ex.submit(_run, c) for c in sorted(cmds, key=lambda c: "pm_slots" not in c[-3])]:
             f.result()
     tmp = LIB + ".tmp"
     _run([NVCC, *ARCH, "-shared", "-Xlinker", "-soname=libpfd.so", "-o", tmp, *objs, "-ccbin", "/usr/bin/g++"])

@@ -991,21 +991,17 @@ static pfd_status tune_shape(pfd_ctx* ctx, Frame& f, pfd::PmParams P, int iter, 
     pfd_status st = PFD_OK;
     const pfd::FrameDev F = sweep_dev(ctx, f);
     for (int shape = 0; shape < pfd::kSweepShapes && st == PFD_OK; ++shape) {
-        if (pfd::sweep_warp_smem_bytes(P, f.has_blur, shape, F.tex != nullptr) > 227 * 1024) continue;
         int n_ctas = 0;
-        if (pfd::sweep_warp_grid(F, P, &n_ctas, shape) != cudaSuccess) {
+        const int smem = pfd::slots_plan(P, f.has_blur, shape, f.V);
+        if (!smem) continue;
+        if (pfd::slots_sweep_grid(F, P, smem, &n_ctas, shape) != cudaSuccess) {
             cudaGetLastError();                      // this shape does not fit the plan: not a candidate
             continue;
         }
-        st = ensure_scratch(ctx, pfd::sweep_warp_scratch_bytes(P, n_ctas, shape));
-        if (st != PFD_OK) break;
-        pfd::PmParams Q = P;
-        Q.cost_scratch = ctx->d_scratch;
-        Q.scratch_floats = ctx->scratch_bytes / sizeof(float);
         cudaError_t e = cudaEventRecord(a, ctx->stream);
         if (e == cudaSuccess)
-            e = pfd::launch_sweep_warp(F, Q, f.s[f.cur], f.s[f.cur ^ 1], iter, phase, n_ctas, ctx->d_err,
-                                       ctx->stream, shape);
+            e = pfd::launch_slots_sweep(F, P, f.s[f.cur], f.s[f.cur ^ 1], iter, phase, smem, n_ctas, ctx->d_err,
+                                        ctx->stream, shape);
         if (e == cudaSuccess) e = cudaEventRecord(b, ctx->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(b);
         float ms = 0.0f;
@@ -1033,7 +1029,7 @@ static pfd_status tune_shape(pfd_ctx* ctx, Frame& f, pfd::PmParams P, int iter, 
 
 // The shape the context's next half-sweep of frame f runs: the fixed one, or
 // under PFD_SHAPE_AUTOTUNE the tuned one (tuning on this half-sweep when the
-// key is new).  Tap counting runs shape 0.
+// key is new).  Tap counting and texture fetches have one shape.
 static pfd_status sweep_shape_for(pfd_ctx* ctx, Frame& f, const pfd::PmParams& P, int iter, int phase, int* shape)
 {
     *shape = 0;
@@ -1042,9 +1038,15 @@ static pfd_status sweep_shape_for(pfd_ctx* ctx, Frame& f, const pfd::PmParams& P
         *shape = ctx->sweep_shape;
         return PFD_OK;
     }
-    const int c = cached_shape(shape_key(ctx, f, P));
+    const ShapeKey key = shape_key(ctx, f, P);
+    const int c = cached_shape(key);
     if (c >= 0) {
         *shape = c;
+        return PFD_OK;
+    }
+    if (key.tex) {
+        std::lock_guard<std::mutex> lock(g_shape_mu);
+        g_shape_cache[key] = 0;
         return PFD_OK;
     }
     return tune_shape(ctx, f, P, iter, phase, shape);
@@ -1061,11 +1063,10 @@ pfd_status pfd_set_sweep_shape(pfd_ctx* ctx, int shape)
 
 pfd_status pfd_sweep_shape_info(int shape, int* warps_per_cta, int* ctas_per_sm)
 {
-    static const int kMin[PFD_SWEEP_SHAPES] = { 4, 3, 6, 2 };
     static_assert(PFD_SWEEP_SHAPES == pfd::kSweepShapes, "shape tables");
     if (shape < 0 || shape >= PFD_SWEEP_SHAPES) return PFD_EINVAL;
-    if (warps_per_cta) *warps_per_cta = pfd::sweep_shape_warps(shape);
-    if (ctas_per_sm) *ctas_per_sm = kMin[shape];
+    if (warps_per_cta) *warps_per_cta = pfd::slots_shape_warps(shape);
+    if (ctas_per_sm) *ctas_per_sm = pfd::slots_shape_ctas(shape);
     return PFD_OK;
 }
 
@@ -1077,6 +1078,31 @@ pfd_status pfd_tuned_sweep_shape(pfd_ctx* ctx, int frame_id, const pfd_pm_params
     const pfd_status st = check_params(ctx, *f, params);
     if (st != PFD_OK) return st;
     *shape = cached_shape(shape_key(ctx, *f, make_params(ctx, *f, params, 0)));
+    return PFD_OK;
+}
+
+// Tap counting and texture fetches run the warp-per-pixel kernel.
+static bool uses_warp_sweep(const pfd::FrameDev& F, const pfd::PmParams& P) { return F.tex != nullptr || P.tap_counter; }
+
+static pfd_status check_sweep_fits(pfd_ctx* ctx, const Frame& f, const pfd::PmParams& P, const pfd::FrameDev& F)
+{
+    if (pfd::sweep_warp_smem_bytes(P, f.has_blur, F.tex != nullptr) > 227 * 1024)
+        return fail(ctx, PFD_EINVAL, "window %dx%d with %d neighbours does not fit shared memory", f.mi_w, f.mi_h, f.K);
+    return PFD_OK;
+}
+
+// Enqueues one half-sweep of the slot kernel, from the frame's current state into
+// its other buffer.
+static pfd_status slots_sweep(pfd_ctx* ctx, Frame& f, pfd::PmParams& P, const pfd::FrameDev& F, int iter, int phase,
+                              int shape)
+{
+    const int smem = pfd::slots_plan(P, f.has_blur, shape, f.V);
+    if (!smem)
+        return fail(ctx, PFD_EINVAL, "window %dx%d with %d neighbours does not fit shared memory", f.mi_w, f.mi_h, f.K);
+    int n_ctas = 0;
+    CU(pfd::slots_sweep_grid(F, P, smem, &n_ctas, shape));
+    CU(pfd::launch_slots_sweep(F, P, f.s[f.cur], f.s[f.cur ^ 1], iter, phase, smem, n_ctas, ctx->d_err, ctx->stream,
+                               shape));
     return PFD_OK;
 }
 
@@ -1096,20 +1122,23 @@ pfd_status pfd_pm_sweep(pfd_ctx* ctx, int frame_id, const pfd_pm_params* params,
     st = tex_refresh(ctx, *f);
     if (st != PFD_OK) return st;
     const pfd::FrameDev F = sweep_dev(ctx, *f);
-    if (pfd::sweep_warp_smem_bytes(P, f->has_blur, 0, F.tex != nullptr) > 227 * 1024)
-        return fail(ctx, PFD_EINVAL, "window %dx%d with %d neighbours does not fit shared memory", f->mi_w, f->mi_h, f->K);
-    int shape = 0;
-    st = sweep_shape_for(ctx, *f, P, iter, phase, &shape);
-    if (st != PFD_OK) return st;
-    int n_ctas = 0;
-    CU(pfd::sweep_warp_grid(F, P, &n_ctas, shape));
-    st = ensure_scratch(ctx, pfd::sweep_warp_scratch_bytes(P, n_ctas, shape));
-    if (st != PFD_OK) return st;
-    P.cost_scratch = ctx->d_scratch;
-    P.scratch_floats = ctx->scratch_bytes / sizeof(float);
+    if ((st = check_sweep_fits(ctx, *f, P, F)) != PFD_OK) return st;
     P.cvec_ok = !ctx->counting && cvec_usable(*f, *params, phase, cost_mode(ctx));
-    CU(pfd::launch_sweep_warp(F, P, f->s[f->cur], f->s[f->cur ^ 1], iter, phase, n_ctas, ctx->d_err,
-                              ctx->stream, shape));
+    int n_ctas = 0;
+    if (uses_warp_sweep(F, P)) {
+        CU(pfd::sweep_warp_grid(F, P, &n_ctas));
+        st = ensure_scratch(ctx, pfd::sweep_warp_scratch_bytes(P, n_ctas));
+        if (st != PFD_OK) return st;
+        P.cost_scratch = ctx->d_scratch;
+        P.scratch_floats = ctx->scratch_bytes / sizeof(float);
+        CU(pfd::launch_sweep_warp(F, P, f->s[f->cur], f->s[f->cur ^ 1], iter, phase, n_ctas, ctx->d_err, ctx->stream));
+    } else {
+        int shape = 0;
+        st = sweep_shape_for(ctx, *f, P, iter, phase, &shape);
+        if (st != PFD_OK) return st;
+        st = slots_sweep(ctx, *f, P, F, iter, phase, shape);
+        if (st != PFD_OK) return st;
+    }
     ctx->launches += 1;
     f->cur ^= 1;
     if (ctx->counting) f->cvec_valid = 0;        // tap counting evaluates everything and stores nothing
@@ -1234,8 +1263,11 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
         std::vector<int> solo, rest;
         for (int b = 0; b < n; ++b) {
             int n_ctas = 0;
-            const pfd::PmParams P = make_params(ctx, *fr[b], &params[b], seeds[b]);
-            if (pfd::sweep_warp_grid(sweep_dev(ctx, *fr[b]), P, &n_ctas, 0) != cudaSuccess) {
+            pfd::PmParams P = make_params(ctx, *fr[b], &params[b], seeds[b]);
+            const pfd::FrameDev F = sweep_dev(ctx, *fr[b]);
+            const int smem = pfd::slots_plan(P, fr[b]->has_blur, 0, fr[b]->V);
+            if ((F.tex ? pfd::sweep_warp_grid(F, P, &n_ctas)
+                       : (smem ? pfd::slots_sweep_grid(F, P, smem, &n_ctas, 0) : cudaSuccess)) != cudaSuccess) {
                 cudaGetLastError();
                 n_ctas = 0;
             }
@@ -1269,7 +1301,7 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
     int half_sweeps = 0;
     for (int b = 0; b < n; ++b) {
         const pfd::PmParams P = make_params(ctx, *fr[b], &params[b], seeds[b]);
-        if (pfd::sweep_warp_smem_bytes(P, fr[b]->has_blur, 0, sweep_dev(ctx, *fr[b]).tex != nullptr) > 227 * 1024)
+        if (pfd::sweep_warp_smem_bytes(P, fr[b]->has_blur, sweep_dev(ctx, *fr[b]).tex != nullptr) > 227 * 1024)
             return fail(ctx, PFD_EINVAL, "frame %d: window %dx%d with %d neighbours does not fit shared memory",
                         frame_ids[b], fr[b]->mi_w, fr[b]->mi_h, fr[b]->K);
         half_sweeps = std::max(half_sweeps, 2 * params[b].max_iterations);
@@ -1285,11 +1317,11 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
         const pfd::PmParams Pb = make_params(ctx, *fr[big], &params[big], seeds[big]);
         const pfd_status st = sweep_shape_for(ctx, *fr[big], Pb, 0, 0, &shape_of_blur[grp]);
         if (st != PFD_OK) return st;
-        for (int b = 0; b < n; ++b)          // a shape every frame of the group fits, or the default
-            if ((fr[b]->has_blur ? 1 : 0) == grp &&
-                pfd::sweep_warp_smem_bytes(make_params(ctx, *fr[b], &params[b], seeds[b]), grp == 1,
-                                           shape_of_blur[grp], sweep_dev(ctx, *fr[b]).tex != nullptr) > 227 * 1024)
+        for (int b = 0; b < n; ++b) {        // a shape every frame of the group fits, or the default
+            pfd::PmParams Q = make_params(ctx, *fr[b], &params[b], seeds[b]);
+            if ((fr[b]->has_blur ? 1 : 0) == grp && !pfd::slots_plan(Q, grp == 1, shape_of_blur[grp], fr[b]->V))
                 shape_of_blur[grp] = 0;
+        }
     }
     // launch groups: frames with the same blur channel and fetch whose own
     // shared-memory plans allow the same CTAs per SM share a launch, so no frame
@@ -1300,10 +1332,14 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
     for (int b = 0; b < n; ++b) {
         const int blur = fr[b]->has_blur ? 1 : 0, shape = shape_of_blur[blur];
         const int tex = sweep_dev(ctx, *fr[b]).tex != nullptr ? 1 : 0;
-        const int sm = pfd::sweep_warp_smem_bytes(make_params(ctx, *fr[b], &params[b], seeds[b]), blur == 1, shape,
-                                                  tex == 1);
+        pfd::PmParams Q = make_params(ctx, *fr[b], &params[b], seeds[b]);
+        const int sm = tex ? pfd::sweep_warp_smem_bytes(Q, blur == 1, true) : pfd::slots_plan(Q, blur == 1, shape, fr[b]->V);
+        if (!sm)
+            return fail(ctx, PFD_EINVAL, "frame %d: window %dx%d with %d neighbours does not fit shared memory",
+                        frame_ids[b], fr[b]->mi_w, fr[b]->mi_h, fr[b]->K);
         int ctas = 0;
-        CU(pfd::sweep_batch_grid(sm, blur == 1, shift, tex == 1, &ctas, shape));
+        if (tex) CU(pfd::sweep_batch_grid(sm, blur == 1, shift, &ctas));
+        else CU(pfd::slots_batch_grid(sm, blur == 1, shift, &ctas, shape));
         int g = -1;
         for (size_t k = 0; k < groups.size(); ++k)
             if (groups[k].blur == blur && groups[k].tex == tex && groups[k].ctas == ctas) g = (int)k;
@@ -1323,7 +1359,7 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
     for (const Group& g : groups) {
         pfd::PmParams Pk = {};
         Pk.K = k_max;                                  // the scratch of the group's CTAs at that stride
-        scratch = std::max(scratch, pfd::sweep_warp_scratch_bytes(Pk, g.ctas, g.shape));
+        if (g.tex) scratch = std::max(scratch, pfd::sweep_warp_scratch_bytes(Pk, g.ctas));
     }
     pfd_status st = ensure_scratch(ctx, scratch);
     if (st != PFD_OK) return st;
@@ -1356,6 +1392,7 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
                 it.P.cost_scratch = ctx->d_scratch;
                 it.P.scratch_floats = ctx->scratch_bytes / sizeof(float);
                 it.P.scratch_stride = stride;
+                if (!groups[grp].tex) pfd::slots_plan(it.P, groups[grp].blur == 1, groups[grp].shape, f.V);
                 it.P.cvec_ok = cvec_usable(f, params[b], phase, mode);
                 it.P.view_queue = d_queues + (size_t)s * n + items.size();
                 it.prev = f.s[f.cur];
@@ -1377,8 +1414,10 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
         for (size_t grp = 0; grp < groups.size(); off += count[grp], ++grp) {
             if (!count[grp]) continue;
             const Group& G = groups[grp];
-            const cudaError_t e = pfd::launch_sweep_batch(row + off, count[grp], G.blur == 1, shift, G.tex == 1, G.smem,
-                                                          G.ctas, ctx->d_err, ctx->stream, G.shape);
+            const cudaError_t e = G.tex ? pfd::launch_sweep_batch(row + off, count[grp], G.blur == 1, shift, G.smem, G.ctas,
+                                                                  ctx->d_err, ctx->stream)
+                                        : pfd::launch_slots_batch(row + off, count[grp], G.blur == 1, shift, G.smem,
+                                                                  G.ctas, ctx->d_err, ctx->stream, G.shape);
             if (e != cudaSuccess) {
                 st = fail(ctx, PFD_ECUDA, "launch_sweep_batch: %s", cudaGetErrorString(e));
                 break;
@@ -2646,8 +2685,16 @@ extern "C" pfd_status pfd_pm_sweep_noalloc(pfd_ctx* ctx, int frame_id, const pfd
     st = tex_refresh(ctx, *f, false);            // a launch, no allocation (textures only if the frame has them)
     if (st != PFD_OK) return st;
     const pfd::FrameDev F = sweep_dev(ctx, *f);
-    if (pfd::sweep_warp_smem_bytes(P, f->has_blur, 0, F.tex != nullptr) > 227 * 1024)
-        return fail(ctx, PFD_EINVAL, "window %dx%d with %d neighbours does not fit shared memory", f->mi_w, f->mi_h, f->K);
+    if ((st = check_sweep_fits(ctx, *f, P, F)) != PFD_OK) return st;
+    P.cvec_ok = !ctx->counting && cvec_usable(*f, *params, phase, cost_mode(ctx));
+    if (!uses_warp_sweep(F, P)) {                // the slot kernel needs no scratch
+        st = slots_sweep(ctx, *f, P, F, iter, phase, 0);
+        if (st != PFD_OK) return st;
+        ctx->launches += 1;
+        f->cur ^= 1;
+        cvec_swept(*f, *params, phase, cost_mode(ctx));
+        return PFD_OK;
+    }
     int sms = 0;
     CU(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
     const size_t per_cta = pfd::sweep_warp_scratch_bytes(P, 1);
@@ -2672,7 +2719,6 @@ extern "C" pfd_status pfd_pm_sweep_noalloc(pfd_ctx* ctx, int frame_id, const pfd
     if (st != PFD_OK) return st;
     P.cost_scratch = scratch;
     P.scratch_floats = kNoAllocScratchBytes / sizeof(float);
-    P.cvec_ok = !ctx->counting && cvec_usable(*f, *params, phase, cost_mode(ctx));
     CU(pfd::launch_sweep_warp(F, P, f->s[f->cur], f->s[f->cur ^ 1], iter, phase, n_ctas, ctx->d_err,
                               ctx->stream));
     ctx->launches += 1;

@@ -38,6 +38,7 @@ struct PmParams {
     int shifted;            // 0: the reference's raw NCC moments; 1: moments of (pixel - centre pixel)
     int* view_queue;        // sweep: micro-images are handed out in order from this counter (zeroed per launch)
     float blur_gain;        // blur penalty gain: 2 (Frame matcher), 0.8 (ACMM matcher)
+    int slots, task_cap, parts;   // slot sweep: pixels in flight per CTA, NCC list entries, items per micro-image
     int acmm;               // 1: ACMM write-back (top-k cost, views and disp of the final plane)
 };
 
@@ -135,7 +136,8 @@ __device__ __forceinline__ float4 geo_disp(const NbGeo& g, int px, int py, float
 
 // GenerateRandomNormal_MIPM (AdaptMIPMUtil.cu:463-492); the rejection loop is
 // bounded at 64 pairs (probability of reaching it ~1e-43), then +z.
-__device__ __forceinline__ float4 random_normal(DrawStream& g)
+template <class Draws>
+__device__ __forceinline__ float4 random_normal(Draws& g)
 {
     float q1 = 1.0f, q2 = 1.0f, s = 2.0f;
     int attempts = 0;
@@ -152,7 +154,8 @@ __device__ __forceinline__ float4 random_normal(DrawStream& g)
 }
 
 // GenerateRandomPlaneHypothesis_MIPM (AdaptMIPMUtil.cu:494-501)
-__device__ __forceinline__ float4 random_plane(DrawStream& g, float dmin, float dmax)
+template <class Draws>
+__device__ __forceinline__ float4 random_plane(Draws& g, float dmin, float dmax)
 {
     const float depth = __fmaf_rn(g.uniform(), __fsub_rn(dmax, dmin), dmin);
     float4 h = random_normal(g);

@@ -19,35 +19,46 @@ cudaError_t launch_init(const FrameDev& F, const PmParams& P, const StateDev& ou
 cudaError_t launch_ncc(const FrameDev& F, const PmParams& P, int nseg, int npb, const int* seg_vid,
                        const int* seg_start, const int* seg_len, const int* hyp_pxy, const float4* hyp_plane,
                        const int* hyp_out, float* costs, int* err, cudaStream_t st);
-// The warp-per-pixel sweep (pm_sweep.cu): grid, shared memory, and the global
-// scratch it needs (P.cost_scratch: per warp, the cost vectors of one pixel).
-// shape selects one of kSweepShapes launch shapes (warps per CTA and CTAs per
-// SM the registers are sized for); every shape computes the same result bit
-// for bit.  Shape 0 is the default; tap counting always runs shape 0.
+// The half-sweep (pm_slots.cu).  shape selects one of kSweepShapes launch shapes
+// (warps per CTA and CTAs per SM); every shape computes the same result bit for
+// bit.  Shape 0 is the default.
 constexpr int kSweepShapes = 4;
-int sweep_shape_warps(int shape);
-// The sweep fetches neighbour samples from F.tex when the frame has textures
-// (tap counting excepted), else from shared-memory quads; tex selects the plan.
-cudaError_t sweep_warp_grid(const FrameDev& F, const PmParams& P, int* n_ctas, int shape = 0);
-int sweep_warp_smem_bytes(const PmParams& P, bool blur, int shape, bool tex);
-size_t sweep_warp_scratch_bytes(const PmParams& P, int n_ctas, int shape = 0);
-// Floats of global scratch one warp uses for K neighbours (PmParams::scratch_stride).
-int sweep_warp_stride(int K);
-cudaError_t launch_sweep_warp(const FrameDev& F, const PmParams& P, const StateDev& prev, const StateDev& next,
-                              int iter, int phase, int n_ctas, int* err, cudaStream_t st, int shape = 0);
-// One frame's half-sweep in a launch over several frames (pm_sweep_batch_kernel).
+int slots_shape_warps(int shape);
+int slots_shape_ctas(int shape);
+// Fills P.slots, P.task_cap and P.parts for a launch over a frame of n_views
+// micro-images and returns the dynamic shared memory of the plan, or 0 when none
+// fits.
+int slots_plan(PmParams& P, bool blur, int shape, int n_views);
+cudaError_t slots_sweep_grid(const FrameDev& F, const PmParams& P, int smem, int* n_ctas, int shape);
+cudaError_t launch_slots_sweep(const FrameDev& F, const PmParams& P, const StateDev& prev, const StateDev& next, int iter,
+                               int phase, int smem, int n_ctas, int* err, cudaStream_t st, int shape);
+// One frame's half-sweep in a launch over several frames.
 struct SweepItem {
     FrameDev F;
     PmParams P;             // P.view_queue: this frame's counter, zeroed before the launch
     StateDev prev, next;
     int iter, phase;
 };
-// Grid of the batch kernel for `smem` bytes of dynamic shared memory per CTA.
-cudaError_t sweep_batch_grid(int smem, bool blur, bool shift, bool tex, int* n_ctas, int shape = 0);
-// items: device array of n frames, all with or all without a blur channel, all
-// with textures (tex) or none.
-cudaError_t launch_sweep_batch(const SweepItem* items, int n, bool blur, bool shift, bool tex, int smem, int n_ctas,
-                               int* err, cudaStream_t st, int shape = 0);
+// items: device array of n frames, all with or all without a blur channel; smem
+// covers every frame's plan.
+cudaError_t slots_batch_grid(int smem, bool blur, bool shift, int* n_ctas, int shape);
+cudaError_t launch_slots_batch(const SweepItem* items, int n, bool blur, bool shift, int smem, int n_ctas, int* err,
+                               cudaStream_t st, int shape);
+
+// The warp-per-pixel half-sweep (pm_sweep.cu) of tap counting (P.tap_counter) and
+// of texture fetches (F.tex): grid, shared memory, and the global scratch it
+// needs (P.cost_scratch: per warp, the cost vectors of one pixel).
+cudaError_t sweep_warp_grid(const FrameDev& F, const PmParams& P, int* n_ctas);
+int sweep_warp_smem_bytes(const PmParams& P, bool blur, bool tex);
+size_t sweep_warp_scratch_bytes(const PmParams& P, int n_ctas);
+// Floats of global scratch one warp uses for K neighbours (PmParams::scratch_stride).
+int sweep_warp_stride(int K);
+cudaError_t launch_sweep_warp(const FrameDev& F, const PmParams& P, const StateDev& prev, const StateDev& next,
+                              int iter, int phase, int n_ctas, int* err, cudaStream_t st);
+// Texture fetches over several frames in one launch; all frames have textures.
+cudaError_t sweep_batch_grid(int smem, bool blur, bool shift, int* n_ctas);
+cudaError_t launch_sweep_batch(const SweepItem* items, int n, bool blur, bool shift, int smem, int n_ctas, int* err,
+                               cudaStream_t st);
 
 // Fills the layered float textures of a frame's tiles: texel (x, y) of layer
 // v % layers of surface v / layers is tiles[v * tile_stride + y * W + x].

@@ -1,0 +1,1419 @@
+// pm_slots.cu -- CheckerboardUpdateFrame (MIStereo/AdaptMIPMFrame.cu:520-947)
+// with pixel slots and pooled NCC evaluations.
+//
+// A CTA stages one micro-image and its neighbours and keeps up to 32 of its
+// pixels in flight, one slot (half a warp) each.  It runs in rounds: every slot
+// carries its pixel to the next point where costs are needed (the propagation
+// candidates; the cross-view proposals and refinement candidates; a proposal or
+// the candidates rebuilt because an earlier proposal won; the completion of the
+// winner's cost vector), and puts the (hypothesis, neighbour) NCCs it needs into
+// one list.  The list is sorted by the size of each NCC's tap rectangle, and the
+// CTA's warps evaluate it 32 NCCs at a time, one per lane, whichever pixels they
+// belong to.  A slot whose pixel is finished takes the next one.
+//
+// The tap rectangle of an NCC is the pixel's patch window cut down to the taps
+// whose source sample can lie in the neighbour window under the hypothesis; a
+// lane walks its own rectangle from its own origin, x offset outer, y offset
+// inner, so each NCC keeps the reference's accumulation order, and a tap whose
+// sample leaves the window adds exact zeros, which leaves the sums as the
+// reference's skipping does.
+//
+// Why: one pixel's NCCs fill 73% of the lanes of whole warps and the taps inside
+// both windows 41-57% of a warp's tap slots; pooled over the slots and sorted,
+// the lanes are full and 92% of the slots carry a tap of the lane's rectangle
+// (500 warp-taps per pixel instead of 860, 2048x1536, 12 neighbours, 15x15).  The
+// scalar code runs on half warps, the two halves of a warp on the same stage.
+// Bound by instruction issue: a warp-tap is about 40 instructions (3 loads, 18
+// FP32 operations, 6 integer products, 11 logical operations); packed pairs
+// (f32x2) halve the issue slots of the coordinates, measured 5% of the sweep.
+// Half-sweep, warp per pixel -> slots: 41 -> 28.1 ms (2048x1536, 12 neighbours,
+// 15x15), 8.0 -> 4.1 ms (1024x768, 6, 11x11), 27 -> 16.5 ms (2048x1536, ACMM, 5x5).
+#include <algorithm>
+#include <cstdint>
+#include <cuda_runtime.h>
+#include "pm_device.cuh"
+#include "pm_kernels.h"
+#include "pm_sweep_device.cuh"
+
+namespace pfd {
+
+namespace {
+
+// Launch shapes: warps per CTA and CTAs per SM.  Shape 0, the default, is the
+// fastest on the frames without a blur channel (2048x1536, 12 neighbours, 15x15:
+// 28.1 ms, 12x2 30.0, 8x3 33.4, 16x1 34.6); one CTA with all the shared memory
+// (shape 3) where the quads of a blur channel leave two CTAs few slots.
+template <int S> struct ShapeOf;
+template <> struct ShapeOf<0> { static constexpr int warps = 16, min_ctas = 2; };
+template <> struct ShapeOf<1> { static constexpr int warps = 12, min_ctas = 2; };
+template <> struct ShapeOf<2> { static constexpr int warps = 8, min_ctas = 3; };
+template <> struct ShapeOf<3> { static constexpr int warps = 16, min_ctas = 1; };
+constexpr int kShapeWarps[kSweepShapes] = { ShapeOf<0>::warps, ShapeOf<1>::warps, ShapeOf<2>::warps, ShapeOf<3>::warps };
+constexpr int kShapeCtas[kSweepShapes] = { ShapeOf<0>::min_ctas, ShapeOf<1>::min_ctas, ShapeOf<2>::min_ctas,
+                                           ShapeOf<3>::min_ctas };
+
+// What a slot keeps of its pixel between rounds.
+struct __align__(16) SlotState {
+    float4 best_plane;       // best plane so far
+    float4 c0, rn;           // refinement draws: random plane, random normal
+    float4 u;                // u1-u3 (perturbed normal), u4 (perturbed depth)
+    uint64_t skip;           // request: rows not to be evaluated
+    uint32_t slots;          // row of propagation slot s in bits [4s, 4s + 4)
+    uint32_t tsel;           // selected views
+    float best_cost;
+    int best_min;            // view of the lowest cost of the best plane
+    int best_row;            // 0: the current plane is still the best
+    int row_lo, row_hi;      // request: rows
+    int n_views;             // request: views; the first n_views entries of the slot's list, or every view (-1)
+    int xy;                  // x | y << 8
+    int r0;                  // row of the first refinement candidate
+    int n, hs;               // walk over the proposals: next one, its speculative row
+    uint32_t flags;          // candidate flags (bits 0-7), kFlag*
+};
+constexpr uint32_t kFlagChanged = 0x100u, kFlagPartial = 0x200u, kFlagSkip3 = 0x400u;
+
+// Where a slot's pixel stands: what the evaluation in flight is for.
+enum Stage : int { kIdle = 0, kNew, kProp, kSpec, kWalk, kRedo, kComplete, kWaits = 16 };
+
+// Hypotheses one slot can hold: 9 propagation rows, or every selected view's
+// proposal, the 5 refinement candidates and one rebuilt proposal.
+__host__ __device__ inline int slot_rows(int K) { return K + 6 > 9 ? K + 6 : 9; }
+// NCCs one request can ask for.
+__host__ __device__ inline int slot_tasks(int K) { return slot_rows(K) * K; }
+
+// Control words.
+enum Ctl : int { kCtlItem = 0, kCtlPixel, kCtlTasks, kCtlPass, kCtlWords = 8 };
+
+struct SlotPlan {
+    int off_ctl, off_Q, off_QB, off_R, off_RB, off_geo, off_ok, off_as, off_ac, off_pc, off_ps, off_bins, off_id, off_order;
+    int off_stage, off_wtab, off_plane, off_dp, off_cost, off_bvec, off_wgt, off_wres, off_wmin, off_aux, off_sel, off_state,
+        off_stages;
+    int rs, tx, ty, tab_n, rows, nbins, total;
+
+    __host__ __device__ static int a16(int v) { return (v + 15) & ~15; }
+    __host__ __device__ static SlotPlan make(int W, int H, int K, int ntap, bool blur, int tile_stride, int slots, int cap)
+    {
+        SlotPlan p;
+        p.rs = H | 1;                                    // odd: columns start in different banks
+        p.tx = ntap < W ? ntap : W;
+        p.ty = ntap < H ? ntap : H;
+        p.tab_n = p.tx * p.ty;
+        p.rows = slot_rows(K);
+        p.nbins = (p.tx / 2 + 1) * p.ty;
+        int o = 16;                                      // the staging barrier is at offset 0 of every plan
+        p.off_ctl = o;   o += kCtlWords * 4;
+        const int q_bytes = a16(K * (H + 1) * (W + 1) * 4), r_bytes = a16((2 * W * p.rs + 2 * H) * 4);
+        p.off_Q = o;     o += q_bytes;
+        p.off_QB = o;    o += blur ? q_bytes : 0;
+        p.off_R = o;     o += r_bytes;
+        p.off_RB = o;    o += blur ? r_bytes : 0;
+        p.off_geo = o;   o += a16(K * (int)sizeof(NbGeo));
+        p.off_ok = o;    o += a16(K * 4);
+        p.off_as = o;    o += a16(ntap * ntap * 4);
+        p.off_ac = o;    o += 256 * 4;
+        p.off_pc = o;    o += a16(W * H * 4);
+        p.off_ps = o;    o += a16(W * H * 4);
+        p.off_bins = o;  o += a16(p.nbins * 4);
+        // the staging buffer shares what follows: it is filled and read only between
+        // views, while no slot holds a pixel
+        p.off_stage = o;
+        const int stage_end = o + a16((1 + K) * tile_stride * (blur ? 2 : 1));
+        p.off_wtab = o;  o += a16(slots * p.tab_n * 4);
+        p.off_plane = o; o += slots * p.rows * 16;
+        p.off_dp = o;    o += slots * p.rows * 16;
+        p.off_cost = o;  o += a16(slots * p.rows * K * 4);
+        p.off_bvec = o;  o += a16(slots * K * 4);
+        p.off_wres = o;  o += a16(slots * p.rows * 4);
+        p.off_wmin = o;  o += a16(slots * p.rows * 4);
+        p.off_wgt = o;   o += a16(slots * K * 4);
+        p.off_aux = o;   o += a16(slots * K * 2);
+        p.off_sel = o;   o += a16(slots * K);
+        p.off_state = o; o += slots * (int)sizeof(SlotState);
+        p.off_stages = o; o += 64 * 4;
+        p.off_id = o;    o += a16(cap * 2);
+        p.off_order = o; o += a16(cap * 2);
+        // a lane that walks past its own rectangle reads at most one window past the tables
+        const int walk_end = p.off_wtab + (slots + 1) * p.tab_n * 4 + 64;
+        if (o < stage_end) o = stage_end;
+        if (o < walk_end) o = a16(walk_end);
+        p.total = o;
+        return p;
+    }
+};
+
+// ---- packed pairs of single-precision values: two taps per instruction ----------
+// Each half is the IEEE operation of the scalar instruction.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi)
+{
+    uint64_t v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ uint64_t fma2_rn(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t fma2_rm(uint64_t a, uint64_t b, uint64_t c)
+{
+    uint64_t d;
+    asm("fma.rm.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ uint64_t add2_rn(uint64_t a, uint64_t b)
+{
+    uint64_t d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ float lds_f32(uint32_t addr)
+{
+    float v;
+    asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+    return v;
+}
+
+// sb / 255 for sb = k / 256, 0 <= k < 2^16: the product with the rounded
+// reciprocal and one fused correction give the correctly rounded quotient
+// (division by a constant, Brisebarre and Muller), checked for all 2^16 values.
+__device__ __forceinline__ float div255(float sb)
+{
+    const float r = 0x1.010102p-8f;                      // 1 / 255 rounded
+    const float q = __fmul_rn(sb, r);
+    return __fmaf_rn(__fmaf_rn(-q, 255.0f, sb), r, q);
+}
+
+// The six moment sums of one NCC (and the blur sums).
+struct Moments {
+    float sr, srr, ss, sss, srs, sw, bsx, bsy;
+};
+
+// One tap: sample position (sx, sy) with its texture coordinates (tx, ty), the
+// tap's weight w and reference texel r.  A tap outside the neighbour window
+// (its bits compare above the window's) or with in false adds zeros.
+template <bool BLUR, bool SHIFT>
+__device__ __forceinline__ void tap(Moments& M, float sx, float sy, float tx, float ty, float w, float r, float rb,
+                                    float sh, bool in, uint32_t wb, uint32_t hb, uint32_t base, uint32_t kq,
+                                    uint32_t qb_delta)
+{
+    const bool v = in && (__float_as_uint(sx) < wb) && (__float_as_uint(sy) < hb);
+    // (a, b, ix, iy) in the four bytes; the entry's address is base + 4 ix + row iy
+    const uint32_t p = __byte_perm(__float_as_uint(tx), __float_as_uint(ty), 0x5140);
+    const uint32_t addr = v ? __dp4a(p, kq, base) : base;
+    const uint32_t a = __float_as_uint(tx) & 0xFFu, b = __float_as_uint(ty) & 0xFFu;
+    const uint32_t w11 = (a * b + 128u) >> 8;
+    const uint32_t hi = w11 * 65535u + b;
+    const uint32_t lo = a * 65535u + 256u - hi;
+    const uint32_t q = lds_u32(addr);
+    float s = __fsub_rn(__uint_as_float(__dp2a_lo(lo, q, __dp2a_hi(hi, q, 0x47000000u))), 32768.0f);
+    if (SHIFT) { s = __fsub_rn(s, sh); r = __fsub_rn(r, sh); }
+    const float wv = v ? w : 0.0f;
+    const float wr = __fmul_rn(wv, r), ws = __fmul_rn(wv, s);
+    M.sr = __fmaf_rn(wv, r, M.sr);
+    M.srr = __fmaf_rn(wr, r, M.srr);
+    M.ss = __fmaf_rn(wv, s, M.ss);
+    M.sss = __fmaf_rn(ws, s, M.sss);
+    M.srs = __fmaf_rn(wr, s, M.srs);
+    M.sw = __fadd_rn(M.sw, wv);
+    if (BLUR) {
+        const uint32_t qb = lds_u32(addr + qb_delta);
+        const float sb = __fsub_rn(__uint_as_float(__dp2a_lo(lo, qb, __dp2a_hi(hi, qb, 0x47000000u))), 32768.0f);
+        const float db = div255(sb);
+        M.bsx = __fadd_rn(M.bsx, v ? rb : 0.0f);
+        M.bsy = __fadd_rn(M.bsy, v ? db : 0.0f);
+    }
+}
+
+// The NCC cost of its moments (ComputeBilateralNCC_Frame, AdaptMIPMFrame.cu:140-179).
+template <bool BLUR>
+__device__ __forceinline__ float ncc_cost(const Moments& M, float blur_gain)
+{
+    float c = kCostMax;
+    if (M.sw > 1e-6f) {
+        const float inv = __fdiv_rn(1.0f, M.sw);
+        const float m_r = __fmul_rn(M.sr, inv), m_rr = __fmul_rn(M.srr, inv);
+        const float m_s = __fmul_rn(M.ss, inv), m_ss = __fmul_rn(M.sss, inv);
+        const float m_rs = __fmul_rn(M.srs, inv);
+        const float var_r = __fmaf_rn(-m_r, m_r, m_rr);
+        const float var_s = __fmaf_rn(-m_s, m_s, m_ss);
+        if (!(var_r < 1e-5f || var_s < 1e-5f)) {
+            const float cov = __fmaf_rn(-m_r, m_s, m_rs);
+            const float vv = __fsqrt_rn(__fmul_rn(var_r, var_s));
+            c = clamp_cost(__fsub_rn(1.0f, __fdiv_rn(cov, vv)));
+        }
+    }
+    if (BLUR) {
+        const float tb = __fsub_rn(M.bsx, M.bsy);
+        const float bw = pfd_expf(__fmul_rn(__fmul_rn(-0.007368f, tb), tb));
+        c = clamp_cost(__fmaf_rn(blur_gain, __fsub_rn(1.0f, bw), c));
+    }
+    return c;
+}
+
+// What the evaluation of a list entry reads, as shared-window addresses.
+struct EvalEnv {
+    uint32_t wtab, R, RB_delta, Q, QB_delta;
+    int q_bytes, tab_n, rs, inc;
+    uint32_t wb, hb, kq;
+};
+
+// One lane's NCC: the rectangle's tap columns and rows (nx, ny; 0 for a lane
+// without an entry), the addresses of its first tap (weight wa, reference texel
+// ra), the weight table's column step wstep in bytes, its first tap position
+// (fx, fy) and the neighbour's quads (base).  All lanes walk the widest and
+// tallest rectangle of the warp; taps past a lane's own rectangle add zeros.
+// Two taps per iteration, their coordinates in packed pairs.
+template <bool BLUR, bool SHIFT>
+__device__ __forceinline__ void walk(Moments& M, const EvalEnv& E, float3 dp, float stx, float sty, int nx, int ny,
+                                     uint32_t wa, uint32_t ra, uint32_t wstep, float fx, float fy, uint32_t base, float sh)
+{
+    const int NX = __reduce_max_sync(kFullMask, nx), NY = __reduce_max_sync(kFullMask, ny);
+    const int NYm = __reduce_min_sync(kFullMask, nx > 0 ? ny : NY);      // rows every lane with an entry keeps
+    const float finc = (float)E.inc;
+    const uint32_t rinc = (uint32_t)E.inc * 4u, rstep = (uint32_t)(E.inc * E.rs) * 4u;
+    const uint64_t dpy2 = pack2(dp.y, dp.y), dpz2 = pack2(dp.z, dp.z), stx2 = pack2(stx, stx), sty2 = pack2(sty, sty);
+    const uint64_t half2 = pack2(0.5f, 0.5f), scale2 = pack2(256.0f, 256.0f), magic2 = pack2(8388480.5f, 8388480.5f);
+    const uint64_t fy_start = pack2(fy, __fadd_rn(fy, finc)), fy_step = pack2(2.0f * finc, 2.0f * finc);
+    for (int ix = 0; ix < NX; ++ix) {
+        // a lane past its last column gets no sample position inside the window
+        const float axr = ix < nx ? __fmul_rn(dp.x, fx) : __int_as_float(0x7fffffff);
+        const uint64_t axr2 = pack2(axr, axr), fx2 = pack2(fx, fx);
+        uint64_t fy2 = fy_start;
+        uint32_t wp = wa, rp = ra;
+        int iy = 0;
+        for (; iy + 2 <= NYm; iy += 2) {
+            const uint64_t d2 = add2_rn(fma2_rn(dpy2, fy2, axr2), dpz2);
+            const uint64_t sx2 = fma2_rn(stx2, d2, fx2), sy2 = fma2_rn(sty2, d2, fy2);
+            const uint64_t tx2 = fma2_rm(add2_rn(sx2, half2), scale2, magic2);
+            const uint64_t ty2 = fma2_rm(add2_rn(sy2, half2), scale2, magic2);
+            float sx0, sx1, sy0, sy1, tx0, tx1, ty0, ty1;
+            unpack2(sx2, sx0, sx1);
+            unpack2(sy2, sy0, sy1);
+            unpack2(tx2, tx0, tx1);
+            unpack2(ty2, ty0, ty1);
+            const float w0 = lds_f32(wp), w1 = lds_f32(wp + 4u);
+            const float r0 = lds_f32(rp), r1 = lds_f32(rp + rinc);
+            const float b0 = BLUR ? lds_f32(rp + E.RB_delta) : 0.0f, b1 = BLUR ? lds_f32(rp + rinc + E.RB_delta) : 0.0f;
+            tap<BLUR, SHIFT>(M, sx0, sy0, tx0, ty0, w0, r0, b0, sh, true, E.wb, E.hb, base, E.kq, E.QB_delta);
+            tap<BLUR, SHIFT>(M, sx1, sy1, tx1, ty1, w1, r1, b1, sh, true, E.wb, E.hb, base, E.kq, E.QB_delta);
+            fy2 = add2_rn(fy2, fy_step);
+            wp += 8u;
+            rp += 2u * rinc;
+        }
+        float fyr, fyr1;
+        unpack2(fy2, fyr, fyr1);
+        for (; iy < NY; ++iy) {
+            const float d = __fadd_rn(__fmaf_rn(dp.y, fyr, axr), dp.z);
+            const float sx = __fmaf_rn(stx, d, fx), sy = __fmaf_rn(sty, d, fyr);
+            const float tx = __int_as_float(tex_coord_bits(sx)), ty = __int_as_float(tex_coord_bits(sy));
+            const float b = BLUR ? lds_f32(rp + E.RB_delta) : 0.0f;
+            tap<BLUR, SHIFT>(M, sx, sy, tx, ty, lds_f32(wp), lds_f32(rp), b, sh, iy < ny, E.wb, E.hb, base, E.kq,
+                             E.QB_delta);
+            fyr = __fadd_rn(fyr, finc);
+            wp += 4u;
+            rp += rinc;
+        }
+        fx = __fadd_rn(fx, finc);
+        wa += wstep;
+        ra += rstep;
+    }
+}
+
+// pixel_window without its divisions for a tap step of 1.
+__device__ __forceinline__ PixWin slot_window(const PmParams& P, int px, int py)
+{
+    if (P.inc != 1) return pixel_window(P, px, py);
+    PixWin w;
+    const int r = P.radius;
+    w.x0 = max(0, px - r);
+    w.y0 = max(0, py - r);
+    w.ii0 = w.x0 - px + r;
+    w.jj0 = w.y0 - py + r;
+    w.nX = min(P.W - 1, px + r) - w.x0 + 1;
+    w.nY = min(P.H - 1, py + r) - w.y0 + 1;
+    return w;
+}
+
+// The tap indices [i0, i1] (positions p0 + i inc) whose sample p + s can lie in
+// [0, lim) when the shift s is in [smin, smax]; eps covers the rounding of the
+// sample positions.  Rounding to integers by the addition of 1.5 * 2^23.
+__device__ __forceinline__ void cut_taps(float smin, float smax, float eps, float lim, float p0, float inv_inc, float& i0,
+                                         float& i1)
+{
+    const float lo = __fadd_rn(__fadd_ru((-smax - eps - p0) * inv_inc - 0.001f, kRneMagic), -kRneMagic);
+    const float hi = __fadd_rn(__fadd_rd((lim - smin + eps - p0) * inv_inc + 0.001f, kRneMagic), -kRneMagic);
+    i0 = fmaxf(i0, lo);
+    i1 = fminf(i1, hi);
+}
+
+// The rectangle of taps (first column and row, counts; 0 when empty) an NCC of
+// plane dp against a neighbour with steps (stx, sty) can keep.  The disparity is
+// affine over the window, so its range is at the corners; the second cut uses the
+// range over the first.
+__device__ __forceinline__ uint32_t tap_rect(const PixWin& pw, const PmParams& P, float3 dp, float stx, float sty,
+                                             float inv_inc)
+{
+    float i0 = 0.0f, i1 = (float)(pw.nX - 1), j0 = 0.0f, j1 = (float)(pw.nY - 1);
+    const float finc = (float)P.inc, X0 = (float)pw.x0, Y0 = (float)pw.y0;
+    const float mag = fabsf(dp.x) * (float)P.W + fabsf(dp.y) * (float)P.H + fabsf(dp.z);
+    if (mag * fmaxf(fabsf(stx), fabsf(sty)) < 1e6f) {    // false for NaN: the whole window
+        const float ex = 0.01f + 4e-6f * mag * fabsf(stx), ey = 0.01f + 4e-6f * mag * fabsf(sty);
+        const float dx = dp.x * finc, dy = dp.y * finc, d0 = dp.z + dp.x * X0 + dp.y * Y0;
+#pragma unroll
+        for (int rep = 0; rep < 2; ++rep) {
+            const float xa = dx * i0, xb = dx * i1, ya = dy * j0, yb = dy * j1;
+            const float dmin = d0 + fminf(xa, xb) + fminf(ya, yb), dmax = d0 + fmaxf(xa, xb) + fmaxf(ya, yb);
+            const float ax = stx * dmin, bx = stx * dmax, ay = sty * dmin, by = sty * dmax;
+            cut_taps(fminf(ax, bx), fmaxf(ax, bx), ex, (float)P.W, X0, inv_inc, i0, i1);
+            cut_taps(fminf(ay, by), fmaxf(ay, by), ey, (float)P.H, Y0, inv_inc, j0, j1);
+        }
+    }
+    if (!(i0 <= i1 && j0 <= j1)) return 0u;
+    const uint32_t a = (uint32_t)(int)i0, b = (uint32_t)(int)j0, c = (uint32_t)(int)i1, d = (uint32_t)(int)j1;
+    return a | (b << 8) | ((c - a + 1u) << 16) | ((d - b + 1u) << 24);
+}
+
+// Bin of a rectangle: columns in pairs from the widest down, rows up and down in
+// turn, so that neighbours in the sorted list differ by little.
+__device__ __forceinline__ int rect_bin(uint32_t rect, int tx, int ty)
+{
+    const int bx = ((int)((rect >> 16) & 0xFFu) - 1) >> 1, ry = (int)(rect >> 24) - 1;
+    return ((tx - 1) / 2 - bx) * ty + ((bx & 1) ? ry : ty - 1 - ry);
+}
+
+// ---- half-warp collectives -----------------------------------------------------
+struct Half {
+    uint32_t mask;           // the half's lanes in the warp
+    int hl, shift;           // lane in the half; 0 or 16
+    __device__ __forceinline__ float shfl(float v, int src) const { return __shfl_sync(mask, v, src, 16); }
+    __device__ __forceinline__ int shfl(int v, int src) const { return __shfl_sync(mask, v, src, 16); }
+    __device__ __forceinline__ uint32_t ballot(bool p) const { return (__ballot_sync(mask, p) >> shift) & 0xFFFFu; }
+    __device__ __forceinline__ uint32_t below(uint32_t bits) const { return bits & ((1u << hl) - 1u); }
+    __device__ __forceinline__ void sync() const { __syncwarp(mask); }
+};
+
+// A pixel's draw stream whose first 32 draws are worked out by the half's lanes
+// side by side (lane i holds draws i and 16 + i).
+struct HalfDraws {
+    const Half& hf;
+    uint64_t seed;
+    uint32_t sweep, pixel;
+    float d0, d1;
+    int n;
+    __device__ __forceinline__ float one(int i) const
+    {
+        const uint4 b = philox4x32_10(make_uint4((uint32_t)i >> 2, sweep, pixel, 0u),
+                                      make_uint2((uint32_t)seed, (uint32_t)(seed >> 32)));
+        const uint32_t w = (uint32_t)i & 3u;
+        const uint32_t r = w == 0 ? b.x : (w == 1 ? b.y : (w == 2 ? b.z : b.w));
+        return __fmul_rn((float)((r >> 8) + 1u), 0x1p-24f);
+    }
+    __device__ __forceinline__ HalfDraws(const Half& h, uint64_t s, uint32_t sw, uint32_t px)
+        : hf(h), seed(s), sweep(sw), pixel(px), n(0)
+    {
+        d0 = one(h.hl);
+        d1 = one(16 + h.hl);
+    }
+    __device__ __forceinline__ float uniform()
+    {
+        const int i = n++;
+        if (i < 16) return hf.shfl(d0, i);
+        if (i < 32) return hf.shfl(d1, i - 16);
+        return one(i);
+    }
+};
+
+// The CTA's view, as every slot sees it.
+struct View {
+    const float* R;          // [2 W][rs] reference texels, column-major, zeros past the window
+    const NbGeo* geo;        // [K]
+    const int* nb_ok;        // [K]
+    const float* a_s;        // [ntap * ntap]
+    const float* a_c;        // [256]
+    const float* pc;         // [ppv] previous costs
+    const uint32_t* ps;      // [ppv] previous selected views
+    int vid, nc, rs;
+    size_t vbase;
+};
+
+// A slot's arrays.
+struct Slot {
+    SlotState* st;
+    float* wtab;             // [tab_n] bilateral weights of the pixel's window, x outer
+    float4* plane;           // [rows]
+    float4* dp;              // [rows] disparity plane and the disparity at the pixel
+    float* cost;             // [rows][K]
+    float* bvec;             // [K] cost vector of the best plane
+    float* wgt;              // [K] view weights (draws per view)
+    uint8_t* sel;            // [K] the selected views, ascending
+    float* wres;             // [rows] weighted cost
+    int* wmin;               // [rows] view of the lowest cost
+    int16_t* aux;            // [K] proposals' sample positions, or -1
+};
+
+// ComputeWeightedCost_Frame (AdaptMIPMFrame.cu:284-317) of rows [lo, hi), one lane
+// per row, on every view or on the selected ones (nsel of them; the others have
+// weight 0 and unknown costs).
+__device__ __forceinline__ void weigh_rows(const Half& hf, const Slot& S, int K, int lo, int hi, int nc, int nsel)
+{
+    const int n = nsel >= 0 ? nsel : nc;
+    for (int h = lo + hf.hl; h < hi; h += 16) {
+        WeightedCost wc;
+        for (int i = 0; i < n; ++i) {
+            const int k = nsel >= 0 ? S.sel[i] : i;
+            wc.add(k, S.cost[h * K + k], S.wgt[k]);
+        }
+        S.wres[h] = wc.result();
+        S.wmin[h] = wc.min_idx;
+    }
+    hf.sync();
+}
+
+// The g-th pixel (row-major) whose colour (x + y) & 1 equals `colour`: two rows
+// hold W of them.
+__device__ __forceinline__ void nth_pixel(int g, int colour, int W, int& x, int& y)
+{
+    const int r2 = g / W;
+    int rem = g - r2 * W;
+    const int even = (W - colour + 1) >> 1;              // pixels of an even row
+    y = 2 * r2;
+    if (rem >= even) { rem -= even; ++y; }
+    x = 2 * rem + ((colour ^ y) & 1);
+}
+
+__device__ __forceinline__ bool same_bits(float4 a, float4 b)
+{
+    return __float_as_uint(a.x) == __float_as_uint(b.x) && __float_as_uint(a.y) == __float_as_uint(b.y) &&
+           __float_as_uint(a.z) == __float_as_uint(b.z) && __float_as_uint(a.w) == __float_as_uint(b.w);
+}
+
+__device__ __forceinline__ void request(SlotState& st, int row_lo, int row_hi, uint64_t skip, int n_views)
+{
+    st.row_lo = row_lo;
+    st.row_hi = row_hi;
+    st.skip = skip;
+    st.n_views = n_views;
+}
+
+// The disparity planes of rows [lo, hi), one lane per row.
+__device__ __forceinline__ void plane_rows(const Half& hf, const Slot& S, int lo, int hi, int x, int y)
+{
+    for (int h = lo + hf.hl; h < hi; h += 16) {
+        const float3 dp = disparity_plane(x, y, S.plane[h]);
+        S.dp[h] = make_float4(dp.x, dp.y, dp.z, to_disparity(x, y, dp));
+    }
+}
+
+// Takes pixel g: its weight table, the propagation candidates (AdaptMIPMFrame.cu:
+// 589-795) and the request for their costs.  Lane a < 8 works on direction a (up,
+// down, left, right; near on even lanes, far on odd ones).  Row 0 holds the
+// current plane, then one row per distinct candidate plane: a cost vector depends
+// only on the pixel and the plane.  The current plane's vector is the stored one
+// when that store is valid.
+__device__ __forceinline__ void begin_pixel(const Half& hf, const Slot& S, const View& V, const PmParams& P,
+                                            const StateDev& prev, int g, int phase)
+{
+    const int W = P.W, H = P.H, hl = hf.hl;
+    int x, y;
+    nth_pixel(g, phase, W, x, y);
+    const int center = y * W + x;
+    const size_t idx = V.vbase + center;
+    {
+        const PixWin pw = slot_window(P, x, y);
+        const float rc = V.R[x * V.rs + y];
+        const int n = pw.nX * pw.nY;
+        const uint32_t magic = pw.nY > 1 ? 0xFFFFFFFFu / (uint32_t)pw.nY + 1u : 0u;
+        for (int t = hl; t < n; t += 16) {
+            const int ix = pw.nY > 1 ? (int)__umulhi((uint32_t)t, magic) : t, iy = t - ix * pw.nY;
+            const float rv = V.R[(pw.x0 + ix * P.inc) * V.rs + pw.y0 + iy * P.inc];
+            const float cd = fabsf(__fsub_rn(rv, rc));
+            const int cdi = __float_as_int(__fadd_rn(cd, 8388608.0f)) & 0xFF;
+            const int ti = (pw.ii0 + ix) * P.ntap + (pw.jj0 + iy);
+            S.wtab[t] = pfd_expf_nonpos(__fsub_rn(V.a_s[ti], V.a_c[cdi]));
+        }
+    }
+    const int a = hl & 7, dir = a >> 1;
+    const bool vert = dir < 2, neg = (dir & 1) == 0;
+    const int D = dir == 0 ? y : (dir == 1 ? H - 1 - y : (dir == 2 ? x : W - 1 - x));
+    const int lat_lo = vert ? x : y, lat_hi = vert ? W - 1 - x : H - 1 - y;
+    const int sp = vert ? 1 : W, su = neg ? -(vert ? W : 1) : (vert ? W : 1);
+    const float* pc = V.pc;
+    int pos = center;
+    bool own = false;                                    // a sample of its own (not the near one's)
+    auto take = [&](float& cm, int q) { if (pc[q] < cm) { cm = pc[q]; pos = q; } };
+    if (!(a & 1)) {
+        if (D > 0) {
+            own = true;
+            pos = center + su;
+            float cm = pc[pos];
+            const int s = pos;
+            if (D > 1) take(cm, s + su);
+            if (D > 2 && lat_lo > 1) take(cm, s + 2 * su - sp);
+            if (D > 2 && lat_hi > 1) take(cm, s + 2 * su + sp);
+        }
+    } else if (D > 2) {
+        own = true;
+        pos = center + 3 * su;
+        float cm = pc[pos];
+        const int s = pos;
+        if (D > 3) take(cm, s + su);
+    }
+    const float4 cur = prev.plane[idx];
+    float4 q = cur;
+    if (own) q = prev.plane[V.vbase + pos];
+    const uint32_t flags = hf.ballot(D > 0) & 0xFFu, owns = hf.ballot(own) & 0xFFu;
+    const bool eqcur = same_bits(q, cur);
+    int match = -1;
+    for (int t = 0; t < 7; ++t) {
+        const float4 o = make_float4(hf.shfl(q.x, t), hf.shfl(q.y, t), hf.shfl(q.z, t), hf.shfl(q.w, t));
+        if (match < 0 && t < a && ((owns >> t) & 1u) && same_bits(o, q)) match = t;
+    }
+    const bool lead = own && hl < 8 && !eqcur && match < 0;
+    const uint32_t leads = hf.ballot(lead);
+    int row = lead ? 1 + __popc(hf.below(leads)) : 0;
+    const int mrow = hf.shfl(row, match < 0 ? 0 : match);
+    if (own && !eqcur && match >= 0) row = mrow;
+    const int nrow = hf.shfl(row, hl & ~1);              // the near sample's row
+    if (!own) row = (D > 0) ? nrow : 0;
+    if (lead) S.plane[row] = q;
+    const uint32_t slots = __reduce_or_sync(hf.mask, hl < 8 ? (uint32_t)row << (4 * hl) : 0u);
+    const bool use_cvec = P.cvec_ok != 0;
+    if (use_cvec)
+        for (int k = hl; k < V.nc; k += 16) S.cost[k] = P.cvec[idx * P.K + k];
+    if (hl == 0) {
+        S.plane[0] = cur;
+        S.st->xy = x | (y << 8);
+        S.st->slots = slots;
+        S.st->flags = flags;
+        request(*S.st, use_cvec ? 1 : 0, 1 + __popc(leads), 0ull, -1);
+    }
+    hf.sync();
+    plane_rows(hf, S, use_cvec ? 1 : 0, 1 + __popc(leads), x, y);
+}
+
+// After the propagation costs: view-selection priors and sampling (AdaptMIPMFrame.cu:
+// 797-875), the best propagation plane, the refinement's draws, and the request for
+// the cross-view proposals (:907-936) and the refinement candidates (:400-471), both
+// built from the best plane so far.
+__device__ __forceinline__ void after_propagation(const Half& hf, const Slot& S, const View& V, const FrameDev& F,
+                                                  const PmParams& P, const StateDev& prev, uint32_t sweep_id, float thr,
+                                                  float p_default)
+{
+    const int W = P.W, H = P.H, K = P.K, nc = V.nc, hl = hf.hl;
+    SlotState& st = *S.st;
+    const int x = st.xy & 0xFF, y = st.xy >> 8, center = y * W + x;
+    const uint32_t slots = st.slots, flags = st.flags;
+    HalfDraws g(hf, P.seed, sweep_id, (uint32_t)(V.vbase + center));
+    const int dpos[4] = { (y > 0) ? center - W : -1, (y < H - 1) ? center + W : -1, (x > 0) ? center - 1 : -1,
+                          (x < W - 1) ? center + 1 : -1 };
+    float pr[2] = { 0.0f, 0.0f };
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+        const int i = hl + 16 * half;
+        if (i >= nc) continue;
+        float prior = 0.0f;
+        for (int ii = 0; ii < 4; ++ii) {
+            if (dpos[ii] < 0) continue;
+            prior = __fadd_rn(prior, ((V.ps[dpos[ii]] >> i) & 1u) ? 0.9f : 0.1f);
+        }
+        float count = 0.0f, tmpw = 0.0f, p = 0.0f;
+        int count_false = 0;
+        for (int j = 0; j < 8; ++j) {
+            if (!((flags >> j) & 1u)) continue;
+            const float c = S.cost[(int)((slots >> (4 * j)) & 15u) * K + i];
+            if (c < thr) {
+                tmpw = __fadd_rn(tmpw, pfd_expf(__fdiv_rn(__fmul_rn(c, c), -0.18f)));
+                count = __fadd_rn(count, 1.0f);
+            }
+            if (c > 1.2f) count_false++;
+        }
+        if (count > 2.0f && count_false < 3) p = __fdiv_rn(tmpw, count);
+        else if (count_false < 3) p = p_default;
+        pr[half] = __fmul_rn(p, prior);
+    }
+    // the sums over views run in view order, as the reference's loops do
+    float psum = 0.0f;
+    for (int i = 0; i < nc; ++i) psum = __fadd_rn(psum, hf.shfl(i < 16 ? pr[0] : pr[1], i & 15));
+    // TransformPDFToCDF (CudaUtil.cu:491-507) and the 15 draws, one per lane: a draw's
+    // view is the first whose CDF exceeds it
+    uint32_t tsel = 0;
+    {
+        const float inv = __fdiv_rn(1.0f, psum);
+        const float rp = __fsub_rn(g.d0, 1.1920928955078125e-07f);
+        bool open = hl < 15;
+        float cum = 0.0f;
+        int c0 = 0, c1 = 0;                              // draws of this lane's views hl and 16 + hl
+        for (int i = 0; i < nc; ++i) {
+            cum = __fmaf_rn(hf.shfl(i < 16 ? pr[0] : pr[1], i & 15), inv, cum);
+            const bool hit = open && cum > rp;
+            open = open && !hit;
+            const uint32_t hits = hf.ballot(hit);
+            if (hits) tsel |= 1u << i;
+            if (hl == (i & 15)) { if (i < 16) c0 = __popc(hits); else c1 = __popc(hits); }
+        }
+        if (tsel == 0) {
+            tsel = nc < 32 ? (1u << nc) - 1u : ~0u;
+            c0 = c1 = 1;
+        }
+        if (hl < nc) {
+            S.wgt[hl] = (float)c0;
+            if ((tsel >> hl) & 1u) S.sel[__popc(tsel & ((1u << hl) - 1u))] = (uint8_t)hl;
+        }
+        if (16 + hl < nc) {
+            S.wgt[16 + hl] = (float)c1;
+            if ((tsel >> (16 + hl)) & 1u) S.sel[__popc(tsel & ((1u << (16 + hl)) - 1u))] = (uint8_t)(16 + hl);
+        }
+        hf.sync();
+    }
+    g.n = 15;
+    const int nh = st.row_hi;
+    weigh_rows(hf, S, K, 0, nh, nc, -1);
+    // current plane, then the candidates in slot order
+    float best_cost = S.wres[0];
+    int best_row = 0;
+    for (int s = 0; s < 8; ++s) {
+        if (!((flags >> s) & 1u)) continue;
+        const int r = (int)((slots >> (4 * s)) & 15u);
+        const float c = S.wres[r];
+        if (c < best_cost) { best_cost = c; best_row = r; }
+    }
+    const int best_min = S.wmin[best_row];
+    const float4 best_plane = S.plane[best_row];
+    for (int k = hl; k < nc; k += 16) S.bvec[k] = S.cost[best_row * K + k];
+    (void)g.uniform();                                   // depth_rand: drawn, never used
+    const float4 rn = random_normal(g);
+    const float u1 = g.uniform(), u2 = g.uniform(), u3 = g.uniform();
+    const float u4 = g.uniform();
+    const float4 c0 = random_plane(g, P.depth_min, P.depth_max);
+    hf.sync();                                           // every lane has read the rows before they are reused
+    const int nsel = __popc(tsel);
+    int nact = 0;
+    for (int n0 = 0; n0 < nsel; n0 += 16) {
+        const int n = n0 + hl;
+        int q = -1, k = -1, nvid = -1;
+        if (n < nsel) {
+            k = S.sel[n];
+            nvid = F.nb_ids[V.vid * K + k];
+            if (nvid >= 0) q = proposal_pos(V.geo[k], x, y, W, H, best_plane);
+        }
+        const uint32_t act = hf.ballot(q >= 0);
+        if (q >= 0)
+            S.plane[nact + __popc(hf.below(act))] =
+                proposal_plane(V.geo[k], prev.plane + (size_t)nvid * P.ppv, q, x, y, W);
+        if (n < nsel) S.aux[n] = (int16_t)q;
+        nact += __popc(act);
+    }
+    float4 cand[5];
+    refine_candidates(x, y, best_plane, c0, rn, u1, u2, u3, u4, P.pert_pi, cand);
+    // the candidate equal to the best plane has the best cost and cannot win
+    const bool skip3 = __float_as_uint(cand[3].w) == __float_as_uint(best_plane.w);
+    if (hl == 0) {
+        for (int i = 0; i < 5; ++i) S.plane[nact + i] = cand[i];
+        st.best_plane = best_plane;
+        st.best_cost = best_cost;
+        st.best_min = best_min;
+        st.best_row = best_row;
+        st.c0 = c0;
+        st.rn = rn;
+        st.u = make_float4(u1, u2, u3, u4);
+        st.tsel = tsel;
+        st.r0 = nact;
+        st.n = 0;
+        st.hs = 0;
+        st.flags = skip3 ? kFlagSkip3 : 0u;
+        request(st, 0, nact + 5, skip3 ? (1ull << (nact + 3)) : 0ull, nsel);
+    }
+    hf.sync();
+    plane_rows(hf, S, 0, nact + 5, x, y);
+}
+
+// The walk over the proposals in reference order and the refinement candidates
+// after it.  stage: what the costs that have just come in were for.  Returns the
+// stage of the next request, or kNew when the pixel's best plane is final and its
+// cost vector is known.
+__device__ __forceinline__ int after_speculation(const Half& hf, const Slot& S, const View& V, const FrameDev& F,
+                                                 const PmParams& P, const StateDev& prev, int stage)
+{
+    const int W = P.W, H = P.H, K = P.K, nc = V.nc, hl = hf.hl;
+    SlotState& st = *S.st;
+    const int x = st.xy & 0xFF, y = st.xy >> 8;
+    const int nsel = __popc(st.tsel), r0 = st.r0;
+    weigh_rows(hf, S, K, st.row_lo, st.row_hi, nc, nsel);
+    float best_cost = st.best_cost;
+    float4 best_plane = st.best_plane;
+    int best_min = st.best_min, n = st.n, hs = st.hs;
+    uint32_t flags = st.flags;
+    hf.sync();
+    if (stage != kRedo) {
+        bool resumed = stage == kWalk;
+        for (; n < nsel; ++n) {
+            const int spec_q = S.aux[n];
+            int q = spec_q, k = -1, nvid = -1;
+            if (flags & kFlagChanged) {
+                k = S.sel[n];
+                nvid = F.nb_ids[V.vid * K + k];
+                q = (nvid >= 0) ? proposal_pos(V.geo[k], x, y, W, H, best_plane) : -1;
+            }
+            if (q >= 0) {
+                const int row = (spec_q >= 0) ? hs : r0 + 5;
+                if (q != spec_q && !resumed) {
+                    // the best plane moved the sample position: rebuild this proposal in its
+                    // own row (or the spare row after the refinement candidates)
+                    const float4 proxy = proposal_plane(V.geo[k], prev.plane + (size_t)nvid * P.ppv, q, x, y, W);
+                    if (hl == 0) {
+                        S.plane[row] = proxy;
+                        st.best_plane = best_plane;
+                        st.best_cost = best_cost;
+                        st.best_min = best_min;
+                        st.n = n;
+                        st.hs = hs;
+                        st.flags = flags;
+                        request(st, row, row + 1, 0ull, nsel);
+                    }
+                    hf.sync();
+                    plane_rows(hf, S, row, row + 1, x, y);
+                    return kWalk;
+                }
+                const float c = S.wres[row];
+                if (c < best_cost) {
+                    best_cost = c;
+                    best_plane = S.plane[row];
+                    best_min = S.wmin[row];
+                    flags |= kFlagChanged | kFlagPartial;
+                }
+            }
+            resumed = false;
+            if (spec_q >= 0) ++hs;
+        }
+        if (flags & kFlagChanged) {
+            // candidates 2-4 follow the best plane: rebuild and evaluate them again
+            float4 cand[5];
+            refine_candidates(x, y, best_plane, st.c0, st.rn, st.u.x, st.u.y, st.u.z, st.u.w, P.pert_pi, cand);
+            const bool skip3 = __float_as_uint(cand[3].w) == __float_as_uint(best_plane.w);
+            flags = (flags & ~kFlagSkip3) | (skip3 ? kFlagSkip3 : 0u);
+            hf.sync();                                   // proposal rows may be read above
+            if (hl == 0) {
+                for (int i = 2; i < 5; ++i) S.plane[r0 + i] = cand[i];
+                st.best_plane = best_plane;
+                st.best_cost = best_cost;
+                st.best_min = best_min;
+                st.flags = flags;
+                request(st, r0 + 2, r0 + 5, skip3 ? (1ull << (r0 + 3)) : 0ull, nsel);
+            }
+            hf.sync();
+            plane_rows(hf, S, r0 + 2, r0 + 5, x, y);
+            return kRedo;
+        }
+    }
+    for (int i = 0; i < 5; ++i) {
+        if (i == 3 && (flags & kFlagSkip3)) continue;
+        const float c = S.wres[r0 + i];
+        if (c < best_cost) {
+            best_cost = c;
+            best_plane = S.plane[r0 + i];
+            best_min = S.wmin[r0 + i];
+            flags |= kFlagPartial;
+        }
+    }
+    hf.sync();
+    // proposals and refinement candidates were evaluated on the selected views only,
+    // which fixes their weighted cost; the winner's lowest-cost view runs over every
+    // view, and its vector is stored, so the whole vector is evaluated
+    if (hl == 0) {
+        st.best_plane = best_plane;
+        st.best_cost = best_cost;
+        st.best_min = best_min;
+        st.flags = flags;
+        if (flags & kFlagPartial) {
+            S.plane[0] = best_plane;
+            request(st, 0, 1, 0ull, -1);
+        }
+    }
+    hf.sync();
+    if (!(flags & kFlagPartial)) return kNew;
+    plane_rows(hf, S, 0, 1, x, y);
+    return kComplete;
+}
+
+// Writes the pixel's new state.  completed: row 0 holds the winner's cost vector
+// (a proposal or refinement candidate won); otherwise bvec does.
+__device__ __forceinline__ void finish_pixel(const Half& hf, const Slot& S, const View& V, const PmParams& P,
+                                             const StateDev& next, bool completed)
+{
+    const int K = P.K, nc = V.nc, hl = hf.hl, W = P.W;
+    SlotState& st = *S.st;
+    const int x = st.xy & 0xFF, y = st.xy >> 8;
+    const size_t idx = V.vbase + y * W + x;
+    int best_min = st.best_min, best_row = st.best_row;
+    const float* vec = S.bvec;
+    if (completed) {
+        weigh_rows(hf, S, K, 0, 1, nc, -1);
+        best_min = S.wmin[0];
+        best_row = -1;
+        vec = S.cost;
+    }
+    // the stored vector of the new current plane (unchanged when the current
+    // plane stays and its stored vector was used)
+    if (P.cvec && !(best_row == 0 && P.cvec_ok))
+        for (int k = hl; k < nc; k += 16) P.cvec[idx * K + k] = vec[k];
+    if (hl == 0) {
+        const float4 best_plane = st.best_plane;
+        uint32_t sel_out = st.tsel;
+        float cost_out = st.best_cost;
+        int disp_view = best_min;
+        if (P.acmm) {
+            // ACMM write-back (AdaptMIPMFrameACMM.cu:880-900, RecomputeSupportCostDisp_Frame
+            // :259-280): the final plane's vector over every view gives the stored cost
+            // (mean of the top-k), the selected views (the top-k mask) and the disp of the
+            // lowest-cost view; DetailRestorer_FrameACMM does nothing without a warm start
+            disp_view = -1;
+            int valid = 0;
+            for (int i = 0; i < nc; ++i)
+                if (vec[i] < 2.0f) {
+                    ++valid;
+                    if (disp_view < 0 || vec[i] < vec[disp_view]) disp_view = i;
+                }
+            cost_out = 2.0f;
+            sel_out = 0;
+            if (valid > 0) {
+                const int kk = min(valid, P.top_k);
+                float* tmp = S.cost + K;                 // row 1: free by now
+                for (int i = 0; i < nc; ++i) tmp[i] = vec[i];
+                for (int i = 0; i < kk; ++i)
+                    for (int j = i + 1; j < nc; ++j)
+                        if (tmp[j] < tmp[i]) { const float t = tmp[i]; tmp[i] = tmp[j]; tmp[j] = t; }
+                float m = 0.0f;
+                for (int i = 0; i < kk; ++i) m = __fadd_rn(m, tmp[i]);
+                cost_out = __fdiv_rn(m, (float)kk);
+                for (int i = 0; i < nc; ++i)
+                    if (vec[i] <= tmp[kk - 1]) sel_out |= 1u << i;
+            }
+        }
+        float4 best_disp = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (disp_view >= 0)
+            best_disp = geo_disp(V.geo[disp_view], x, y, to_disparity(x, y, disparity_plane(x, y, best_plane)));
+        next.plane[idx] = best_plane;
+        next.cost[idx] = cost_out;
+        next.disp[idx] = best_disp;
+        next.sel[idx] = sel_out;
+    }
+    hf.sync();
+}
+
+}  // namespace
+
+// One half-sweep of one frame by this CTA: it takes (micro-image, pixel part)
+// items from P.view_queue until none is left.  parity: the staging barrier's
+// phase, carried across frames.  Returns false when a staging wait gave up.
+template <bool BLUR, bool SHIFT, int WARPS>
+__device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev& F, const PmParams& P,
+                                            const StateDev& prev, const StateDev& next, int iter, int phase, int* err,
+                                            uint32_t& parity)
+{
+    const int W = P.W, H = P.H, K = P.K, ts = P.tile_stride;
+    const int n_slots = P.slots, cap = P.task_cap;
+    const SlotPlan L = SlotPlan::make(W, H, K, P.ntap, BLUR, ts, n_slots, cap);
+    {
+        // the plan must fit what the launch has (the decision is the same in every thread)
+        uint32_t dyn;
+        asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        if (!(L.total <= (int)dyn && P.view_queue != nullptr && n_slots >= 1 && n_slots <= 2 * WARPS && n_slots <= 32 &&
+              cap >= slot_tasks(K) && P.parts >= 1)) {
+            if (threadIdx.x == 0) atomicOr(err, PFD_DEVERR_SWEEP_CHECK);
+            return false;
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
+    Half hf;
+    hf.shift = lane & 16;
+    hf.hl = lane & 15;
+    hf.mask = 0xFFFFu << hf.shift;
+    int* ctl = (int*)(smem + L.off_ctl);
+    float* R = (float*)(smem + L.off_R);
+    float* RB = (float*)(smem + L.off_RB);
+    float* pc = (float*)(smem + L.off_pc);
+    uint32_t* ps = (uint32_t*)(smem + L.off_ps);
+    int* bins = (int*)(smem + L.off_bins);
+    int* stages = (int*)(smem + L.off_stages), *next_stages = stages + 32;
+    uint16_t* t_id = (uint16_t*)(smem + L.off_id);
+    uint16_t* t_order = (uint16_t*)(smem + L.off_order);
+    NbGeo* geo = (NbGeo*)(smem + L.off_geo);
+    int* okk = (int*)(smem + L.off_ok);
+    auto slot_at = [&](int s) {
+        Slot S;
+        S.st = (SlotState*)(smem + L.off_state) + s;
+        S.wtab = (float*)(smem + L.off_wtab) + s * L.tab_n;
+        S.plane = (float4*)(smem + L.off_plane) + s * L.rows;
+        S.dp = (float4*)(smem + L.off_dp) + s * L.rows;
+        S.cost = (float*)(smem + L.off_cost) + s * L.rows * K;
+        S.bvec = (float*)(smem + L.off_bvec) + s * K;
+        S.wgt = (float*)(smem + L.off_wgt) + s * K;
+        S.wres = (float*)(smem + L.off_wres) + s * L.rows;
+        S.wmin = (int*)(smem + L.off_wmin) + s * L.rows;
+        S.aux = (int16_t*)(smem + L.off_aux) + s * K;
+        S.sel = (uint8_t*)(smem + L.off_sel) + s * K;
+        return S;
+    };
+    const float inv_inc = 1.0f / (float)P.inc;
+    const int n_upd = (P.ppv + (phase == 0 ? 1 : 0)) / 2;      // pixels with (x + y) & 1 == phase
+    const uint32_t sweep_id = (uint32_t)(1 + 2 * iter + phase);
+    const float thr = __fmul_rn(0.8f, pfd_expf(__fdiv_rn((float)(iter * iter), -90.0f)));
+    const float p_default = pfd_expf(__fdiv_rn(__fmul_rn(thr, thr), -0.32f));
+
+    // per-launch tables
+    {
+        float* a_s = (float*)(smem + L.off_as);
+        float* a_c = (float*)(smem + L.off_ac);
+        for (int t = tid; t < P.ntap * P.ntap; t += blockDim.x) {
+            const float fi = (float)(-P.radius + (t / P.ntap) * P.inc);
+            const float fj = (float)(-P.radius + (t % P.ntap) * P.inc);
+            const float sd = __fsqrt_rn(__fmaf_rn(fj, fj, __fmul_rn(fi, fi)));
+            a_s[t] = __fdiv_rn(-sd, P.ss2);
+        }
+        for (int c = tid; c < 256; c += blockDim.x) a_c[c] = __fdiv_rn((float)c, P.cc2);
+        for (int e = tid; e < 2 * W * L.rs + 2 * H; e += blockDim.x) {
+            R[e] = 0.0f;
+            if (BLUR) RB[e] = 0.0f;
+        }
+        for (int e = tid; e < L.nbins; e += blockDim.x) bins[e] = 0;
+    }
+    EvalEnv E;
+    E.wtab = smem_u32(smem + L.off_wtab);
+    E.R = smem_u32(R);
+    E.RB_delta = BLUR ? (uint32_t)(L.off_RB - L.off_R) : 0u;
+    E.Q = smem_u32(smem + L.off_Q);
+    E.QB_delta = BLUR ? (uint32_t)(L.off_QB - L.off_Q) : 0u;
+    E.q_bytes = (H + 1) * (W + 1) * 4;
+    E.tab_n = L.tab_n;
+    E.rs = L.rs;
+    E.inc = P.inc;
+    E.wb = P.W_bits;
+    E.hb = P.H_bits;
+    E.kq = ((uint32_t)(W + 1) * 4u << 24) | (4u << 16);
+    View V;
+    V.R = R;
+    V.geo = geo;
+    V.nb_ok = okk;
+    V.a_s = (const float*)(smem + L.off_as);
+    V.a_c = (const float*)(smem + L.off_ac);
+    V.pc = pc;
+    V.ps = ps;
+    V.rs = L.rs;
+
+    // the CTAs take items one at a time from a shared counter, so a CTA that drew cheap
+    // ones takes more; which CTA updates a pixel does not change its result
+    for (;;) {
+        __syncthreads();                                 // every thread has read the previous item
+        if (tid == 0) ctl[kCtlItem] = atomicAdd(P.view_queue, 1);
+        __syncthreads();
+        const int item = ctl[kCtlItem];
+        if (item >= F.V * P.parts) break;
+        const int vid = item / P.parts, part = item - vid * P.parts;
+        const int g_lo = (int)((long long)n_upd * part / P.parts), g_hi = (int)((long long)n_upd * (part + 1) / P.parts);
+        const int nc = min(F.nb_counts[vid], K);
+        const size_t vbase = (size_t)vid * P.ppv;
+        V.vid = vid;
+        V.nc = nc;
+        V.vbase = vbase;
+        if (nc > 0 && tid == 0) {
+            // bulk copies of the 8-bit tiles; the threads' accesses to the shared area before
+            // the last barrier are ordered before them
+            uint8_t* stage = (uint8_t*)(smem + L.off_stage);
+            uint64_t* bar = (uint64_t*)smem;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_arrive_expect_tx(bar, (uint32_t)((1 + nc) * ts * (BLUR ? 2 : 1)));
+            for (int i = 0; i < 1 + nc; ++i) {
+                const int v = (i == 0) ? vid : F.nb_ids[vid * K + i - 1];
+                const int vv = (v < 0 || v >= F.V) ? vid : v;
+                bulk_copy_g2s(stage + i * ts, F.gray + (size_t)vv * ts, (uint32_t)ts, bar);
+                if (BLUR) bulk_copy_g2s(stage + (1 + nc + i) * ts, F.blur + (size_t)vv * ts, (uint32_t)ts, bar);
+            }
+        }
+        // the other colour keeps its state; so does every pixel of a view without neighbours
+        for (int e = tid; e < P.ppv; e += blockDim.x) {
+            const int ey = e / W, ex = e - ey * W;
+            const float c = prev.cost[vbase + e];
+            const uint32_t sv = prev.sel[vbase + e];
+            pc[e] = c;
+            ps[e] = sv;
+            if (part != 0 || (nc > 0 && ((ex + ey) & 1) == phase)) continue;
+            next.plane[vbase + e] = prev.plane[vbase + e];
+            next.cost[vbase + e] = c;
+            next.disp[vbase + e] = prev.disp[vbase + e];
+            next.sel[vbase + e] = sv;
+        }
+        if (nc <= 0) continue;
+        const float2 c0 = F.centers[vid];
+        for (int k = tid; k < K; k += blockDim.x) {
+            int v = (k < nc) ? F.nb_ids[vid * K + k] : -1;
+            if (v >= F.V) { atomicOr(err, PFD_DEVERR_SWEEP_CHECK); v = -1; }
+            okk[k] = (v >= 0);
+            geo[k] = make_geo(c0, F.centers[v >= 0 ? v : vid], P);
+        }
+        if (tid == 0) {
+            ctl[kCtlPixel] = g_lo;
+            ctl[kCtlTasks] = 0;
+        }
+        const bool ok = mbar_wait_bounded((uint64_t*)smem, parity, err);
+        if (__syncthreads_or(!ok)) return false;
+        parity ^= 1u;
+        {
+            const uint8_t* stage = (const uint8_t*)(smem + L.off_stage);
+            for (int e = tid; e < W * H; e += blockDim.x) {
+                const int ey = e / W, ex = e - ey * W;
+                R[ex * L.rs + ey] = (float)stage[e];
+                if (BLUR) RB[ex * L.rs + ey] = __fdiv_rn((float)stage[(1 + nc) * ts + e], 255.0f);
+            }
+            const int qs = W + 1, qn = (H + 1) * qs;
+            uint32_t* Q = (uint32_t*)(smem + L.off_Q);
+            uint32_t* QB = (uint32_t*)(smem + L.off_QB);
+            for (int e = tid; e < nc * qn; e += blockDim.x) {
+                const int k = e / qn, r = e - k * qn;
+                const int iy = r / qs, ix = r - iy * qs;
+                const int y0 = min(iy, H - 1), y1 = min(iy + 1, H - 1);
+                const int x0 = min(ix, W - 1), x1 = min(ix + 1, W - 1);
+                const uint8_t* s = stage + (1 + k) * ts;
+                Q[e] = (uint32_t)s[y0 * W + x0] | ((uint32_t)s[y0 * W + x1] << 8) | ((uint32_t)s[y1 * W + x0] << 16) |
+                       ((uint32_t)s[y1 * W + x1] << 24);
+                if (BLUR) {
+                    const uint8_t* sb = stage + (2 + nc + k) * ts;
+                    QB[e] = (uint32_t)sb[y0 * W + x0] | ((uint32_t)sb[y0 * W + x1] << 8) |
+                            ((uint32_t)sb[y1 * W + x0] << 16) | ((uint32_t)sb[y1 * W + x1] << 24);
+                }
+            }
+        }
+        // stage of every slot; a slot whose request did not fit the list keeps it (kWaits set)
+        if (tid < 32) { stages[tid] = tid < n_slots ? kNew : kIdle; next_stages[tid] = kIdle; }
+        __syncthreads();
+
+        for (;;) {
+            // ---- every slot on to its next request.  The halves take the slots ordered by
+            // stage, so the two halves of a warp mostly run the same code.
+            {
+                const int mine = stages[lane];
+                int rank = 0, below = 0;
+#pragma unroll
+                for (int k = kComplete; k >= kIdle; --k) {
+                    const uint32_t m = __ballot_sync(kFullMask, mine == k || (k == kIdle && (mine & kWaits)));
+                    if (mine == k || (k == kIdle && (mine & kWaits))) rank = below + __popc(m & ((1u << lane) - 1u));
+                    below += __popc(m);
+                }
+                int slot = -1;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t m = __ballot_sync(kFullMask, rank == 2 * warp + h);
+                    if (h == (lane >> 4)) slot = __ffs(m) - 1;
+                }
+                int stage = slot >= 0 ? stages[slot] : kIdle;
+                __syncwarp();
+                if (stage != kIdle && !(stage & kWaits)) {
+                    const Slot S = slot_at(slot);
+                    if (stage == kProp) {
+                        after_propagation(hf, S, V, F, P, prev, sweep_id, thr, p_default);
+                        stage = kSpec;
+                    } else {
+                        if (stage == kComplete) {
+                            finish_pixel(hf, S, V, P, next, true);
+                            stage = kNew;
+                        } else if (stage != kNew) {
+                            stage = after_speculation(hf, S, V, F, P, prev, stage);
+                            if (stage == kNew) finish_pixel(hf, S, V, P, next, false);
+                        }
+                        if (stage == kNew) {
+                            int g = 0;
+                            if (hf.hl == 0) g = atomicAdd(&ctl[kCtlPixel], 1);
+                            g = hf.shfl(g, 0);
+                            if (g < g_hi) {
+                                begin_pixel(hf, S, V, P, prev, g, phase);
+                                stage = kProp;
+                            } else {
+                                stage = kIdle;
+                            }
+                        }
+                    }
+                    if (hf.hl == 0) next_stages[slot] = stage;
+                } else if (slot >= 0 && hf.hl == 0) {
+                    next_stages[slot] = stage & ~kWaits;
+                }
+            }
+            __syncthreads();
+            // ---- the requests' NCCs into the list, 32 (row, view) pairs per warp at a time.
+            // Slots whose pairs do not fit the list wait for the next round.
+            {
+                const int stage = next_stages[lane];
+                int pairs = 0;
+                if (stage != kIdle) {
+                    const SlotState& st = *slot_at(lane).st;
+                    pairs = (st.row_hi - st.row_lo) * (st.n_views >= 0 ? st.n_views : nc);
+                }
+                if (!__any_sync(kFullMask, stage != kIdle)) break;       // the same in every warp
+                int upto = pairs;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(kFullMask, upto, o);
+                    if (lane >= o) upto += t;
+                }
+                const bool fits = upto <= cap;
+                if (warp == 0) stages[lane] = fits ? stage : (stage | kWaits);
+                int units = fits ? (pairs + 31) >> 5 : 0, first = units;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(kFullMask, first, o);
+                    if (lane >= o) first += t;
+                }
+                const int n_units = __shfl_sync(kFullMask, first, 31);
+                first -= units;
+                for (int u = warp; u < n_units; u += WARPS) {
+                    const uint32_t holds = __ballot_sync(kFullMask, units > 0 && first <= u);
+                    const int slot = 31 - __clz(holds);
+                    const int e = (u - __shfl_sync(kFullMask, first, slot)) * 32 + lane, total = __shfl_sync(kFullMask, pairs, slot);
+                    const Slot S = slot_at(slot);
+                    const SlotState& st = *S.st;
+                    const int nv = st.n_views, x = st.xy & 0xFF, y = st.xy >> 8;
+                    const uint64_t skip = st.skip;
+                    const PixWin pw = slot_window(P, x, y);
+                    const int per = nv >= 0 ? nv : nc;
+                    const uint32_t magic = per > 1 ? 0xFFFFFFFFu / (uint32_t)per + 1u : 0u;
+                    const int hr = per > 1 ? (int)__umulhi((uint32_t)e, magic) : e;
+                    const int h = st.row_lo + hr;
+                    int k = e - hr * per;
+                    uint32_t rect = 0u;
+                    if (e < total && !((skip >> h) & 1ull)) {
+                        if (nv >= 0) k = S.sel[k];
+                        if (okk[k]) {
+                            const float4 d = S.dp[h];
+                            const NbGeo g = geo[k];
+                            const float2 a = geo_anchor(g, x, y, d.w);
+                            if ((__float_as_uint(a.x) < P.W_bits) && (__float_as_uint(a.y) < P.H_bits))
+                                rect = tap_rect(pw, P, make_float3(d.x, d.y, d.z), g.stx, g.sty, inv_inc);
+                        }
+                        // no anchor in the window, or no tap: 2 without evaluation.  The cell of an
+                        // NCC to be evaluated holds its rectangle until its cost is known.
+                        S.cost[h * K + k] = rect ? __uint_as_float(rect) : kCostMax;
+                    }
+                    const uint32_t m = __ballot_sync(kFullMask, rect != 0u);
+                    if (!m) continue;
+                    int at = 0;
+                    if (lane == 0) at = atomicAdd(&ctl[kCtlTasks], __popc(m));
+                    at = __shfl_sync(kFullMask, at, 0) + __popc(m & ((1u << lane) - 1u));
+                    if (rect) {
+                        t_id[at] = (uint16_t)((slot << 11) | (h << 5) | k);
+                        atomicAdd(&bins[rect_bin(rect, L.tx, L.ty)], 1);
+                    }
+                }
+            }
+            __syncthreads();
+            // ---- sort by rectangle: bin offsets, then the order
+            const int n_tasks = ctl[kCtlTasks];
+            if (warp == 0) {
+                const int per = (L.nbins + 31) / 32;
+                int sum = 0;
+                for (int i = 0; i < per; ++i) {
+                    const int b = lane * per + i;
+                    if (b < L.nbins) sum += bins[b];
+                }
+                int off = sum;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int t = __shfl_up_sync(kFullMask, off, o);
+                    if (lane >= o) off += t;
+                }
+                off -= sum;
+                for (int i = 0; i < per; ++i) {
+                    const int b = lane * per + i;
+                    if (b < L.nbins) { const int c = bins[b]; bins[b] = off; off += c; }
+                }
+                if (lane == 0) ctl[kCtlPass] = 0;
+            }
+            __syncthreads();
+            for (int i = tid; i < n_tasks; i += blockDim.x)
+            {
+                const int id = t_id[i];
+                const uint32_t rect = ((const uint32_t*)(smem + L.off_cost))[((id >> 11) * L.rows + ((id >> 5) & 63)) * K + (id & 31)];
+                t_order[atomicAdd(&bins[rect_bin(rect, L.tx, L.ty)], 1)] = (uint16_t)id;
+            }
+            __syncthreads();
+            for (int e = tid; e < L.nbins; e += blockDim.x) bins[e] = 0;
+            if (tid == 0) ctl[kCtlTasks] = 0;
+            // ---- evaluate, 32 NCCs per warp at a time
+            for (;;) {
+                int p = 0;
+                if (lane == 0) p = atomicAdd(&ctl[kCtlPass], 1);
+                p = __shfl_sync(kFullMask, p, 0);
+                if (p * 32 >= n_tasks) break;
+                const bool act = p * 32 + lane < n_tasks;
+                const int id = act ? t_order[p * 32 + lane] : 0;
+                const int s = id >> 11, h = (id >> 5) & 63, k = id & 31;
+                float* cell = (float*)(smem + L.off_cost) + (s * L.rows + h) * K + k;
+                const uint32_t rect = act ? __float_as_uint(*cell) : 0u;
+                const float4 d = ((const float4*)(smem + L.off_dp))[s * L.rows + h];
+                const int xy = ((const SlotState*)(smem + L.off_state))[s].xy;
+                const int x = xy & 0xFF, y = xy >> 8;
+                const PixWin pw = slot_window(P, act ? x : 0, act ? y : 0);
+                const int i0 = rect & 0xFF, j0 = (rect >> 8) & 0xFF;
+                const int X = pw.x0 + i0 * P.inc, Y = pw.y0 + j0 * P.inc;
+                Moments M = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
+                const float sh = SHIFT ? R[(act ? x * L.rs + y : 0)] : 0.0f;
+                walk<BLUR, SHIFT>(M, E, make_float3(d.x, d.y, d.z), geo[k].stx, geo[k].sty, (int)((rect >> 16) & 0xFFu),
+                                  (int)(rect >> 24), E.wtab + (uint32_t)(s * L.tab_n + i0 * pw.nY + j0) * 4u,
+                                  E.R + (uint32_t)(X * L.rs + Y) * 4u, (uint32_t)pw.nY * 4u, (float)X, (float)Y,
+                                  E.Q + (uint32_t)(k * E.q_bytes), sh);
+                if (act) *cell = ncc_cost<BLUR>(M, P.blur_gain);
+            }
+            __syncthreads();
+        }
+    }
+    return true;
+}
+
+// The staging barrier (offset 0 of every plan), once per launch.
+__device__ __forceinline__ void init_barrier(unsigned char* smem)
+{
+    if (threadIdx.x == 0) mbar_init((uint64_t*)smem, 1);
+    __syncthreads();
+}
+
+template <bool BLUR, bool SHIFT, int SHAPE>
+__global__ void __launch_bounds__(32 * ShapeOf<SHAPE>::warps, ShapeOf<SHAPE>::min_ctas)
+pm_slots_kernel(FrameDev F, PmParams P, StateDev prev, StateDev next, int iter, int phase, int* err)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    init_barrier(smem);
+    uint32_t parity = 0;
+    sweep_slots<BLUR, SHIFT, ShapeOf<SHAPE>::warps>(smem, F, P, prev, next, iter, phase, err, parity);
+}
+
+// Several frames' half-sweeps in one launch, in list order: a CTA that finds a
+// frame's queue empty moves on to the next frame at once, so one frame's tail
+// overlaps the next one's start.  The dynamic shared memory is the largest of
+// the frames' plans.
+template <bool BLUR, bool SHIFT, int SHAPE>
+__global__ void __launch_bounds__(32 * ShapeOf<SHAPE>::warps, ShapeOf<SHAPE>::min_ctas)
+pm_slots_batch_kernel(const SweepItem* items, int n, int* err)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    init_barrier(smem);
+    uint32_t parity = 0;
+    for (int b = 0; b < n; ++b) {
+        const SweepItem it = items[b];
+        if (!sweep_slots<BLUR, SHIFT, ShapeOf<SHAPE>::warps>(smem, it.F, it.P, it.prev, it.next, it.iter, it.phase, err,
+                                                             parity))
+            return;
+    }
+}
+
+int slots_shape_warps(int shape) { return kShapeWarps[(shape >= 0 && shape < kSweepShapes) ? shape : 0]; }
+int slots_shape_ctas(int shape) { return kShapeCtas[(shape >= 0 && shape < kSweepShapes) ? shape : 0]; }
+
+// Slots, list capacity and parts of a half-sweep; returns the dynamic shared
+// memory of its plan, or 0 when none fits.
+int slots_plan(PmParams& P, bool blur, int shape, int n_views)
+{
+    const int warps = slots_shape_warps(shape);
+    for (int ctas = slots_shape_ctas(shape); ctas >= 1; --ctas) {
+        const int budget = std::min(227 * 1024, (228 * 1024) / ctas - 1024);
+        for (int s = std::min(32, 2 * warps); s >= 1; --s) {
+            if (ctas > 1 && s < warps) break;            // fewer slots than warps: fewer CTAs instead
+            const int cap = std::max(slot_tasks(P.K), s * 9 * P.K);
+            const SlotPlan L = SlotPlan::make(P.W, P.H, P.K, P.ntap, blur, P.tile_stride, s, cap);
+            if (L.total > budget) continue;
+            P.slots = s;
+            P.task_cap = cap;
+            P.parts = 1;
+            (void)n_views;
+            return L.total;
+        }
+    }
+    return 0;
+}
+
+template <int SHAPE>
+static const void* slots_kernel_of(bool blur, bool shift)
+{
+    if (shift) return blur ? (const void*)pm_slots_kernel<true, true, SHAPE> : (const void*)pm_slots_kernel<false, true, SHAPE>;
+    return blur ? (const void*)pm_slots_kernel<true, false, SHAPE> : (const void*)pm_slots_kernel<false, false, SHAPE>;
+}
+
+static const void* slots_kernel(int shape, bool blur, bool shift)
+{
+    switch (shape) {
+    case 1: return slots_kernel_of<1>(blur, shift);
+    case 2: return slots_kernel_of<2>(blur, shift);
+    case 3: return slots_kernel_of<3>(blur, shift);
+    default: return slots_kernel_of<0>(blur, shift);
+    }
+}
+
+template <int SHAPE>
+static const void* slots_batch_kernel_of(bool blur, bool shift)
+{
+    if (shift) return blur ? (const void*)pm_slots_batch_kernel<true, true, SHAPE>
+                           : (const void*)pm_slots_batch_kernel<false, true, SHAPE>;
+    return blur ? (const void*)pm_slots_batch_kernel<true, false, SHAPE>
+                : (const void*)pm_slots_batch_kernel<false, false, SHAPE>;
+}
+
+static const void* slots_batch_kernel(int shape, bool blur, bool shift)
+{
+    switch (shape) {
+    case 1: return slots_batch_kernel_of<1>(blur, shift);
+    case 2: return slots_batch_kernel_of<2>(blur, shift);
+    case 3: return slots_batch_kernel_of<3>(blur, shift);
+    default: return slots_batch_kernel_of<0>(blur, shift);
+    }
+}
+
+static cudaError_t slots_grid(const void* k, int threads, int smem, int* n_ctas)
+{
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    *n_ctas = sms * per_sm;
+    return cudaSuccess;
+}
+
+cudaError_t slots_sweep_grid(const FrameDev& F, const PmParams& P, int smem, int* n_ctas, int shape)
+{
+    return slots_grid(slots_kernel(shape, F.blur != nullptr, P.shifted != 0), 32 * slots_shape_warps(shape), smem, n_ctas);
+}
+
+cudaError_t launch_slots_sweep(const FrameDev& F, const PmParams& P, const StateDev& prev, const StateDev& next, int iter,
+                               int phase, int smem, int n_ctas, int* err, cudaStream_t st, int shape)
+{
+    if (smem <= 0 || smem > 227 * 1024) return cudaErrorInvalidConfiguration;
+    const void* k = slots_kernel(shape, F.blur != nullptr, P.shifted != 0);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaMemsetAsync(P.view_queue, 0, sizeof(int), st);
+    if (e != cudaSuccess) return e;
+    const int grid = std::max(1, (int)std::min<long long>(n_ctas, (long long)F.V * P.parts));
+    FrameDev f = F; PmParams p = P; StateDev a = prev, b = next; int it = iter, ph = phase; int* er = err;
+    void* args[] = { &f, &p, &a, &b, &it, &ph, &er };
+    return cudaLaunchKernel(k, dim3(grid), dim3(32 * slots_shape_warps(shape)), args, (size_t)smem, st);
+}
+
+cudaError_t slots_batch_grid(int smem, bool blur, bool shift, int* n_ctas, int shape)
+{
+    return slots_grid(slots_batch_kernel(shape, blur, shift), 32 * slots_shape_warps(shape), smem, n_ctas);
+}
+
+cudaError_t launch_slots_batch(const SweepItem* items, int n, bool blur, bool shift, int smem, int n_ctas, int* err,
+                               cudaStream_t st, int shape)
+{
+    if (n <= 0) return cudaSuccess;
+    if (smem <= 0 || smem > 227 * 1024) return cudaErrorInvalidConfiguration;
+    const void* k = slots_batch_kernel(shape, blur, shift);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const SweepItem* it = items; int nn = n; int* er = err;
+    void* args[] = { &it, &nn, &er };
+    return cudaLaunchKernel(k, dim3(std::max(1, n_ctas)), dim3(32 * slots_shape_warps(shape)), args, (size_t)smem, st);
+}
+
+}  // namespace pfd

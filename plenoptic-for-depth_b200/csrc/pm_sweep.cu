@@ -1,5 +1,7 @@
 // pm_sweep.cu -- CheckerboardUpdateFrame (MIStereo/AdaptMIPMFrame.cu:520-947)
-// with one warp per updated pixel.
+// with one warp per updated pixel: the half-sweep of tap-counting calibration
+// runs and of texture fetches (PFD_FETCH_TEXTURE).  The other half-sweeps run in
+// pm_slots.cu.
 //
 // A CTA stages one micro-image and its neighbours at a time; its warps take the
 // updated pixels of that micro-image one by one.  For a pixel, every cost
@@ -16,43 +18,33 @@
 //
 // Cross-view proposals depend on the best plane so far (AdaptMIPMFrame.cu:
 // 907-936), and the refinement candidates on the best plane after them
-// (:400-471).  Both are built speculatively from the best plane after
-// propagation and evaluated together, then walked in order; a proposal whose
-// neighbour-window sample position changed because an earlier one won is
-// rebuilt and evaluated again, and so are the refinement candidates that
-// follow the best plane, so the result is the sequential one.  A refinement
-// candidate bit-identical to the best plane has its cost and is not evaluated.
+// (:400-471).  Texture fetches build both speculatively from the best plane
+// after propagation, evaluate them together and walk them in order; a proposal
+// whose sample position changed because an earlier one won is rebuilt and
+// evaluated again, and so are the refinement candidates that follow the best
+// plane, so the result is the sequential one.  Tap counting evaluates exactly
+// what the reference does, in its order.
 //
-// Neighbour samples come from the texture unit: the frame's micro-images are
-// layered float textures with the reference's filter settings, and a tap is
-// one tex2DLayered fetch, the reference's own tex2D.  The other form (TEX
-// false, used by the tap-counting calibration) stages the neighbours in shared
-// memory as 32-bit quads, entry (iy, ix) packing the four texels of a bilinear
-// footprint, T(iy,ix), T(iy,ix+1), T(iy+1,ix), T(iy+1,ix+1), indices clamped
-// to the window, and blends them as the texture unit does (measured, and equal
-// to the fetches bit for bit).
+// Texture fetches: the frame's micro-images are layered float textures with the
+// reference's filter settings, and a tap is one tex2DLayered fetch, the
+// reference's own tex2D.  Tap counting stages the neighbours in shared memory
+// as 32-bit quads, entry (iy, ix) packing the four texels of a bilinear
+// footprint, T(iy,ix), T(iy,ix+1), T(iy+1,ix), T(iy+1,ix+1), indices clamped to
+// the window, and blends them as the texture unit does (measured, and equal to
+// the fetches bit for bit).
 #include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 #include "pm_device.cuh"
 #include "pm_kernels.h"
+#include "pm_sweep_device.cuh"
 
 namespace pfd {
 
 namespace {
 
-// Launch shapes: (warps per CTA, CTAs per SM the registers are sized for).
-// Shape 0 is the default; the others are the autotuner's alternatives
-// (pfd_set_autotune), which trade resident CTAs for warps per CTA and
-// registers per thread as the frame's shared-memory plan allows.
-template <int S> struct ShapeOf;
-template <> struct ShapeOf<0> { static constexpr int warps = 7, min_ctas = 4; };
-template <> struct ShapeOf<1> { static constexpr int warps = 8, min_ctas = 3; };
-template <> struct ShapeOf<2> { static constexpr int warps = 4, min_ctas = 6; };
-template <> struct ShapeOf<3> { static constexpr int warps = 10, min_ctas = 2; };
-constexpr int kShapeWarps[kSweepShapes] = { ShapeOf<0>::warps, ShapeOf<1>::warps, ShapeOf<2>::warps, ShapeOf<3>::warps };
-constexpr int kShapeCtas[kSweepShapes] = { ShapeOf<0>::min_ctas, ShapeOf<1>::min_ctas, ShapeOf<2>::min_ctas,
-                                           ShapeOf<3>::min_ctas };
+// Launch shape: warps per CTA, and the CTAs per SM the registers are sized for.
+constexpr int kWarps = 7, kMinCtas = 4;
 
 struct Quad {
     const float* R;          // [H][W] reference texels
@@ -156,85 +148,6 @@ struct Plan {
     }
 };
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ float4 lds_f4(uint32_t addr)
-{
-    float4 v;
-    asm("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
-    return v;
-}
-
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr)
-{
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-    return v;
-}
-
-// Linear-filter fetch of the measured texture unit (see Tiles in pm_device.cuh)
-// from a quad entry: 256 s = 256 T00 + a (T10 - T00) + b (T01 - T00) + w11 (T11 - T01 - T10 + T00)
-// with w11 = (a b + 128) >> 8, regrouped per texel as
-// 256 s = T00 w00 + T10 w10 + T01 w01 + T11 w11, w10 = a - w11, w01 = b - w11,
-// w00 = 256 - w10 - b: all four weights lie in [0, 256], so two 16-bit pairs of
-// weights against the quad's four bytes make the sum with two dp2a, exactly.
-struct QuadWeights {
-    uint32_t lo;             // w00 | w10 << 16, against T00, T10 (the quad's low bytes)
-    uint32_t hi;             // w01 | w11 << 16, against T01, T11
-};
-
-// hi = w01 + 65536 w11 = b + 65535 w11, and lo + hi = 256 + 65535 a (w00 + w01 =
-// 256 - a, w10 + w11 = a), so lo = 256 + 65535 a - hi: no weight is negative, so
-// no half borrows from the other.
-__device__ __forceinline__ QuadWeights quad_weights(int tbx, int tby)
-{
-    const uint32_t a = (uint32_t)tbx & 0xFFu, b = (uint32_t)tby & 0xFFu;
-    const uint32_t w11 = (a * b + 128u) >> 8;
-    QuadWeights q;
-    q.hi = w11 * 65535u + b;
-    q.lo = a * 65535u + 256u - q.hi;
-    return q;
-}
-
-__device__ __forceinline__ float quad_blend(const QuadWeights& w, uint32_t q)
-{
-    const uint32_t s256 = __dp2a_lo(w.lo, q, __dp2a_hi(w.hi, q, 0u));
-    return __fsub_rn(__uint_as_float(s256 | 0x47000000u), 32768.0f);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(bar)), "r"(count) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes)
-{
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void bulk_copy_g2s(void* dst, const void* src, uint32_t bytes, uint64_t* bar)
-{
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity)
-{
-    uint32_t done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-                 : "=r"(done) : "r"(smem_u32(bar)), "r"(parity) : "memory");
-    return done != 0;
-}
-// Bounded wait (about 2^22 polls): records PFD_DEVERR_TMA_TIMEOUT and gives up.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int* err)
-{
-    for (uint32_t it = 0; it < (1u << 22); ++it) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if (it > 64) __nanosleep(128);
-    }
-    if (err) atomicOr(err, PFD_DEVERR_TMA_TIMEOUT);
-    return false;
-}
-
 // Stages micro-image vid and its neighbours: bulk copies of the 8-bit tiles,
 // then the reference as floats and the neighbours as quads.  The mbarrier is
 // reused with alternating parity, one phase per staged view.
@@ -315,28 +228,6 @@ __device__ bool stage_view(unsigned char* smem, const Plan& L, const FrameDev& F
     T.txbh = txbh;
     T.txl = txl;
     return true;
-}
-
-// The pixel's patch window: the patch's taps (x offset i, y offset j, step inc)
-// that fall inside the micro-image, as a rectangle of nX x nY taps.
-struct PixWin {
-    int x0, y0, nX, nY;      // first tap position and tap counts
-    int ii0, jj0;            // offset index of the first tap ((x0 - px + r) / inc)
-};
-
-__device__ __forceinline__ PixWin pixel_window(const PmParams& P, int px, int py)
-{
-    PixWin w;
-    const int r = P.radius, inc = P.inc;
-    const int sx = max(0, (r - px + inc - 1) / inc), sy = max(0, (r - py + inc - 1) / inc);
-    w.ii0 = sx;
-    w.jj0 = sy;
-    w.x0 = px - r + sx * inc;
-    w.y0 = py - r + sy * inc;
-    const int ex = min(P.ntap - 1, (P.W - 1 - px + r) / inc), ey = min(P.ntap - 1, (P.H - 1 - py + r) / inc);
-    w.nX = max(0, ex - sx + 1);
-    w.nY = max(0, ey - sy + 1);
-    return w;
 }
 
 // Reference-side table of the pixel: (w, w r, r, r_blur / 255) per tap, x outer.
@@ -603,12 +494,6 @@ __device__ __forceinline__ bool nth_pixel(int g, int colour, int W, int H, int& 
     return false;
 }
 
-__device__ __forceinline__ int nth_set_bit(uint32_t m, int n)
-{
-    for (int i = 0; i < n && m; ++i) m &= m - 1;
-    return m ? __ffs(m) - 1 : -1;
-}
-
 struct Cands {
     int flag[8];
     int pos[8];
@@ -672,50 +557,6 @@ __device__ __forceinline__ void find_candidates(const float* pc, int x, int y, i
         C.flag[6] = 1; C.pos[6] = scan(s, pts, ok, 4);
     }
     if (x >= W - 3 && x < W - 1) { C.flag[7] = 1; C.pos[7] = C.pos[6]; C.src[7] = 6; }
-}
-
-// BuildCrossViewPlaneProposal (AdaptMIPMFrame.cu:350-398): the sample position
-// q (local index) of pixel (x, y) under `cur` in neighbour k, or -1.  This and
-// proposal_plane are called from three places each and kept out of line: less
-// code between the NCC passes (1.5% of the half-sweep's time, measured).
-__device__ __noinline__ int proposal_pos(const NbGeo& gk, int x, int y, int W, int H, float4 cur)
-{
-    const float dcur = to_disparity(x, y, disparity_plane(x, y, cur));
-    const float2 qf = geo_anchor(gk, x, y, dcur);
-    const float fqx = floorf(__fadd_rn(qf.x, 0.5f)), fqy = floorf(__fadd_rn(qf.y, 0.5f));
-    if (!(fqx >= 0.0f && fqx < (float)W && fqy >= 0.0f && fqy < (float)H)) return -1;
-    return (int)fqy * W + (int)fqx;
-}
-
-__device__ __noinline__ float4 proposal_plane(const NbGeo& gk, const float4* nb_plane, int q, int x, int y, int W)
-{
-    const int qx = q % W, qy = q / W;
-    const float4 hn = nb_plane[q];
-    const float3 dpn = disparity_plane(qx, qy, hn);
-    float denom = __fmaf_rn(dpn.y, gk.by, __fmaf_rn(dpn.x, gk.bx, 1.0f));
-    denom = safe_denom(denom);
-    return encode_plane(x, y, __fdiv_rn(dpn.x, denom), __fdiv_rn(dpn.y, denom), __fdiv_rn(dpn.z, denom));
-}
-
-// The five candidates of PlaneHypothesisRefinement_Frame (AdaptMIPMFrame.cu:
-// 400-471) for the best plane `best`, from the draws already taken (c0: the
-// random plane, rn: the random normal, u1-u3: the perturbation, u4: the depth
-// perturbation).
-__device__ __noinline__ void refine_candidates(int x, int y, float4 best, float4 c0, float4 rn, float u1, float u2,
-                                               float u3, float u4, float pert, float4 (&cand)[5])
-{
-    const float depth_now = best.w;
-    const float4 pn = perturbed_normal_u(x, y, best, u1, u2, u3, pert);
-    const float dmin_p = __fmul_rn(__fsub_rn(1.0f, 0.02f), depth_now);
-    const float dmax_p = __fmul_rn(__fadd_rn(1.0f, 0.02f), depth_now);
-    const float depth_perturbed = __fmaf_rn(u4, __fsub_rn(dmax_p, dmin_p), dmin_p);
-    cand[0] = c0;
-    cand[1] = rn;
-    cand[2] = pn;
-    cand[3] = best;
-    cand[4] = best;
-    cand[4].w = depth_perturbed;
-    for (int i = 1; i < 5; ++i) cand[i].w = to_disparity(x, y, disparity_plane(x, y, cand[i]));
 }
 
 }  // namespace
@@ -1128,171 +969,115 @@ __device__ __forceinline__ void init_barrier(unsigned char* smem)
     __syncthreads();
 }
 
-template <bool BLUR, bool COUNT, bool SHIFT, int SHAPE, bool TEX>
-__global__ void __launch_bounds__(32 * ShapeOf<SHAPE>::warps, ShapeOf<SHAPE>::min_ctas)
+template <bool BLUR, bool COUNT, bool SHIFT, bool TEX>
+__global__ void __launch_bounds__(32 * kWarps, kMinCtas)
 pm_sweep_warp_kernel(FrameDev F, PmParams P, StateDev prev, StateDev next, int iter, int phase, int* err)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     init_barrier(smem);
     uint32_t parity = 0;
-    sweep_frame<BLUR, COUNT, SHIFT, TEX, ShapeOf<SHAPE>::warps>(smem, F, P, prev, next, iter, phase, err, parity);
+    sweep_frame<BLUR, COUNT, SHIFT, TEX, kWarps>(smem, F, P, prev, next, iter, phase, err, parity);
 }
 
 // Several frames' half-sweeps in one launch, in list order: a CTA that finds a
 // frame's queue empty moves on to the next frame at once, so one frame's tail
 // overlaps the next one's start.  The dynamic shared memory is the largest of
 // the frames' plans.
-template <bool BLUR, bool SHIFT, int SHAPE, bool TEX>
-__global__ void __launch_bounds__(32 * ShapeOf<SHAPE>::warps, ShapeOf<SHAPE>::min_ctas)
-pm_sweep_batch_kernel(const SweepItem* items, int n, int* err)
+template <bool BLUR, bool SHIFT>
+__global__ void __launch_bounds__(32 * kWarps, kMinCtas) pm_sweep_batch_kernel(const SweepItem* items, int n, int* err)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     init_barrier(smem);
     uint32_t parity = 0;
     for (int b = 0; b < n; ++b) {
         const SweepItem it = items[b];
-        if (!sweep_frame<BLUR, false, SHIFT, TEX, ShapeOf<SHAPE>::warps>(smem, it.F, it.P, it.prev, it.next, it.iter,
-                                                                         it.phase, err, parity))
+        if (!sweep_frame<BLUR, false, SHIFT, true, kWarps>(smem, it.F, it.P, it.prev, it.next, it.iter, it.phase, err,
+                                                           parity))
             return;
     }
 }
 
-int sweep_shape_warps(int shape) { return kShapeWarps[(shape >= 0 && shape < kSweepShapes) ? shape : 0]; }
-
-// Tap counting stages the neighbours in shared memory; the other sweeps fetch
-// them from the frame's textures when it has them.
-static bool uses_tex(const FrameDev& F, const PmParams& P) { return F.tex != nullptr && P.tap_counter == nullptr; }
-
-int sweep_warp_smem_bytes(const PmParams& P, bool blur, int shape, bool tex)
+int sweep_warp_smem_bytes(const PmParams& P, bool blur, bool tex)
 {
-    return Plan::make(P.W, P.H, P.K, P.ntap, blur, P.tile_stride, sweep_shape_warps(shape), tex && !P.tap_counter).total;
+    return Plan::make(P.W, P.H, P.K, P.ntap, blur, P.tile_stride, kWarps, tex && !P.tap_counter).total;
 }
 
 int sweep_warp_stride(int K) { return sweep_warp_words(K); }
 
-size_t sweep_warp_scratch_bytes(const PmParams& P, int n_ctas, int shape)
+size_t sweep_warp_scratch_bytes(const PmParams& P, int n_ctas)
 {
-    return (size_t)n_ctas * sweep_shape_warps(shape) * (size_t)sweep_warp_words(P.K) * 4u;
+    return (size_t)n_ctas * kWarps * (size_t)sweep_warp_words(P.K) * 4u;
 }
 
 // Dynamic shared memory of a sweep kernel, and for the texture-fetch kernels the
-// carveout they ask for: the shared memory of the CTAs per SM the shape's
-// registers allow (with the 1 KB each CTA reserves), so the rest of the SM's
-// 256 KB stays L1 and texture cache.  The shared-memory kernels keep the
-// driver's choice.
-static cudaError_t set_smem(const void* k, int smem, int shape, bool tex)
+// carveout they ask for: the shared memory of the CTAs per SM the registers
+// allow (with the 1 KB each CTA reserves), so the rest of the SM's 256 KB stays
+// L1 and texture cache.
+static cudaError_t set_smem(const void* k, int smem, bool tex)
 {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess || !tex) return e;
-    const int ctas = kShapeCtas[(shape >= 0 && shape < kSweepShapes) ? shape : 0];
-    const long need = (long)ctas * (smem + 1024);
+    const long need = (long)kMinCtas * (smem + 1024);
     const int pct = (int)std::min<long>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024) + 1);
     return cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 
-template <class Kern>
-static cudaError_t launch_k(Kern k, dim3 grid, dim3 block, int smem, int shape, bool tex, cudaStream_t st,
-                            void** args)
-{
-    cudaError_t e = set_smem((const void*)k, smem, shape, tex);
-    if (e != cudaSuccess) return e;
-    return cudaLaunchKernel((const void*)k, grid, block, args, (size_t)smem, st);
-}
-
-// The half-sweep kernel of one variant; tap counting exists in shape 0 with
-// shared-memory fetches only.
-template <int SHAPE, bool TEX>
-static const void* warp_kernel_of(bool blur, bool shift)
-{
-    if (shift) return blur ? (const void*)pm_sweep_warp_kernel<true, false, true, SHAPE, TEX>
-                           : (const void*)pm_sweep_warp_kernel<false, false, true, SHAPE, TEX>;
-    return blur ? (const void*)pm_sweep_warp_kernel<true, false, false, SHAPE, TEX>
-                : (const void*)pm_sweep_warp_kernel<false, false, false, SHAPE, TEX>;
-}
-
-template <int SHAPE>
-static const void* warp_kernel_of(bool blur, bool shift, bool tex)
-{
-    return tex ? warp_kernel_of<SHAPE, true>(blur, shift) : warp_kernel_of<SHAPE, false>(blur, shift);
-}
-
-static const void* warp_kernel(int shape, bool blur, bool count, bool shift, bool tex)
+// The half-sweep kernel of one variant: tap counting (shared-memory fetches) or
+// texture fetches.
+static const void* warp_kernel(bool blur, bool count, bool shift)
 {
     if (count) {
-        if (shift) return blur ? (const void*)pm_sweep_warp_kernel<true, true, true, 0, false>
-                               : (const void*)pm_sweep_warp_kernel<false, true, true, 0, false>;
-        return blur ? (const void*)pm_sweep_warp_kernel<true, true, false, 0, false>
-                    : (const void*)pm_sweep_warp_kernel<false, true, false, 0, false>;
+        if (shift) return blur ? (const void*)pm_sweep_warp_kernel<true, true, true, false>
+                               : (const void*)pm_sweep_warp_kernel<false, true, true, false>;
+        return blur ? (const void*)pm_sweep_warp_kernel<true, true, false, false>
+                    : (const void*)pm_sweep_warp_kernel<false, true, false, false>;
     }
-    switch (shape) {
-    case 1: return warp_kernel_of<1>(blur, shift, tex);
-    case 2: return warp_kernel_of<2>(blur, shift, tex);
-    case 3: return warp_kernel_of<3>(blur, shift, tex);
-    default: return warp_kernel_of<0>(blur, shift, tex);
-    }
+    if (shift) return blur ? (const void*)pm_sweep_warp_kernel<true, false, true, true>
+                           : (const void*)pm_sweep_warp_kernel<false, false, true, true>;
+    return blur ? (const void*)pm_sweep_warp_kernel<true, false, false, true>
+                : (const void*)pm_sweep_warp_kernel<false, false, false, true>;
 }
 
-template <int SHAPE, bool TEX>
-static const void* batch_kernel_of(bool blur, bool shift)
+static const void* batch_kernel(bool blur, bool shift)
 {
-    if (blur) return shift ? (const void*)pm_sweep_batch_kernel<true, true, SHAPE, TEX>
-                           : (const void*)pm_sweep_batch_kernel<true, false, SHAPE, TEX>;
-    return shift ? (const void*)pm_sweep_batch_kernel<false, true, SHAPE, TEX>
-                 : (const void*)pm_sweep_batch_kernel<false, false, SHAPE, TEX>;
+    if (blur) return shift ? (const void*)pm_sweep_batch_kernel<true, true> : (const void*)pm_sweep_batch_kernel<true, false>;
+    return shift ? (const void*)pm_sweep_batch_kernel<false, true> : (const void*)pm_sweep_batch_kernel<false, false>;
 }
 
-template <int SHAPE>
-static const void* batch_kernel_of(bool blur, bool shift, bool tex)
-{
-    return tex ? batch_kernel_of<SHAPE, true>(blur, shift) : batch_kernel_of<SHAPE, false>(blur, shift);
-}
-
-static const void* batch_kernel(int shape, bool blur, bool shift, bool tex)
-{
-    switch (shape) {
-    case 1: return batch_kernel_of<1>(blur, shift, tex);
-    case 2: return batch_kernel_of<2>(blur, shift, tex);
-    case 3: return batch_kernel_of<3>(blur, shift, tex);
-    default: return batch_kernel_of<0>(blur, shift, tex);
-    }
-}
-
-static cudaError_t grid_for(const void* k, int threads, int smem, int shape, bool tex, int* n_ctas)
+static cudaError_t grid_for(const void* k, int smem, bool tex, int* n_ctas)
 {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = set_smem(k, smem, shape, tex);
+    cudaError_t e = set_smem(k, smem, tex);
     if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kWarps, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     *n_ctas = sms * per_sm;
     return cudaSuccess;
 }
 
-cudaError_t sweep_warp_grid(const FrameDev& F, const PmParams& P, int* n_ctas, int shape)
+cudaError_t sweep_warp_grid(const FrameDev& F, const PmParams& P, int* n_ctas)
 {
-    const bool blur = F.blur != nullptr, tex = uses_tex(F, P);
-    if (P.tap_counter) shape = 0;
-    return grid_for(warp_kernel(shape, blur, P.tap_counter != nullptr, P.shifted != 0, tex),
-                    32 * sweep_shape_warps(shape), sweep_warp_smem_bytes(P, blur, shape, tex), shape, tex, n_ctas);
+    const bool blur = F.blur != nullptr, count = P.tap_counter != nullptr;
+    return grid_for(warp_kernel(blur, count, P.shifted != 0), sweep_warp_smem_bytes(P, blur, !count), !count, n_ctas);
 }
 
 cudaError_t launch_sweep_warp(const FrameDev& F, const PmParams& P, const StateDev& prev, const StateDev& next,
-                              int iter, int phase, int n_ctas, int* err, cudaStream_t st, int shape)
+                              int iter, int phase, int n_ctas, int* err, cudaStream_t st)
 {
-    const bool blur = F.blur != nullptr, tex = uses_tex(F, P);
-    if (P.tap_counter) shape = 0;
-    const int smem = sweep_warp_smem_bytes(P, blur, shape, tex);
+    const bool blur = F.blur != nullptr, count = P.tap_counter != nullptr;
+    const int smem = sweep_warp_smem_bytes(P, blur, !count);
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     const int grid = std::max(1, std::min(n_ctas, F.V));
-    cudaError_t qe = cudaMemsetAsync(P.view_queue, 0, sizeof(int), st);
-    if (qe != cudaSuccess) return qe;
-    FrameDev f = F; PmParams p = P; StateDev a = prev, b = next; int it = iter, ph = phase; int* e = err;
-    void* args[] = { &f, &p, &a, &b, &it, &ph, &e };
-    return launch_k(warp_kernel(shape, blur, P.tap_counter != nullptr, P.shifted != 0, tex), grid,
-                    32 * sweep_shape_warps(shape), smem, shape, tex, st, args);
+    const void* k = warp_kernel(blur, count, P.shifted != 0);
+    cudaError_t e = cudaMemsetAsync(P.view_queue, 0, sizeof(int), st);
+    if (e == cudaSuccess) e = set_smem(k, smem, !count);
+    if (e != cudaSuccess) return e;
+    FrameDev f = F; PmParams p = P; StateDev a = prev, b = next; int it = iter, ph = phase; int* er = err;
+    void* args[] = { &f, &p, &a, &b, &it, &ph, &er };
+    return cudaLaunchKernel(k, dim3(grid), dim3(32 * kWarps), args, (size_t)smem, st);
 }
 
 // One thread per texel; a write outside a surface is dropped (boundary mode
@@ -1323,20 +1108,22 @@ cudaError_t launch_tex_fill(const uint8_t* tiles, int V, int W, int H, int tile_
     return cudaGetLastError();
 }
 
-cudaError_t sweep_batch_grid(int smem, bool blur, bool shift, bool tex, int* n_ctas, int shape)
+cudaError_t sweep_batch_grid(int smem, bool blur, bool shift, int* n_ctas)
 {
-    return grid_for(batch_kernel(shape, blur, shift, tex), 32 * sweep_shape_warps(shape), smem, shape, tex, n_ctas);
+    return grid_for(batch_kernel(blur, shift), smem, true, n_ctas);
 }
 
-cudaError_t launch_sweep_batch(const SweepItem* items, int n, bool blur, bool shift, bool tex, int smem, int n_ctas,
-                               int* err, cudaStream_t st, int shape)
+cudaError_t launch_sweep_batch(const SweepItem* items, int n, bool blur, bool shift, int smem, int n_ctas, int* err,
+                               cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
     if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
-    const SweepItem* it = items; int nn = n; int* e = err;
-    void* args[] = { &it, &nn, &e };
-    return launch_k(batch_kernel(shape, blur, shift, tex), dim3(std::max(1, n_ctas)), 32 * sweep_shape_warps(shape),
-                    smem, shape, tex, st, args);
+    const void* k = batch_kernel(blur, shift);
+    cudaError_t e = set_smem(k, smem, true);
+    if (e != cudaSuccess) return e;
+    const SweepItem* it = items; int nn = n; int* er = err;
+    void* args[] = { &it, &nn, &er };
+    return cudaLaunchKernel(k, dim3(std::max(1, n_ctas)), dim3(32 * kWarps), args, (size_t)smem, st);
 }
 
 }  // namespace pfd
