@@ -893,6 +893,19 @@ pfd_status pfd_frame_free(pfd_ctx* ctx, int frame_id)
     return PFD_OK;
 }
 
+// Enqueues the initialisation (refit: the post-refine pass) of state s.  Windows
+// and neighbour counts whose tap-counting plan exceeds shared memory are refused
+// with or without counting.
+static pfd_status init_state(pfd_ctx* ctx, const Frame& f, const pfd::PmParams& P, const pfd::StateDev& s, bool refit)
+{
+    if (!pfd::init_plan_fits(P, f.has_blur))
+        return fail(ctx, PFD_ECUDA, "initialisation: window %dx%d with %d neighbours does not fit shared memory", f.mi_w,
+                    f.mi_h, f.K);
+    if (P.tap_counter) CU(pfd::launch_init_count(frame_dev(f), P, s, ctx->d_err, ctx->stream, refit));
+    else CU(pfd::launch_init(frame_dev(f), P, s, ctx->d_err, ctx->stream, refit));
+    return PFD_OK;
+}
+
 pfd_status pfd_pm_init(pfd_ctx* ctx, int frame_id, const pfd_pm_params* params, uint64_t seed)
 {
     if (!ctx) return PFD_EINVAL;
@@ -905,7 +918,7 @@ pfd_status pfd_pm_init(pfd_ctx* ctx, int frame_id, const pfd_pm_params* params, 
     if (ctx->counting) P.tap_counter = ctx->d_taps;
     f->cur = 0;
     f->cvec_valid = 0;
-    CU(pfd::launch_init(frame_dev(*f), P, f->s[0], ctx->d_err, ctx->stream));
+    if ((st = init_state(ctx, *f, P, f->s[0], false)) != PFD_OK) return st;
     ctx->launches += 1;
     f->has_state = true;
     f->cvec_valid = 3u;
@@ -1444,7 +1457,7 @@ pfd_status pfd_acmm_post_refine(pfd_ctx* ctx, int frame_id, const pfd_pm_params*
     DeviceGuard g(ctx->device);
     pfd::PmParams P = make_params(ctx, *f, params, 0);
     if (ctx->counting) P.tap_counter = ctx->d_taps;
-    CU(pfd::launch_init(frame_dev(*f), P, f->s[f->cur], ctx->d_err, ctx->stream, true));
+    if ((st = init_state(ctx, *f, P, f->s[f->cur], true)) != PFD_OK) return st;
     ctx->launches += 1;
     // the pass stores every pixel's vector of its current plane
     f->cvec_valid = 3u;

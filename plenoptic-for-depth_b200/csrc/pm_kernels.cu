@@ -2,7 +2,8 @@
 //
 //   pm_slice_kernel   raw frame -> per-view micro-image tiles (Slice_RawMLAImage,
 //                     DepthSolver.cpp:1951-1997)
-//   pm_init_kernel    RandomInitializationForFrame (AdaptMIPMFrame.cu:474-518)
+//   pm_init_count_kernel  RandomInitializationForFrame (AdaptMIPMFrame.cu:474-518)
+//                     counting the NCC taps (calibration; pm_slots.cu otherwise)
 //   pm_ncc_kernel     per-hypothesis cost vectors (ComputeMultiViewCostVector_Frame)
 //
 // One CTA owns one reference micro-image (and a batch of its pixels).  Its own
@@ -200,14 +201,14 @@ __global__ void pm_slice_kernel(const uint8_t* raw, int raw_pitch, const int2* o
 }
 
 // --------------------------------------------------------------------------
-// RandomInitializationForFrame.  One thread per pixel; every lane of a warp
-// takes part in the warp-collective cost evaluation.
+// RandomInitializationForFrame, counting the in-bounds NCC taps.  One thread per
+// pixel; every lane of a warp takes part in the warp-collective cost evaluation.
 // --------------------------------------------------------------------------
 // With refit set, the pixel keeps its plane from out.plane and only its cost,
 // selected views and disp are recomputed: PostRefineMetadataFrame of the ACMM
 // matcher (AdaptMIPMFrameACMM.cu:903-929), which is the same top-k evaluation.
-template <bool BLUR, bool COUNT>
-__global__ void __launch_bounds__(256) pm_init_kernel(FrameDev F, PmParams P, StateDev out, int* err, int refit)
+template <bool BLUR>
+__global__ void __launch_bounds__(256) pm_init_count_kernel(FrameDev F, PmParams P, StateDev out, int* err, int refit)
 {
     extern __shared__ __align__(16) unsigned char smem[];
     const int vid = blockIdx.x;
@@ -227,7 +228,7 @@ __global__ void __launch_bounds__(256) pm_init_kernel(FrameDev F, PmParams P, St
     float4 h = make_float4(0.f, 0.f, 1.f, 0.f);
     if (act) h = refit ? out.plane[idx] : random_plane(g, P.depth_min, P.depth_max);
     float* cs = (float*)(smem + L.off_cost) + t;           // [k][npb]
-    cost_vector<BLUR, COUNT>(T, P, x, y, act, h, nc, cs, npb);
+    cost_vector<BLUR, true>(T, P, x, y, act, h, nc, cs, npb);
     if (!act) return;
 
     // ComputeSelectedViewsTopK_Frame (AdaptMIPMFrame.cu:227-282)
@@ -309,8 +310,15 @@ cudaError_t launch_slice(const uint8_t* raw, int raw_pitch, const int2* origin, 
     return cudaGetLastError();
 }
 
-cudaError_t launch_init(const FrameDev& F, const PmParams& P, const StateDev& out, int* err, cudaStream_t st,
-                        bool refit)
+// Whether the shared-memory plan of an initialisation with tap counting fits.
+bool init_plan_fits(const PmParams& P, bool blur)
+{
+    const int npb = P.ppv < 256 ? ((P.ppv + 31) / 32) * 32 : 256;
+    return SmemPlan::make(P.W, P.H, P.K, npb, P.ntap, blur, 1, false, P.tile_stride).total <= 227 * 1024;
+}
+
+cudaError_t launch_init_count(const FrameDev& F, const PmParams& P, const StateDev& out, int* err, cudaStream_t st,
+                              bool refit)
 {
     const bool blur = F.blur != nullptr;
     const int npb = P.ppv < 256 ? ((P.ppv + 31) / 32) * 32 : 256;
@@ -318,11 +326,8 @@ cudaError_t launch_init(const FrameDev& F, const PmParams& P, const StateDev& ou
     dim3 grid(F.V, (P.ppv + npb - 1) / npb);
     FrameDev f = F; PmParams p = P; StateDev o = out; int* e = err; int r = refit ? 1 : 0;
     void* args[] = { &f, &p, &o, &e, &r };
-    if (P.tap_counter)
-        return blur ? launch(pm_init_kernel<true, true>, grid, npb, smem, st, args)
-                    : launch(pm_init_kernel<false, true>, grid, npb, smem, st, args);
-    return blur ? launch(pm_init_kernel<true, false>, grid, npb, smem, st, args)
-                : launch(pm_init_kernel<false, false>, grid, npb, smem, st, args);
+    return blur ? launch(pm_init_count_kernel<true>, grid, npb, smem, st, args)
+                : launch(pm_init_count_kernel<false>, grid, npb, smem, st, args);
 }
 
 cudaError_t launch_ncc(const FrameDev& F, const PmParams& P, int nseg, int npb, const int* seg_vid, const int* seg_start,

@@ -16,6 +16,10 @@ cudaError_t launch_slice(const uint8_t* raw, int raw_pitch, const int2* origin, 
 // and disp (the ACMM matcher's post-refine pass).
 cudaError_t launch_init(const FrameDev& F, const PmParams& P, const StateDev& out, int* err, cudaStream_t st,
                         bool refit = false);
+// The same with the in-bounds taps counted into P.tap_counter.
+cudaError_t launch_init_count(const FrameDev& F, const PmParams& P, const StateDev& out, int* err, cudaStream_t st,
+                              bool refit);
+bool init_plan_fits(const PmParams& P, bool blur);
 cudaError_t launch_ncc(const FrameDev& F, const PmParams& P, int nseg, int npb, const int* seg_vid,
                        const int* seg_start, const int* seg_len, const int* hyp_pxy, const float4* hyp_plane,
                        const int* hyp_out, float* costs, int* err, cudaStream_t st);

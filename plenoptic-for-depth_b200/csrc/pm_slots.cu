@@ -386,6 +386,126 @@ __device__ __forceinline__ int rect_bin(uint32_t rect, int tx, int ty)
     return ((tx - 1) / 2 - bx) * ty + ((bx & 1) ? ry : ty - 1 - ry);
 }
 
+// ---- staging, shared by the half-sweep and the initialisation -------------------
+// Shared-memory arrays of the CTA's view.
+struct StageDst {
+    unsigned char* stage;    // 8-bit tiles of the view and its neighbours, filled by bulk copies
+    uint64_t* bar;
+    float* R;                // reference texels, column-major with stride rs
+    float* RB;               // reference blur / 255
+    uint32_t* Q;             // [K][H + 1][W + 1] quads
+    uint32_t* QB;
+    NbGeo* geo;
+    int* ok;
+    int rs;
+};
+
+// Thread 0 starts the bulk copies of view vid and its nc neighbours.  The threads'
+// accesses to the shared area before the last barrier are ordered before them.
+template <bool BLUR>
+__device__ __forceinline__ void start_copies(const StageDst& D, const FrameDev& F, const PmParams& P, int vid, int nc)
+{
+    const int ts = P.tile_stride;
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    mbar_arrive_expect_tx(D.bar, (uint32_t)((1 + nc) * ts * (BLUR ? 2 : 1)));
+    for (int i = 0; i < 1 + nc; ++i) {
+        const int v = (i == 0) ? vid : F.nb_ids[vid * P.K + i - 1];
+        const int vv = (v < 0 || v >= F.V) ? vid : v;
+        bulk_copy_g2s(D.stage + i * ts, F.gray + (size_t)vv * ts, (uint32_t)ts, D.bar);
+        if (BLUR) bulk_copy_g2s(D.stage + (1 + nc + i) * ts, F.blur + (size_t)vv * ts, (uint32_t)ts, D.bar);
+    }
+}
+
+// The neighbours' geometry; needs no copied tile.
+__device__ __forceinline__ void stage_geo(const StageDst& D, const FrameDev& F, const PmParams& P, int vid, int nc, int* err)
+{
+    const float2 c0 = F.centers[vid];
+    for (int k = threadIdx.x; k < P.K; k += blockDim.x) {
+        int v = (k < nc) ? F.nb_ids[vid * P.K + k] : -1;
+        if (v >= F.V) { atomicOr(err, PFD_DEVERR_SWEEP_CHECK); v = -1; }
+        D.ok[k] = (v >= 0);
+        D.geo[k] = make_geo(c0, F.centers[v >= 0 ? v : vid], P);
+    }
+}
+
+// The copied tiles as floats (reference) and quads (neighbours); between barriers.
+template <bool BLUR>
+__device__ __forceinline__ void expand_tiles(const StageDst& D, const PmParams& P, int nc)
+{
+    const int W = P.W, H = P.H, ts = P.tile_stride;
+    const uint8_t* stage = (const uint8_t*)D.stage;
+    for (int e = threadIdx.x; e < W * H; e += blockDim.x) {
+        const int ey = e / W, ex = e - ey * W;
+        D.R[ex * D.rs + ey] = (float)stage[e];
+        if (BLUR) D.RB[ex * D.rs + ey] = __fdiv_rn((float)stage[(1 + nc) * ts + e], 255.0f);
+    }
+    const int qs = W + 1, qn = (H + 1) * qs;
+    for (int e = threadIdx.x; e < nc * qn; e += blockDim.x) {
+        const int k = e / qn, r = e - k * qn;
+        const int iy = r / qs, ix = r - iy * qs;
+        const int y0 = min(iy, H - 1), y1 = min(iy + 1, H - 1);
+        const int x0 = min(ix, W - 1), x1 = min(ix + 1, W - 1);
+        const uint8_t* s = stage + (1 + k) * ts;
+        D.Q[e] = (uint32_t)s[y0 * W + x0] | ((uint32_t)s[y0 * W + x1] << 8) | ((uint32_t)s[y1 * W + x0] << 16) |
+                 ((uint32_t)s[y1 * W + x1] << 24);
+        if (BLUR) {
+            const uint8_t* sb = stage + (2 + nc + k) * ts;
+            D.QB[e] = (uint32_t)sb[y0 * W + x0] | ((uint32_t)sb[y0 * W + x1] << 8) | ((uint32_t)sb[y1 * W + x0] << 16) |
+                      ((uint32_t)sb[y1 * W + x1] << 24);
+        }
+    }
+}
+
+// The launch's weight tables (exponents of the spatial and the colour distance),
+// and zeros behind the reference texels.
+template <bool BLUR>
+__device__ __forceinline__ void fill_tables(const PmParams& P, float* a_s, float* a_c, float* R, float* RB, int rs)
+{
+    for (int t = threadIdx.x; t < P.ntap * P.ntap; t += blockDim.x) {
+        const float fi = (float)(-P.radius + (t / P.ntap) * P.inc);
+        const float fj = (float)(-P.radius + (t % P.ntap) * P.inc);
+        const float sd = __fsqrt_rn(__fmaf_rn(fj, fj, __fmul_rn(fi, fi)));
+        a_s[t] = __fdiv_rn(-sd, P.ss2);
+    }
+    for (int c = threadIdx.x; c < 256; c += blockDim.x) a_c[c] = __fdiv_rn((float)c, P.cc2);
+    for (int e = threadIdx.x; e < 2 * P.W * rs + 2 * P.H; e += blockDim.x) {
+        R[e] = 0.0f;
+        if (BLUR) RB[e] = 0.0f;
+    }
+}
+
+// Bilateral weight of window tap (ix, iy) of pixel (x, y) with centre texel rc.
+__device__ __forceinline__ float tap_weight(const float* R, int rs, const float* a_s, const float* a_c, const PmParams& P,
+                                            const PixWin& pw, int ix, int iy, float rc)
+{
+    const float rv = R[(pw.x0 + ix * P.inc) * rs + pw.y0 + iy * P.inc];
+    const float cd = fabsf(__fsub_rn(rv, rc));
+    const int cdi = __float_as_int(__fadd_rn(cd, 8388608.0f)) & 0xFF;
+    const int ti = (pw.ii0 + ix) * P.ntap + (pw.jj0 + iy);
+    return pfd_expf_nonpos(__fsub_rn(a_s[ti], a_c[cdi]));
+}
+
+// Bin counts to bin offsets (one warp).
+__device__ __forceinline__ void scan_bins(int* bins, int n, int lane)
+{
+    const int per = (n + 31) / 32;
+    int sum = 0;
+    for (int i = 0; i < per; ++i) {
+        const int b = lane * per + i;
+        if (b < n) sum += bins[b];
+    }
+    int off = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kFullMask, off, o);
+        if (lane >= o) off += t;
+    }
+    off -= sum;
+    for (int i = 0; i < per; ++i) {
+        const int b = lane * per + i;
+        if (b < n) { const int c = bins[b]; bins[b] = off; off += c; }
+    }
+}
+
 // ---- half-warp collectives -----------------------------------------------------
 struct Half {
     uint32_t mask;           // the half's lanes in the warp
@@ -530,11 +650,7 @@ __device__ __forceinline__ void begin_pixel(const Half& hf, const Slot& S, const
         const uint32_t magic = pw.nY > 1 ? 0xFFFFFFFFu / (uint32_t)pw.nY + 1u : 0u;
         for (int t = hl; t < n; t += 16) {
             const int ix = pw.nY > 1 ? (int)__umulhi((uint32_t)t, magic) : t, iy = t - ix * pw.nY;
-            const float rv = V.R[(pw.x0 + ix * P.inc) * V.rs + pw.y0 + iy * P.inc];
-            const float cd = fabsf(__fsub_rn(rv, rc));
-            const int cdi = __float_as_int(__fadd_rn(cd, 8388608.0f)) & 0xFF;
-            const int ti = (pw.ii0 + ix) * P.ntap + (pw.jj0 + iy);
-            S.wtab[t] = pfd_expf_nonpos(__fsub_rn(V.a_s[ti], V.a_c[cdi]));
+            S.wtab[t] = tap_weight(V.R, V.rs, V.a_s, V.a_c, P, pw, ix, iy, rc);
         }
     }
     const int a = hl & 7, dir = a >> 1;
@@ -965,23 +1081,18 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
     const float thr = __fmul_rn(0.8f, pfd_expf(__fdiv_rn((float)(iter * iter), -90.0f)));
     const float p_default = pfd_expf(__fdiv_rn(__fmul_rn(thr, thr), -0.32f));
 
-    // per-launch tables
-    {
-        float* a_s = (float*)(smem + L.off_as);
-        float* a_c = (float*)(smem + L.off_ac);
-        for (int t = tid; t < P.ntap * P.ntap; t += blockDim.x) {
-            const float fi = (float)(-P.radius + (t / P.ntap) * P.inc);
-            const float fj = (float)(-P.radius + (t % P.ntap) * P.inc);
-            const float sd = __fsqrt_rn(__fmaf_rn(fj, fj, __fmul_rn(fi, fi)));
-            a_s[t] = __fdiv_rn(-sd, P.ss2);
-        }
-        for (int c = tid; c < 256; c += blockDim.x) a_c[c] = __fdiv_rn((float)c, P.cc2);
-        for (int e = tid; e < 2 * W * L.rs + 2 * H; e += blockDim.x) {
-            R[e] = 0.0f;
-            if (BLUR) RB[e] = 0.0f;
-        }
-        for (int e = tid; e < L.nbins; e += blockDim.x) bins[e] = 0;
-    }
+    fill_tables<BLUR>(P, (float*)(smem + L.off_as), (float*)(smem + L.off_ac), R, RB, L.rs);
+    for (int e = tid; e < L.nbins; e += blockDim.x) bins[e] = 0;
+    StageDst D;
+    D.stage = smem + L.off_stage;
+    D.bar = (uint64_t*)smem;
+    D.R = R;
+    D.RB = RB;
+    D.Q = (uint32_t*)(smem + L.off_Q);
+    D.QB = (uint32_t*)(smem + L.off_QB);
+    D.geo = geo;
+    D.ok = okk;
+    D.rs = L.rs;
     EvalEnv E;
     E.wtab = smem_u32(smem + L.off_wtab);
     E.R = smem_u32(R);
@@ -1020,20 +1131,7 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
         V.vid = vid;
         V.nc = nc;
         V.vbase = vbase;
-        if (nc > 0 && tid == 0) {
-            // bulk copies of the 8-bit tiles; the threads' accesses to the shared area before
-            // the last barrier are ordered before them
-            uint8_t* stage = (uint8_t*)(smem + L.off_stage);
-            uint64_t* bar = (uint64_t*)smem;
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_arrive_expect_tx(bar, (uint32_t)((1 + nc) * ts * (BLUR ? 2 : 1)));
-            for (int i = 0; i < 1 + nc; ++i) {
-                const int v = (i == 0) ? vid : F.nb_ids[vid * K + i - 1];
-                const int vv = (v < 0 || v >= F.V) ? vid : v;
-                bulk_copy_g2s(stage + i * ts, F.gray + (size_t)vv * ts, (uint32_t)ts, bar);
-                if (BLUR) bulk_copy_g2s(stage + (1 + nc + i) * ts, F.blur + (size_t)vv * ts, (uint32_t)ts, bar);
-            }
-        }
+        if (nc > 0 && tid == 0) start_copies<BLUR>(D, F, P, vid, nc);
         // the other colour keeps its state; so does every pixel of a view without neighbours
         for (int e = tid; e < P.ppv; e += blockDim.x) {
             const int ey = e / W, ex = e - ey * W;
@@ -1048,13 +1146,7 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
             next.sel[vbase + e] = sv;
         }
         if (nc <= 0) continue;
-        const float2 c0 = F.centers[vid];
-        for (int k = tid; k < K; k += blockDim.x) {
-            int v = (k < nc) ? F.nb_ids[vid * K + k] : -1;
-            if (v >= F.V) { atomicOr(err, PFD_DEVERR_SWEEP_CHECK); v = -1; }
-            okk[k] = (v >= 0);
-            geo[k] = make_geo(c0, F.centers[v >= 0 ? v : vid], P);
-        }
+        stage_geo(D, F, P, vid, nc, err);
         if (tid == 0) {
             ctl[kCtlPixel] = g_lo;
             ctl[kCtlTasks] = 0;
@@ -1062,31 +1154,8 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
         const bool ok = mbar_wait_bounded((uint64_t*)smem, parity, err);
         if (__syncthreads_or(!ok)) return false;
         parity ^= 1u;
-        {
-            const uint8_t* stage = (const uint8_t*)(smem + L.off_stage);
-            for (int e = tid; e < W * H; e += blockDim.x) {
-                const int ey = e / W, ex = e - ey * W;
-                R[ex * L.rs + ey] = (float)stage[e];
-                if (BLUR) RB[ex * L.rs + ey] = __fdiv_rn((float)stage[(1 + nc) * ts + e], 255.0f);
-            }
-            const int qs = W + 1, qn = (H + 1) * qs;
-            uint32_t* Q = (uint32_t*)(smem + L.off_Q);
-            uint32_t* QB = (uint32_t*)(smem + L.off_QB);
-            for (int e = tid; e < nc * qn; e += blockDim.x) {
-                const int k = e / qn, r = e - k * qn;
-                const int iy = r / qs, ix = r - iy * qs;
-                const int y0 = min(iy, H - 1), y1 = min(iy + 1, H - 1);
-                const int x0 = min(ix, W - 1), x1 = min(ix + 1, W - 1);
-                const uint8_t* s = stage + (1 + k) * ts;
-                Q[e] = (uint32_t)s[y0 * W + x0] | ((uint32_t)s[y0 * W + x1] << 8) | ((uint32_t)s[y1 * W + x0] << 16) |
-                       ((uint32_t)s[y1 * W + x1] << 24);
-                if (BLUR) {
-                    const uint8_t* sb = stage + (2 + nc + k) * ts;
-                    QB[e] = (uint32_t)sb[y0 * W + x0] | ((uint32_t)sb[y0 * W + x1] << 8) |
-                            ((uint32_t)sb[y1 * W + x0] << 16) | ((uint32_t)sb[y1 * W + x1] << 24);
-                }
-            }
-        }
+        expand_tiles<BLUR>(D, P, nc);
+        __syncthreads();
         // stage of every slot; a slot whose request did not fit the list keeps it (kWaits set)
         if (tid < 32) { stages[tid] = tid < n_slots ? kNew : kIdle; next_stages[tid] = kIdle; }
         __syncthreads();
@@ -1209,22 +1278,7 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
             // ---- sort by rectangle: bin offsets, then the order
             const int n_tasks = ctl[kCtlTasks];
             if (warp == 0) {
-                const int per = (L.nbins + 31) / 32;
-                int sum = 0;
-                for (int i = 0; i < per; ++i) {
-                    const int b = lane * per + i;
-                    if (b < L.nbins) sum += bins[b];
-                }
-                int off = sum;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(kFullMask, off, o);
-                    if (lane >= o) off += t;
-                }
-                off -= sum;
-                for (int i = 0; i < per; ++i) {
-                    const int b = lane * per + i;
-                    if (b < L.nbins) { const int c = bins[b]; bins[b] = off; off += c; }
-                }
+                scan_bins(bins, L.nbins, lane);
                 if (lane == 0) ctl[kCtlPass] = 0;
             }
             __syncthreads();
@@ -1275,6 +1329,284 @@ __device__ __forceinline__ void init_barrier(unsigned char* smem)
     __syncthreads();
 }
 
+// ---- initialisation --------------------------------------------------------------
+// RandomInitializationForFrame (AdaptMIPMFrame.cu:474-518): a random plane per
+// pixel, its cost vector, and from it the stored cost, views and disp
+// (ComputeSelectedViewsTopK_Frame, :227-282).  A CTA takes a micro-image and runs
+// its pixels in chunks: the chunk's weight tables and planes, one list of all its
+// (pixel, neighbour) NCCs sorted by tap rectangle and evaluated 32 at a time as in
+// the half-sweep, then one thread per pixel for the views.  With refit set a pixel
+// keeps its plane (PostRefineMetadataFrame, AdaptMIPMFrameACMM.cu:903-929).
+// Bound by instruction issue, as the half-sweep.  Against one thread per pixel
+// over chunks of neighbours (the lanes' windows and taps differ, IEEE divisions per
+// blur tap): 16.0 -> 4.2 ms (2048x1536, 12 neighbours, 15x15), 51.8 -> 3.6 ms
+// (1531x1147, 17, 13x13, blur, shifted), 1.78 -> 0.58 ms (1024x768, 6, 11x11).
+namespace {
+
+constexpr int kInitWarps = 16, kInitCtas = 2;
+
+struct InitPlan {
+    int off_ctl, off_Q, off_QB, off_R, off_RB, off_geo, off_ok, off_as, off_ac, off_bins;
+    int off_stage, off_wtab, off_plane, off_dp, off_cost, off_id, off_order;
+    int rs, tx, ty, tab_n, nbins, kc, total;
+
+    __host__ __device__ static int a16(int v) { return (v + 15) & ~15; }
+    __host__ __device__ static InitPlan make(int W, int H, int K, int ntap, bool blur, int tile_stride, int chunk)
+    {
+        InitPlan p;
+        p.rs = H | 1;
+        p.tx = ntap < W ? ntap : W;
+        p.ty = ntap < H ? ntap : H;
+        p.tab_n = p.tx * p.ty;
+        p.nbins = (p.tx / 2 + 1) * p.ty;
+        p.kc = K | 1;                                    // odd: threads read rows side by side
+        int o = 16;
+        p.off_ctl = o;   o += 16;
+        const int q_bytes = a16(K * (H + 1) * (W + 1) * 4), r_bytes = a16((2 * W * p.rs + 2 * H) * 4);
+        p.off_Q = o;     o += q_bytes;
+        p.off_QB = o;    o += blur ? q_bytes : 0;
+        p.off_R = o;     o += r_bytes;
+        p.off_RB = o;    o += blur ? r_bytes : 0;
+        p.off_geo = o;   o += a16(K * (int)sizeof(NbGeo));
+        p.off_ok = o;    o += a16(K * 4);
+        p.off_as = o;    o += a16(ntap * ntap * 4);
+        p.off_ac = o;    o += 256 * 4;
+        p.off_bins = o;  o += a16(p.nbins * 4);
+        p.off_stage = o;                                 // shares what follows, as in the half-sweep
+        const int stage_end = o + a16((1 + K) * tile_stride * (blur ? 2 : 1));
+        p.off_wtab = o;  o += a16(chunk * p.tab_n * 4);
+        p.off_plane = o; o += chunk * 16;
+        p.off_dp = o;    o += chunk * 16;
+        p.off_cost = o;  o += a16(chunk * p.kc * 4);
+        p.off_id = o;    o += a16(chunk * K * 2);
+        p.off_order = o; o += a16(chunk * K * 2);
+        const int walk_end = p.off_wtab + (chunk + 1) * p.tab_n * 4 + 64;
+        if (o < stage_end) o = stage_end;
+        if (o < walk_end) o = a16(walk_end);
+        p.total = o;
+        return p;
+    }
+};
+
+}  // namespace
+
+template <bool BLUR, bool SHIFT>
+__global__ void __launch_bounds__(32 * kInitWarps, kInitCtas)
+pm_init_kernel(FrameDev F, PmParams P, StateDev out, int* err, int refit, int chunk, int parts)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int W = P.W, H = P.H, K = P.K;
+    const InitPlan L = InitPlan::make(W, H, K, P.ntap, BLUR, P.tile_stride, chunk);
+    {
+        uint32_t dyn;
+        asm volatile("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn));
+        if (L.total > (int)dyn || chunk < 1 || chunk * 32 > 65536 || parts < 1) {
+            if (threadIdx.x == 0) atomicOr(err, PFD_DEVERR_SWEEP_CHECK);
+            return;
+        }
+    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
+    int* ctl = (int*)(smem + L.off_ctl);                 // 0: tasks, 1: next pass
+    float* R = (float*)(smem + L.off_R);
+    int* bins = (int*)(smem + L.off_bins);
+    const float* a_s = (const float*)(smem + L.off_as);
+    const float* a_c = (const float*)(smem + L.off_ac);
+    float* wtab = (float*)(smem + L.off_wtab);
+    float4* plane = (float4*)(smem + L.off_plane);
+    float4* dps = (float4*)(smem + L.off_dp);
+    float* cost = (float*)(smem + L.off_cost);
+    uint16_t* t_id = (uint16_t*)(smem + L.off_id);
+    uint16_t* t_order = (uint16_t*)(smem + L.off_order);
+    StageDst D;
+    D.stage = smem + L.off_stage;
+    D.bar = (uint64_t*)smem;
+    D.R = R;
+    D.RB = (float*)(smem + L.off_RB);
+    D.Q = (uint32_t*)(smem + L.off_Q);
+    D.QB = (uint32_t*)(smem + L.off_QB);
+    D.geo = (NbGeo*)(smem + L.off_geo);
+    D.ok = (int*)(smem + L.off_ok);
+    D.rs = L.rs;
+    EvalEnv E;
+    E.wtab = smem_u32(wtab);
+    E.R = smem_u32(R);
+    E.RB_delta = BLUR ? (uint32_t)(L.off_RB - L.off_R) : 0u;
+    E.Q = smem_u32(D.Q);
+    E.QB_delta = BLUR ? (uint32_t)(L.off_QB - L.off_Q) : 0u;
+    E.q_bytes = (H + 1) * (W + 1) * 4;
+    E.tab_n = L.tab_n;
+    E.rs = L.rs;
+    E.inc = P.inc;
+    E.wb = P.W_bits;
+    E.hb = P.H_bits;
+    E.kq = ((uint32_t)(W + 1) * 4u << 24) | (4u << 16);
+    const float inv_inc = 1.0f / (float)P.inc;
+    if (tid == 0) mbar_init(D.bar, 1);
+    fill_tables<BLUR>(P, (float*)(smem + L.off_as), (float*)(smem + L.off_ac), R, D.RB, L.rs);
+    for (int e = tid; e < L.nbins; e += blockDim.x) bins[e] = 0;
+    uint32_t parity = 0;
+    for (int item = blockIdx.x; item < F.V * parts; item += gridDim.x) {
+        const int vid = item / parts, part = item - vid * parts;
+        const int p_lo = (int)((long long)P.ppv * part / parts), p_hi = (int)((long long)P.ppv * (part + 1) / parts);
+        const int nc = min(F.nb_counts[vid], K);
+        const size_t vbase = (size_t)vid * P.ppv;
+        __syncthreads();                                 // the previous item's shared memory is free
+        if (tid == 0) {
+            start_copies<BLUR>(D, F, P, vid, nc > 0 ? nc : 0);
+            ctl[0] = 0;
+        }
+        stage_geo(D, F, P, vid, nc, err);
+        const bool ok = mbar_wait_bounded(D.bar, parity, err);
+        if (__syncthreads_or(!ok)) return;
+        parity ^= 1u;
+        expand_tiles<BLUR>(D, P, nc > 0 ? nc : 0);
+        __syncthreads();
+        for (int e0 = p_lo; e0 < p_hi; e0 += chunk) {
+            const int np = min(chunk, p_hi - e0);
+            // ---- planes, weight tables
+            for (int p = tid; p < np; p += blockDim.x) {
+                const int e = e0 + p, y = e / W, x = e - y * W;
+                const size_t idx = vbase + e;
+                float4 h;
+                if (refit) {
+                    h = out.plane[idx];
+                } else {
+                    DrawStream g;
+                    g.init(P.seed, 0u, (uint32_t)idx);
+                    h = random_plane(g, P.depth_min, P.depth_max);
+                }
+                plane[p] = h;
+                const float3 dp = disparity_plane(x, y, h);
+                dps[p] = make_float4(dp.x, dp.y, dp.z, to_disparity(x, y, dp));
+            }
+            for (int p = warp; p < np; p += kInitWarps) {
+                const int e = e0 + p, y = e / W, x = e - y * W;
+                const PixWin pw = slot_window(P, x, y);
+                const float rc = R[x * L.rs + y];
+                const int n = pw.nX * pw.nY;
+                const uint32_t magic = pw.nY > 1 ? 0xFFFFFFFFu / (uint32_t)pw.nY + 1u : 0u;
+                for (int t = lane; t < n; t += 32) {
+                    const int ix = pw.nY > 1 ? (int)__umulhi((uint32_t)t, magic) : t, iy = t - ix * pw.nY;
+                    wtab[p * L.tab_n + t] = tap_weight(R, L.rs, a_s, a_c, P, pw, ix, iy, rc);
+                }
+            }
+            __syncthreads();
+            // ---- the NCCs of the chunk, sorted by rectangle
+            const int total = np * nc;
+            for (int i0 = warp * 32; i0 < total; i0 += 32 * kInitWarps) {
+                const int i = i0 + lane;
+                const int p = i / nc, k = i - p * nc;
+                uint32_t rect = 0u;
+                if (i < total) {
+                    const int e = e0 + p, y = e / W, x = e - y * W;
+                    if (D.ok[k]) {
+                        const float4 d = dps[p];
+                        const NbGeo g = D.geo[k];
+                        const float2 a = geo_anchor(g, x, y, d.w);
+                        if ((__float_as_uint(a.x) < P.W_bits) && (__float_as_uint(a.y) < P.H_bits))
+                            rect = tap_rect(slot_window(P, x, y), P, make_float3(d.x, d.y, d.z), g.stx, g.sty, inv_inc);
+                    }
+                    cost[p * L.kc + k] = rect ? __uint_as_float(rect) : kCostMax;
+                }
+                const uint32_t m = __ballot_sync(kFullMask, rect != 0u);
+                if (!m) continue;
+                int at = 0;
+                if (lane == 0) at = atomicAdd(&ctl[0], __popc(m));
+                at = __shfl_sync(kFullMask, at, 0) + __popc(m & ((1u << lane) - 1u));
+                if (rect) {
+                    t_id[at] = (uint16_t)((p << 5) | k);
+                    atomicAdd(&bins[rect_bin(rect, L.tx, L.ty)], 1);
+                }
+            }
+            __syncthreads();
+            const int n_tasks = ctl[0];
+            if (warp == 0) {
+                scan_bins(bins, L.nbins, lane);
+                if (lane == 0) ctl[1] = 0;
+            }
+            __syncthreads();
+            for (int i = tid; i < n_tasks; i += blockDim.x) {
+                const int id = t_id[i];
+                const uint32_t rect = __float_as_uint(cost[(id >> 5) * L.kc + (id & 31)]);
+                t_order[atomicAdd(&bins[rect_bin(rect, L.tx, L.ty)], 1)] = (uint16_t)id;
+            }
+            __syncthreads();
+            for (int e = tid; e < L.nbins; e += blockDim.x) bins[e] = 0;
+            if (tid == 0) ctl[0] = 0;
+            for (;;) {
+                int q = 0;
+                if (lane == 0) q = atomicAdd(&ctl[1], 1);
+                q = __shfl_sync(kFullMask, q, 0);
+                if (q * 32 >= n_tasks) break;
+                const bool act = q * 32 + lane < n_tasks;
+                const int id = act ? t_order[q * 32 + lane] : 0;
+                const int p = id >> 5, k = id & 31;
+                const int e = e0 + p, y = e / W, x = e - y * W;
+                float* cell = cost + p * L.kc + k;
+                const uint32_t rect = act ? __float_as_uint(*cell) : 0u;
+                const float4 d = dps[p];
+                const PixWin pw = slot_window(P, x, y);
+                const int i0 = rect & 0xFF, j0 = (rect >> 8) & 0xFF;
+                const int X = pw.x0 + i0 * P.inc, Y = pw.y0 + j0 * P.inc;
+                Moments M = { 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f };
+                const float sh = SHIFT ? R[x * L.rs + y] : 0.0f;
+                walk<BLUR, SHIFT>(M, E, make_float3(d.x, d.y, d.z), D.geo[k].stx, D.geo[k].sty,
+                                  (int)((rect >> 16) & 0xFFu), (int)(rect >> 24),
+                                  E.wtab + (uint32_t)(p * L.tab_n + i0 * pw.nY + j0) * 4u,
+                                  E.R + (uint32_t)(X * L.rs + Y) * 4u, (uint32_t)pw.nY * 4u, (float)X, (float)Y,
+                                  E.Q + (uint32_t)(k * E.q_bytes), sh);
+                if (act) *cell = ncc_cost<BLUR>(M, P.blur_gain);
+            }
+            __syncthreads();
+            // ---- the pixel's cost, views and disp: the top-k of its vector
+            for (int p = tid; p < np; p += blockDim.x) {
+                const int e = e0 + p, y = e / W, x = e - y * W;
+                const size_t idx = vbase + e;
+                const float* cs = cost + p * L.kc;
+                int best_idx = -1, valid = 0;
+                for (int i = 0; i < nc; ++i) {
+                    const float c = cs[i];
+                    if (c < 2.0f) {
+                        ++valid;
+                        if (best_idx < 0 || c < cs[best_idx]) best_idx = i;
+                    }
+                }
+                float mean = 2.0f;
+                uint32_t mask = 0;
+                if (valid > 0) {
+                    // the k smallest in ascending order
+                    const int kk = min(valid, P.top_k);
+                    uint32_t used = 0;
+                    float m = 0.0f, low = 0.0f;
+                    for (int i = 0; i < kk; ++i) {
+                        int at = -1;
+                        for (int j = 0; j < nc; ++j)
+                            if (!((used >> j) & 1u) && (at < 0 || cs[j] < low)) { at = j; low = cs[j]; }
+                        used |= 1u << at;
+                        m = __fadd_rn(m, low);
+                    }
+                    mean = __fdiv_rn(m, (float)kk);
+                    for (int i = 0; i < nc; ++i)
+                        if (cs[i] <= low) mask |= (1u << i);
+                }
+                const float4 h = plane[p];
+                float4 disp = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (best_idx >= 0) disp = geo_disp(D.geo[best_idx], x, y, to_disparity(x, y, disparity_plane(x, y, h)));
+                if (!refit) out.plane[idx] = h;
+                out.cost[idx] = mean;
+                out.disp[idx] = disp;
+                out.sel[idx] = mask;
+            }
+            if (P.cvec)
+                for (int i = tid; i < total; i += blockDim.x) {
+                    const int p = i / nc, k = i - p * nc;
+                    P.cvec[(vbase + e0 + p) * K + k] = cost[p * L.kc + k];
+                }
+            __syncthreads();                             // the chunk's planes and costs are free
+        }
+    }
+}
+
 template <bool BLUR, bool SHIFT, int SHAPE>
 __global__ void __launch_bounds__(32 * ShapeOf<SHAPE>::warps, ShapeOf<SHAPE>::min_ctas)
 pm_slots_kernel(FrameDev F, PmParams P, StateDev prev, StateDev next, int iter, int phase, int* err)
@@ -1302,6 +1634,44 @@ pm_slots_batch_kernel(const SweepItem* items, int n, int* err)
                                                              parity))
             return;
     }
+}
+
+cudaError_t launch_init(const FrameDev& F, const PmParams& P, const StateDev& out, int* err, cudaStream_t st, bool refit)
+{
+    const bool blur = F.blur != nullptr;
+    if (F.V <= 0) return cudaSuccess;
+    // chunk: the pixels whose tables fit two CTAs per SM, or one
+    int chunk = 0, smem = 0;
+    for (int ctas = kInitCtas; ctas >= 1 && !smem; --ctas) {
+        const int budget = std::min(227 * 1024, (228 * 1024) / ctas - 1024);
+        for (int c = std::min(128, P.ppv); c >= 1; --c) {
+            if (ctas > 1 && c < std::min(32, P.ppv)) break;
+            const InitPlan L = InitPlan::make(P.W, P.H, P.K, P.ntap, blur, P.tile_stride, c);
+            if (L.total > budget) continue;
+            chunk = c;
+            smem = L.total;
+            break;
+        }
+    }
+    if (!smem) return cudaErrorInvalidValue;
+    const int chunks = (P.ppv + chunk - 1) / chunk;
+    chunk = (P.ppv + chunks - 1) / chunks;               // equal chunks
+    const void* k = P.shifted ? (blur ? (const void*)pm_init_kernel<true, true> : (const void*)pm_init_kernel<false, true>)
+                              : (blur ? (const void*)pm_init_kernel<true, false> : (const void*)pm_init_kernel<false, false>);
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kInitWarps, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    // a frame of few micro-images splits them by chunks, so that every SM has work
+    int parts = 1;
+    while (parts < chunks && (long long)F.V * parts < 4LL * sms * per_sm) parts = std::min(chunks, parts * 2);
+    const int grid = (int)std::min<long long>((long long)sms * per_sm, (long long)F.V * parts);
+    FrameDev f = F; PmParams p = P; StateDev o = out; int* er = err; int r = refit ? 1 : 0;
+    void* args[] = { &f, &p, &o, &er, &r, &chunk, &parts };
+    return cudaLaunchKernel(k, dim3(grid), dim3(32 * kInitWarps), args, (size_t)smem, st);
 }
 
 int slots_shape_warps(int shape) { return kShapeWarps[(shape >= 0 && shape < kSweepShapes) ? shape : 0]; }
