@@ -6,10 +6,31 @@
 // The filter invalidates rejected pixels in place and walks the micro-images
 // in key order, so a later micro-image reads the already filtered state of
 // earlier neighbours (FilterGlobal, :962-986).  The device keeps exactly that
-// dependency: micro-image (col, row) runs in wavefront step col + c * row, with
-// c chosen on the host so that every neighbour earlier in key order falls in
-// an earlier step and every later one in a later step.  Micro-images of one
-// step are never neighbours of each other and run in parallel.
+// dependency, in three launches:
+//   pm_filter_pairs_kernel    every (pixel, view) test on the unfiltered state.
+//                             What an earlier neighbour's filtering can change is
+//                             only whether one of the four pixels a test reads has
+//                             been rejected (then the view gives no support), so a
+//                             test against an earlier neighbour is kept as (view,
+//                             pixel, passed) and one against a later neighbour is
+//                             final.
+//   pm_filter_resolve_kernel  the rejected pixels of every micro-image as a bit
+//                             mask, from its earlier neighbours' masks, repeated
+//                             for the micro-images whose earlier neighbours changed
+//                             until nothing changes: key order has no cycles, so
+//                             this ends at the one solution, the sequential walk's.
+//                             A cooperative launch; the grid barrier's waits are
+//                             bounded.
+//   pm_filter_apply_kernel    reasons, counters and the rejected pixels' state.
+// A rejected pixel gets disparity -1; where the configuration accepts such a
+// disparity (min_valid_disp < -1) it is not an unusable one, and the filter runs as
+// a wavefront instead (pm_filter_kernel): micro-image (col, row) in step
+// col + c * row, with c chosen on the host so that every neighbour earlier in key
+// order falls in an earlier step and every later one in a later step.
+//
+// The wavefront was bound by the latency of its steps (779 launches of 22 us on the
+// 4080x3068 frame, 34 micro-images each): 17.5 ms, now 1.7 ms (1024x768: 2.74 and
+// 0.18 ms), bound by the gathers of the pairs kernel.
 //
 // Arithmetic is the reference's expressions evaluated as written, one
 // rounding per operation (the library is built with -fmad=false), matching the
@@ -291,6 +312,339 @@ __global__ void pm_filter_kernel(CheckFrame F, FilterCfg cfg, StateDev st, const
         __syncthreads();
         if (threadIdx.x < 8 && stats) atomicAdd(&stats[threadIdx.x], cnt[threadIdx.x]);
         __syncthreads();
+    }
+}
+
+// ---- the filter in three launches -----------------------------------------------
+namespace {
+
+// FilterWork::head of a pixel: what its own state decides, and the counts that are final.
+constexpr uint32_t kHeadInvalid = 0u, kHeadCost = 1u, kHeadNoViews = 2u, kHeadOpen = 3u;
+__device__ __forceinline__ uint32_t make_head(uint32_t cls, int support, int good, int n)
+{
+    return cls | ((uint32_t)support << 2) | ((uint32_t)good << 8) | ((uint32_t)n << 14);
+}
+
+// Bytes -> floats of the view's tile and of its neighbours' tiles (as bytes).
+__device__ __forceinline__ float bilinear_u8(const uint8_t* img, int W, int H, float x, float y)
+{
+    const int x0 = (int)floorf(x), y0 = (int)floorf(y);
+    const int x1 = min(x0 + 1, W - 1), y1 = min(y0 + 1, H - 1);
+    const float ax = x - (float)x0, ay = y - (float)y0;
+    const float v00 = (float)img[y0 * W + x0], v01 = (float)img[y1 * W + x0];
+    const float v10 = (float)img[y0 * W + x1], v11 = (float)img[y1 * W + x1];
+    float s = ((1.0f - ax) * (1.0f - ay)) * v00;
+    s = s + ((1.0f - ax) * ay) * v01;
+    s = s + (ax * (1.0f - ay)) * v10;
+    s = s + (ax * ay) * v11;
+    return s;
+}
+
+// cv::meanStdDev of the 3x3 window centred on (cx, cy): the sums are integers, so
+// they are the double sums exactly.
+__device__ __forceinline__ bool patch_mean_std_u8(const uint8_t* img, int W, int H, int cx, int cy, float& m, float& s)
+{
+    if (cx < 1 || cy < 1 || cx >= W - 1 || cy >= H - 1) return false;
+    int sum = 0, sq = 0;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx) {
+            const int v = img[(cy + dy) * W + cx + dx];
+            sum += v;
+            sq += v * v;
+        }
+    const double scale = 1.0 / 9.0;
+    const double ds = (double)sum * scale;
+    double var = (double)sq * scale - ds * ds;
+    if (var < 0.0) var = 0.0;
+    m = (float)ds;
+    s = (float)sqrt(var);
+    return isfinite(m) && isfinite(s) && s > 1.0e-3f;
+}
+
+__device__ __forceinline__ bool key_before(int2 a, int2 b) { return a.y < b.y || (a.y == b.y && a.x < b.x); }
+
+}  // namespace
+
+__global__ void __launch_bounds__(256) pm_filter_pairs_kernel(CheckFrame F, FilterCfg cfg, StateDev st, FilterWork X)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int W = F.W, H = F.H, N = W * H, v = blockIdx.x;
+    const int nc = min(F.nb_counts[v], F.K);
+    uint8_t* tiles = smem;                               // [1 + K][tile_stride]: the view, its neighbours
+    NbDir* dir = (NbDir*)(smem + (size_t)(1 + F.K) * F.tile_stride);     // [K]
+    int* ids = (int*)(dir + F.K);                        // [K] neighbour, -1 unusable; bit 30: earlier in key order
+    const int words = F.tile_stride >> 4;
+    for (int e = threadIdx.x; e < (1 + nc) * words; e += blockDim.x) {
+        const int t = e / words;
+        const int u = t == 0 ? v : F.nb_ids[v * F.K + t - 1];
+        if (u >= 0) ((uint4*)tiles)[e] = ((const uint4*)(F.gray + (size_t)u * F.tile_stride))[e - t * words];
+    }
+    for (int k = threadIdx.x; k < nc; k += blockDim.x) {
+        const int u = F.nb_ids[v * F.K + k];
+        int id = -1;
+        if (u >= 0) {
+            dir[k] = neighbour_dir(F.centers[v], F.centers[u], F.baseline_unit);
+            if (dir[k].ok) id = u | (key_before(F.keys[u], F.keys[v]) ? 1 << 30 : 0);
+        }
+        ids[k] = id;
+    }
+    __syncthreads();
+    const size_t base = (size_t)v * N;
+    for (int idx = threadIdx.x; idx < N; idx += blockDim.x) {
+        const int x = idx % W, y = idx / W;
+        const float d = st.plane[base + idx].w;
+        uint32_t cls = kHeadInvalid;
+        int support = 0, good = 0, n = 0;
+        if (isfinite(d) && d > cfg.min_valid_disp) {
+            uint32_t mask = cfg.use_selected_views_only ? st.sel[base + idx] : (nc < 32 ? (1u << nc) - 1u : ~0u);
+            if (!cost_ok(st.cost[base + idx], cfg)) {
+                cls = kHeadCost;
+            } else if (mask == 0u || cfg.max_triplet <= 0) {
+                cls = kHeadNoViews;
+            } else {
+                cls = kHeadOpen;
+                const float px = (float)x, py = (float)y;
+                const float Ir = (float)tiles[idx];
+                float mr = 0.0f, sr = 0.0f;
+                const bool ref_ok = cfg.enable_cycle_photo_filter && patch_mean_std_u8(tiles, W, H, x, y, mr, sr);
+                for (int t = 0; mask && t < cfg.max_triplet; ++t) {
+                    const int b = __ffs(mask) - 1;
+                    mask &= mask - 1;
+                    if (b >= nc) continue;
+                    const int id = ids[b];
+                    if (id < 0) continue;
+                    const NbDir g = dir[b];
+                    const float qx = px + (g.dx * d) * g.scale;
+                    const float qy = py + (g.dy * d) * g.scale;
+                    if (qx < 0 || qy < 0 || qx > W - 1 || qy > H - 1) continue;
+                    const size_t nbase = (size_t)(id & ~(1 << 30)) * N;
+                    const float d_nei = bilinear_disp(st.plane + nbase, W, H, qx, qy, cfg.min_valid_disp);
+                    if (!isfinite(d_nei)) continue;
+                    if (cfg.enable_cost_filter && !cost_ok(bilinear_cost(st.cost + nbase, W, H, qx, qy), cfg)) continue;
+                    bool pass = true;
+                    if (cfg.enable_cycle_geo_filter) {
+                        const float phx = qx - (g.dx * d_nei) * g.scale;
+                        const float phy = qy - (g.dy * d_nei) * g.scale;
+                        const float ge = hypot_canon(phx - px, phy - py);
+                        pass = isfinite(ge) && ge <= cfg.max_geo_err_px;
+                    }
+                    if (pass && cfg.enable_cycle_photo_filter) {
+                        // ComputePhotoResidual, MIDisparityFilter.cpp:138-156 (the pixel is on the grid)
+                        const uint8_t* nei = tiles + (size_t)(1 + b) * F.tile_stride;
+                        const float In = bilinear_u8(nei, W, H, qx, qy);
+                        float mn, sn, pe;
+                        if (ref_ok && patch_mean_std_u8(nei, W, H, (int)roundf(qx), (int)roundf(qy), mn, sn))
+                            pe = fabsf((Ir - mr) / sr - (In - mn) / sn);
+                        else
+                            pe = fabsf(In - Ir);
+                        pass = isfinite(pe) && pe <= cfg.max_photo_err_u;
+                    }
+                    if (id & (1 << 30)) {
+                        X.ent[(size_t)n * X.total + base + idx] =
+                            (uint16_t)(b | ((int)floorf(qx) << 5) | ((int)floorf(qy) << 10) | (pass ? 1 << 15 : 0));
+                        ++n;
+                    } else {
+                        ++support;
+                        good += pass;
+                    }
+                }
+            }
+        }
+        X.head[base + idx] = make_head(cls, support, good, n);
+        X.disp[base + idx] = d;
+    }
+}
+
+namespace {
+
+// One view's tests under the masks of its earlier neighbours: per pixel the reject
+// reason (smem why[N]; kPrKeep for a pixel that stays or was never valid).  Ends
+// with a barrier.
+__device__ __forceinline__ void eval_view(const CheckFrame& F, const FilterCfg& cfg, const FilterWork& X, int v,
+                                          uint32_t* nmask, float* dv, uint8_t* keep, uint8_t* why)
+{
+    const int W = F.W, H = F.H, N = W * H, mw = X.mask_words;
+    const int nc = min(F.nb_counts[v], F.K);
+    const size_t base = (size_t)v * N;
+    for (int e = threadIdx.x; e < nc * mw; e += blockDim.x) {
+        const int k = e / mw, u = F.nb_ids[v * F.K + k];
+        nmask[e] = u >= 0 ? __ldcg(X.mask + (size_t)u * mw + (e - k * mw)) : 0u;
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < N; idx += blockDim.x) {
+        const uint32_t head = X.head[base + idx];
+        const uint32_t cls = head & 3u;
+        dv[idx] = X.disp[base + idx];
+        uint8_t r = kPrKeep;
+        bool k1 = false;
+        if (cls == kHeadCost) r = kPrCost;
+        else if (cls == kHeadNoViews) r = kPrNoSupport;
+        else if (cls == kHeadOpen) {
+            int support = (int)((head >> 2) & 63u), good = (int)((head >> 8) & 63u);
+            const int n = (int)(head >> 14);
+            for (int j = 0; j < n; ++j) {
+                const uint32_t e = X.ent[(size_t)j * X.total + base + idx];
+                const uint32_t* m = nmask + (e & 31u) * mw;
+                const int x0 = (int)((e >> 5) & 31u), y0 = (int)((e >> 10) & 31u);
+                const int x1 = min(x0 + 1, W - 1), y1 = min(y0 + 1, H - 1);
+                auto out = [&](int b) { return (m[b >> 5] >> (b & 31)) & 1u; };
+                if (out(y0 * W + x0) | out(y0 * W + x1) | out(y1 * W + x0) | out(y1 * W + x1)) continue;
+                ++support;
+                good += (int)(e >> 15);
+            }
+            if (support < cfg.min_good_neighbors) r = kPrNoSupport;
+            else if (good < cfg.min_good_neighbors) r = kPrCycle;
+            else k1 = true;
+        }
+        keep[idx] = k1;
+        why[idx] = r;
+    }
+    __syncthreads();
+    if (cfg.enable_spike_filter)
+        // spike pass (MIDisparityFilter.cpp:644-676): the disparity against the median
+        // (element n / 2 in ascending order) of the kept neighbours'.  The median is too
+        // low or too high exactly when the values too low, or too high, reach its place.
+        for (int idx = threadIdx.x; idx < N; idx += blockDim.x) {
+            if (!keep[idx]) continue;
+            const int x = idx % W, y = idx / W;
+            const float cur = dv[idx];
+            int n = 0, lo = 0, hi = 0;
+#pragma unroll
+            for (int q = 0; q < 9; ++q) {
+                if (q == 4) continue;
+                const int xn = x + q % 3 - 1, yn = y + q / 3 - 1;
+                if (xn < 0 || yn < 0 || xn >= W || yn >= H) continue;
+                const int ni = yn * W + xn;
+                if (!keep[ni]) continue;
+                const float val = dv[ni];
+                ++n;
+                if (fabsf(cur - val) > cfg.spike_abs_diff) { if (val < cur) ++lo; else ++hi; }
+            }
+            if (n < cfg.spike_min_neighbors || n == 0) continue;
+            if (lo > n / 2 || n - hi <= n / 2) why[idx] = kPrSpike;
+        }
+    __syncthreads();
+}
+
+// Barrier of the whole (cooperative) grid: bounded wait, records a timeout and gives up.
+__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int target, int* err)
+{
+    __syncthreads();
+    int ok = 1;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        ok = 0;
+        for (unsigned int it = 0; it < (1u << 22); ++it) {
+            if (*(volatile unsigned int*)bar >= target) { ok = 1; break; }
+            if (it > 32) __nanosleep(64);
+        }
+        __threadfence();
+        if (!ok) atomicOr(err, 1);
+    }
+    return __syncthreads_and(ok) != 0;
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(256) pm_filter_resolve_kernel(CheckFrame F, FilterCfg cfg, FilterWork X, int* err)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int N = F.W * F.H, mw = X.mask_words;
+    uint32_t* nmask = (uint32_t*)smem;                   // [K][mw]
+    float* dv = (float*)(nmask + F.K * mw);              // [N]
+    uint8_t* keep = (uint8_t*)(dv + N);                  // [N]
+    uint8_t* why = keep + N;                             // [N]
+    unsigned int arrived = 0;
+    // X.ctl: 0 barrier; 1, 2, 3 list lengths of rounds 1, 2, 3 mod 3
+    for (int round = 1; round <= F.V + 2; ++round) {
+        // views with an earlier neighbour that changed in the last round (or already in
+        // this one); all of them in the first round
+        int n_list = F.V;
+        if (round > 1) {
+            if (blockIdx.x == 0 && threadIdx.x == 0) X.ctl[1 + (round + 1) % 3] = 0u;
+            for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < F.V; v += gridDim.x * blockDim.x) {
+                const int nc = min(F.nb_counts[v], F.K);
+                const int2 key = F.keys[v];
+                bool dirty = false;
+                for (int k = 0; k < nc && !dirty; ++k) {
+                    const int u = F.nb_ids[v * F.K + k];
+                    if (u >= 0 && __ldcg(X.changed + u) >= round - 1 && key_before(F.keys[u], key)) dirty = true;
+                }
+                if (dirty) X.list[atomicAdd(X.ctl + 1 + round % 3, 1u)] = v;
+            }
+            if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
+            n_list = (int)__ldcg(X.ctl + 1 + round % 3);
+            if (n_list == 0) return;
+        }
+        for (int i = blockIdx.x; i < n_list; i += gridDim.x) {
+            const int v = round > 1 ? __ldcg(X.list + i) : i;
+            eval_view(F, cfg, X, v, nmask, dv, keep, why);
+            int diff = 0;
+            for (int b0 = 0; b0 < mw * 32; b0 += blockDim.x) {
+                const int b = b0 + threadIdx.x;
+                const uint32_t bits = __ballot_sync(0xffffffffu, b < N && why[b < N ? b : 0] != kPrKeep);
+                if ((threadIdx.x & 31) == 0 && b < mw * 32) {
+                    uint32_t* m = X.mask + (size_t)v * mw + (b >> 5);
+                    if (__ldcg(m) != bits) { __stcg(m, bits); diff = 1; }
+                }
+            }
+            if (__syncthreads_or(diff) && threadIdx.x == 0) __stcg(X.changed + v, round);
+        }
+        if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, 1);       // key order has no cycles: not reached
+}
+
+__global__ void __launch_bounds__(256) pm_filter_apply_kernel(CheckFrame F, FilterCfg cfg, StateDev st, FilterWork X,
+                                                              uint8_t* reason, unsigned long long* stats)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int N = F.W * F.H, v = blockIdx.x;
+    uint32_t* nmask = (uint32_t*)smem;
+    float* dv = (float*)(nmask + F.K * X.mask_words);
+    uint8_t* keep = (uint8_t*)(dv + N);
+    uint8_t* why = keep + N;
+    __shared__ unsigned int cnt[8];
+    if (threadIdx.x < 8) cnt[threadIdx.x] = 0;
+    eval_view(F, cfg, X, v, nmask, dv, keep, why);
+    const size_t base = (size_t)v * N;
+    unsigned int valid = 0, cost = 0, support = 0, cycle = 0, spike = 0;
+    for (int idx = threadIdx.x; idx < N; idx += blockDim.x) {
+        const uint8_t r = why[idx];
+        if (reason) reason[base + idx] = r;
+        if ((X.head[base + idx] & 3u) == kHeadInvalid) continue;
+        ++valid;
+        cost += r == kPrCost;
+        support += r == kPrNoSupport;
+        cycle += r == kPrCycle;
+        spike += r == kPrSpike;
+        if (r == kPrKeep) continue;
+        // InvalidatePixel (MIDisparityFilter.cpp:158-174)
+        st.plane[base + idx] = make_float4(0.0f, 0.0f, 0.0f, -1.0f);
+        st.cost[base + idx] = 2.0f;
+        st.disp[base + idx] = make_float4(-1.0f, -1.0f, 0.0f, 0.0f);
+        if (cfg.clear_selected_views_when_invalid) st.sel[base + idx] = 0u;
+    }
+    const unsigned int part[5] = { valid, cost, support, cycle, spike };
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        const unsigned int t = __reduce_add_sync(0xffffffffu, part[i]);
+        if ((threadIdx.x & 31) == 0 && t) atomicAdd(&cnt[i], t);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned int gone = cnt[1] + cnt[2] + cnt[3] + cnt[4];
+        atomicAdd(stats + kFsTotal, (unsigned long long)N);
+        if (cnt[0]) atomicAdd(stats + kFsValidIn, (unsigned long long)cnt[0]);
+        if (cnt[0] - gone) atomicAdd(stats + kFsKept, (unsigned long long)(cnt[0] - gone));
+        if (gone) atomicAdd(stats + kFsRemoved, (unsigned long long)gone);
+        if (cnt[1]) atomicAdd(stats + kFsCost, (unsigned long long)cnt[1]);
+        if (cnt[2]) atomicAdd(stats + kFsNoSupport, (unsigned long long)cnt[2]);
+        if (cnt[3]) atomicAdd(stats + kFsCycle, (unsigned long long)cnt[3]);
+        if (cnt[4]) atomicAdd(stats + kFsSpike, (unsigned long long)cnt[4]);
     }
 }
 
@@ -585,6 +939,68 @@ cudaError_t launch_cycle(const CheckFrame& F, const CycleCfg& cfg, const StateDe
     if (e != cudaSuccess) return e;
     const int threads = F.W * F.H < 256 ? ((F.W * F.H + 31) / 32) * 32 : 256;
     pm_cycle_kernel<<<F.V, threads < 64 ? 64 : threads, smem, s>>>(F, cfg, st, geo_err, pho_err, texmask, recs, hist);
+    return cudaGetLastError();
+}
+
+// The filter's work area: what filter_work() lays out in a scratch buffer.
+size_t filter_work_bytes(const CheckFrame& F, const FilterCfg& cfg)
+{
+    FilterWork X;
+    return filter_work(F, cfg, nullptr, X);
+}
+
+size_t filter_work(const CheckFrame& F, const FilterCfg& cfg, unsigned char* buf, FilterWork& X)
+{
+    const size_t px = (size_t)F.V * F.W * F.H;
+    size_t o = 0;
+    auto take = [&](size_t bytes) { const size_t at = o; o += (bytes + 255) & ~(size_t)255; return buf + at; };
+    X.total = px;
+    X.mask_words = (F.W * F.H + 31) / 32;
+    X.zeroed = buf;
+    X.ctl = (unsigned int*)take(16);
+    X.changed = (int*)take(sizeof(int) * (size_t)F.V);
+    X.mask = (uint32_t*)take(sizeof(uint32_t) * (size_t)F.V * X.mask_words);
+    X.zeroed_bytes = o;
+    X.list = (int*)take(sizeof(int) * (size_t)F.V);
+    X.head = (uint32_t*)take(sizeof(uint32_t) * px);
+    X.disp = (float*)take(sizeof(float) * px);
+    X.ent = (uint16_t*)take(sizeof(uint16_t) * px * (size_t)(cfg.max_triplet > 0 ? cfg.max_triplet : 1));
+    return o;
+}
+
+cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,
+                          uint8_t* reason, unsigned long long* stats, int* err, cudaStream_t s)
+{
+    if (F.V <= 0) return cudaSuccess;
+    const int N = F.W * F.H;
+    const int smem_a = (1 + F.K) * F.tile_stride + F.K * (int)(sizeof(NbDir) + sizeof(int));
+    const int smem_b = F.K * X.mask_words * 4 + N * 6;
+    cudaError_t e = cudaMemsetAsync(X.zeroed, 0, X.zeroed_bytes, s);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(pm_filter_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_a);
+    if (e != cudaSuccess) return e;
+    const int threads = std::min(256, (N + 31) / 32 * 32);
+    pm_filter_pairs_kernel<<<F.V, threads, smem_a, s>>>(F, cfg, st, X);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pm_filter_resolve_kernel, threads, smem_b);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)std::max(1, std::min(F.V, sms * std::min(per_sm, 4))));
+    lc.blockDim = dim3((unsigned)threads);
+    lc.dynamicSmemBytes = (size_t)smem_b;
+    lc.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    e = cudaLaunchKernelEx(&lc, pm_filter_resolve_kernel, F, cfg, X, err);
+    if (e != cudaSuccess) return e;
+    pm_filter_apply_kernel<<<F.V, threads, smem_b, s>>>(F, cfg, st, X, reason, stats);
     return cudaGetLastError();
 }
 

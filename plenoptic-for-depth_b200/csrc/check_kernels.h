@@ -32,6 +32,7 @@ struct CheckFrame {
     int V, W, H, K, tile_stride;
     const uint8_t* gray;       // [V][tile_stride]
     const float2* centers;
+    const int2* keys;          // tile keys (column, row): the filter's order is row, then column
     const int* nb_ids;
     const int* nb_counts;
     float baseline_unit;       // LightFieldParams::baseline (lens pitch)
@@ -70,6 +71,27 @@ constexpr int kCycleHistBins = 128;                           // 0.5 px bins of 
 int cycle_smem_bytes(const CheckFrame& F);
 cudaError_t launch_cycle(const CheckFrame& F, const CycleCfg& cfg, const StateDev& st, float* geo_err, float* pho_err,
                          uint8_t* texmask, CycleTileRec* recs, unsigned int* hist, cudaStream_t s);
+
+// The filter's work area (see check_kernels.cu): 8 + 2 max_triplet bytes per pixel,
+// and a mask, a stamp and a list entry per micro-image.
+struct FilterWork {
+    size_t total;              // pixels of the frame
+    int mask_words;            // 32-bit words of a micro-image's mask
+    unsigned char* zeroed;     // the part that starts at zero: ctl, changed, mask
+    size_t zeroed_bytes;
+    unsigned int* ctl;
+    int* changed;              // [V] round in which the mask last changed
+    uint32_t* mask;            // [V][mask_words] rejected pixels
+    int* list;                 // [V] micro-images of the round
+    uint32_t* head;            // [total] class and final counts
+    float* disp;               // [total] disparity
+    uint16_t* ent;             // [max_triplet][total] tests against earlier neighbours
+};
+size_t filter_work_bytes(const CheckFrame& F, const FilterCfg& cfg);
+size_t filter_work(const CheckFrame& F, const FilterCfg& cfg, unsigned char* buf, FilterWork& X);
+// The whole filter, three launches; err gets flag 1 when a device wait gave up.
+cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,
+                          uint8_t* reason, unsigned long long* stats, int* err, cudaStream_t s);
 
 int filter_smem_bytes(const CheckFrame& F);
 // One wavefront step: the views step_views[0..n_step) filtered in parallel.

@@ -1544,7 +1544,7 @@ static pfd::CheckFrame check_frame(const Frame& f, float baseline_unit)
 {
     pfd::CheckFrame F;
     F.V = f.V; F.W = f.mi_w; F.H = f.mi_h; F.K = f.K; F.tile_stride = f.tile_stride;
-    F.gray = f.d_gray; F.centers = f.d_centers; F.nb_ids = f.d_nb_ids; F.nb_counts = f.d_nb_counts;
+    F.gray = f.d_gray; F.centers = f.d_centers; F.keys = f.d_tilekeys; F.nb_ids = f.d_nb_ids; F.nb_counts = f.d_nb_counts;
     F.baseline_unit = baseline_unit;
     return F;
 }
@@ -1618,7 +1618,6 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
     if (st != PFD_OK) return st;
     if (!f->has_state) return fail(ctx, PFD_ESTATE, "filter before PatchMatch");
     DeviceGuard g(ctx->device);
-    if ((st = build_steps(ctx, *f)) != PFD_OK) return st;
     const size_t px = (size_t)f->V * f->mi_w * f->mi_h;
     if (!f->d_reason) {
         void* p = nullptr;
@@ -1636,6 +1635,17 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
         f->d_fstats = (unsigned long long*)p;
     }
     unsigned long long* d_stats = f->d_fstats;
+    // three launches over a work area in the context's scratch; as a wavefront where
+    // a rejected pixel's disparity (-1) counts as usable, or where the budget does not
+    // hold the work area (the same result, 10x slower)
+    pfd::FilterWork X;
+    bool wavefront = !(fc.min_valid_disp >= -1.0f);
+    if (!wavefront && ensure_scratch(ctx, pfd::filter_work_bytes(F, fc)) != PFD_OK) wavefront = true;
+    if (wavefront) {
+        if ((st = build_steps(ctx, *f)) != PFD_OK) return st;
+    } else {
+        pfd::filter_work(F, fc, (unsigned char*)ctx->d_scratch, X);
+    }
     // enqueue-only calls under pfd_set_graphs: the first call with a key runs as
     // usual, the second is captured, later ones replay the graph (it reads the
     // state buffer the frame's current state was in at capture)
@@ -1646,6 +1656,7 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
         std::vector<unsigned char> key(sizeof(pfd_filter_cfg) + sizeof(float));
         std::memcpy(key.data(), cfg, sizeof(pfd_filter_cfg));
         std::memcpy(key.data() + sizeof(pfd_filter_cfg), &baseline_unit, sizeof(float));
+        if (G.exec && G.scratch_gen != ctx->scratch_gen) G.reset();   // the scratch moved since the capture
         if (G.exec && G.key == key && G.cur == f->cur) {
             CU(cudaGraphLaunch(G.exec, ctx->stream));
             ctx->launches += G.launches;
@@ -1667,7 +1678,12 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
         fst = fail(ctx, PFD_ECUDA, "filter: counter reset");
     const pfd::StateDev& S = f->s[f->cur];
     f->cvec_valid = 0;                             // rejected pixels get new planes
-    for (size_t s = 0; fst == PFD_OK && s + 1 < f->step_start.size(); ++s) {
+    if (!wavefront && fst == PFD_OK) {
+        const cudaError_t e = pfd::launch_filter(F, fc, S, X, f->d_reason, d_stats, ctx->d_err, ctx->stream);
+        if (e != cudaSuccess) fst = fail(ctx, PFD_ECUDA, "filter: %s", cudaGetErrorString(e));
+        else ctx->launches += 3;
+    }
+    for (size_t s = 0; wavefront && fst == PFD_OK && s + 1 < f->step_start.size(); ++s) {
         const int a = f->step_start[s], b = f->step_start[s + 1];
         cudaError_t e = pfd::launch_filter_step(F, fc, S, f->d_steps + a, b - a, f->d_reason, d_stats, ctx->stream);
         if (e != cudaSuccess) fst = fail(ctx, PFD_ECUDA, "filter step: %s", cudaGetErrorString(e));
@@ -1683,6 +1699,7 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
         if (graph) cudaGraphDestroy(graph);
         if (fst != PFD_OK) { G.reset(); return fst; }
         G.launches = ctx->launches - launches0;
+        G.scratch_gen = ctx->scratch_gen;
         CU(cudaGraphLaunch(G.exec, ctx->stream));
         return PFD_OK;
     }
@@ -1691,7 +1708,7 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
     if (stats) CU(cudaMemcpyAsync(h, d_stats, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     if (reason) CU(cudaMemcpyAsync(reason, f->d_reason, px, cudaMemcpyDeviceToHost, ctx->stream));
     if (stats || reason) {
-        CU(cudaStreamSynchronize(ctx->stream));
+        if ((st = check_device_error(ctx)) != PFD_OK) return st;
         if (stats) for (int i = 0; i < 8; ++i) stats[i] = (long long)h[i];
     }
     return PFD_OK;
