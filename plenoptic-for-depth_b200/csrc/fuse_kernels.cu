@@ -4,17 +4,30 @@
 // The reference visits the reference micro-images in map order and their
 // pixels row by row; a pixel that finds at least two consistent neighbour
 // pixels becomes a fused point and masks the neighbour pixels it used, which
-// everything after it then skips.  Two micro-images depend on each other only
-// through the masks of the micro-images they both touch (themselves and their
-// list entries), so the host groups them into wavefront steps in which no two
-// touch a common micro-image, ordered so that every dependent pair keeps the
-// reference's order; a step runs one warp per micro-image, pixel after pixel,
-// the warp's lanes taking the neighbour-list entries.  Consistent neighbours
-// are summed in list order by shuffles, so every float is the reference's.
+// everything after it then skips.  Which neighbour pixels are consistent does not
+// depend on the masks, so:
+//   pm_fuse_pairs_kernel    per (pixel, list entry) the consistent neighbour pixel,
+//                           or none.
+//   pm_fuse_resolve_kernel  the walk itself, on bits only: one warp per micro-image
+//                           goes through its pixels in order with the masks that the
+//                           micro-images before it leave, and publishes the pixels it
+//                           masks.  All micro-images run side by side; those whose
+//                           predecessors changed run again until nothing changes.  A
+//                           micro-image depends on earlier ones only, so this ends at
+//                           the one solution, the sequential walk's.  A cooperative
+//                           launch; the grid barrier's waits are bounded.
+//   pm_fuse_points_kernel   the fused points, one thread per pixel, their neighbours
+//                           summed in list order, so every float is the reference's.
 // Points that land on the same raw pixel overwrite each other in map order in
 // the reference; here each records its sequence number (micro-image, pixel)
 // with atomicMax and the maps are written from the last one afterwards.
+//
+// A wavefront over the micro-images, one warp each with the tests in its chain of
+// loads (0.5 ms per step), took 553 ms on the 4080x3068 frame and 99 ms on the
+// 1024x768 one; this form 10 and 1.3 ms (12 list entries), bound by the gathers of
+// the pairs kernel and the rounds' walks of 256 dependent steps.
 #include <climits>
+#include <algorithm>
 #include <cstdint>
 #include "fuse_kernels.h"
 
@@ -74,110 +87,337 @@ __device__ __forceinline__ bool valid_vd(float vd)
 
 }  // namespace
 
-__global__ void __launch_bounds__(128) pm_fuse_step_kernel(FuseFrame F, const int* __restrict__ views, int n)
+// The fused point's neighbour test (:1660-1720): the pixel of list entry u that
+// reference pixel (r, c) of view centre cr at virtual depth vdr projects to, when it
+// is consistent; -1 otherwise.
+__device__ __forceinline__ int consistent_pixel(const FuseFrame& F, float3 P, float vdr, int r, int c, float2 cr, int u,
+                                                float2 cu, float cm)
 {
-    const int lane = threadIdx.x & 31;
-    const int wi = blockIdx.x * 4 + (threadIdx.x >> 5);
-    if (wi >= n) return;                              // whole warps leave together
-    const int v = views[wi];
-    const int m = F.m, ppv = F.ppv;
+    const float2 q = back_project(P, cu, cm);
+    const int src_r = trunc_x86(__fadd_rn(q.y, 0.5f)), src_c = trunc_x86(__fadd_rn(q.x, 0.5f));
+    if (!(src_c >= 0 && src_c < F.m && src_r >= 0 && src_r < F.m)) return -1;
+    const int si = src_r * F.m + src_c;
+    const float w = F.plane[(size_t)u * F.ppv + si].w;
+    if (w <= 0.0f) return -1;
+    const float vds = virtual_depth(F.mla_base, w);
+    if (!valid_vd(vds)) return -1;
+    const float3 Ps = virtual_3d(vds, src_c, src_r, cm, cu);
+    const float2 rq = back_project(Ps, cr, cm);
+    const float ex = __fsub_rn((float)c, rq.x), ey = __fsub_rn((float)r, rq.y);
+    const float err = __fsqrt_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)));
+    const float den = vdr < 1.0e-6f ? 1.0e-6f : vdr;
+    const float rel = __fdiv_rn(fabsf(__fsub_rn(vds, vdr)), den);
+    return (err < F.max_reproj_px && rel < F.max_rel_vd) ? si : -1;
+}
+
+// One CTA per micro-image: pair_si[(v, idx)][j] of its list entries, and the mask of
+// the pixels that can become points (a valid depth and enough consistent entries).
+__global__ void __launch_bounds__(256) pm_fuse_pairs_kernel(FuseFrame F, FuseWork X)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int v = blockIdx.x;
+    if (!X.is_ref[v]) return;
+    const int m = F.m, N = F.ppv;
+    const int nl = min(F.list_counts[v], F.max_list);
+    int* ids = (int*)smem;                               // [max_list]
+    float2* cen = (float2*)(ids + ((F.max_list + 1) & ~1));
+    for (int j = threadIdx.x; j < nl; j += blockDim.x) {
+        const int u = F.lists[(size_t)v * F.max_list + j];
+        ids[j] = u;
+        cen[j] = u >= 0 ? F.centers[u] : make_float2(0.f, 0.f);
+    }
+    __syncthreads();
     const float cm = __fadd_rn(__fmul_rn((float)(m - 1), 0.5f), 1.0f);
     const float2 cr = F.centers[v];
+    const int n32 = (N + 31) & ~31;
+    for (int idx = threadIdx.x; idx < n32; idx += blockDim.x) {
+        int num = -1;
+        if (idx < N) {
+            const float w = F.plane[(size_t)v * N + idx].w;
+            const float vdr = virtual_depth(F.mla_base, w);
+            const bool own = !(w < F.min_ref_disp) && valid_vd(vdr);
+            const int r = idx / m, c = idx - r * m;
+            const float3 P = virtual_3d(vdr, c, r, cm, cr);
+            uint16_t* row = X.pair_si + ((size_t)v * N + idx) * F.max_list;
+            if (own) num = 0;
+            for (int j = 0; j < nl; ++j) {
+                int si = -1;
+                if (own && ids[j] >= 0) si = consistent_pixel(F, P, vdr, r, c, cr, ids[j], cen[j], cm);
+                row[j] = si >= 0 ? (uint16_t)si : kFuseNone;
+                num += si >= 0;
+            }
+        }
+        const unsigned bits = __ballot_sync(kFull, num >= 0 && num >= F.min_consistent);
+        if ((threadIdx.x & 31) == 0) X.maybe[(size_t)v * X.mask_words + (idx >> 5)] = bits;
+    }
+}
+
+// Who masks pixels of a micro-image: the (reference micro-image, list entry) pairs
+// that name it, as lists in X.rev.
+__global__ void pm_fuse_rev_count_kernel(FuseFrame F, FuseWork X)
+{
+    const size_t n = (size_t)F.V * F.max_list;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+        const int w = (int)(e / F.max_list), j = (int)(e - (size_t)w * F.max_list);
+        if (!X.is_ref[w] || j >= F.list_counts[w]) continue;
+        const int u = F.lists[e];
+        if (u >= 0) atomicAdd(X.rev_start + u + 1, 1);
+    }
+}
+
+__global__ void __launch_bounds__(1024) pm_fuse_rev_scan_kernel(FuseFrame F, FuseWork X)
+{
+    __shared__ int warp_sum[32];
+    __shared__ int carry;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) carry = 0;
+    __syncthreads();
+    for (int b = 0; b < F.V; b += 1024) {
+        const int i = b + threadIdx.x;
+        int x = i < F.V ? X.rev_start[i + 1] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(kFull, x, o);
+            if (lane >= o) x += t;
+        }
+        if (lane == 31) warp_sum[warp] = x;
+        __syncthreads();
+        if (warp == 0) {
+            int s = warp_sum[lane];
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(kFull, s, o);
+                if (lane >= o) s += t;
+            }
+            warp_sum[lane] = s;
+        }
+        __syncthreads();
+        const int base = carry + (warp ? warp_sum[warp - 1] : 0);
+        if (i < F.V) { X.rev_start[i + 1] = base + x; X.rev_fill[i + 1] = base + x; }
+        __syncthreads();
+        if (threadIdx.x == 1023) carry = base + x;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) { X.rev_start[0] = 0; X.rev_fill[0] = 0; }
+}
+
+__global__ void pm_fuse_rev_fill_kernel(FuseFrame F, FuseWork X)
+{
+    const size_t n = (size_t)F.V * F.max_list;
+    for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+        const int w = (int)(e / F.max_list), j = (int)(e - (size_t)w * F.max_list);
+        if (!X.is_ref[w] || j >= F.list_counts[w]) continue;
+        const int u = F.lists[e];
+        if (u >= 0) X.rev[atomicAdd(X.rev_fill + u, 1)] = make_int2(w, j);
+    }
+}
+
+namespace {
+
+// Barrier of the whole (cooperative) grid: bounded wait, records a timeout and gives up.
+__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int target, int* err)
+{
+    __syncthreads();
+    int ok = 1;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        ok = 0;
+        for (unsigned int it = 0; it < (1u << 22); ++it) {
+            if (*(volatile unsigned int*)bar >= target) { ok = 1; break; }
+            if (it > 32) __nanosleep(64);
+        }
+        __threadfence();
+        if (!ok) atomicOr(err, 1);
+    }
+    return __syncthreads_and(ok) != 0;
+}
+
+// One micro-image's walk by one warp.  taken: [1 + nl][mw] masks of the micro-image
+// itself and of its list entries (entries naming the same micro-image share the
+// first one's), fresh: [nl][mw] what this walk masks.  Publishes the difference.
+__device__ __forceinline__ void walk_view(const FuseFrame& F, const FuseWork& X, int v, uint32_t* taken, uint32_t* fresh,
+                                          int* changed_at)
+{
+    const int lane = threadIdx.x & 31, N = F.ppv, mw = X.mask_words;
     const int nl = min(F.list_counts[v], F.max_list);
     const int nch = (nl + 31) >> 5;
-    int uj[kFuseMaxList / 32];
-    float2 cj[kFuseMaxList / 32];
+    const int* list = F.lists + (size_t)v * F.max_list;
+    for (int e = lane; e < (1 + nl) * mw; e += 32) taken[e] = 0u;
+    for (int e = lane; e < nl * mw; e += 32) fresh[e] = 0u;
+    const uint16_t* rows = X.pair_si + (size_t)v * N * F.max_list;
+    for (int b = lane * 128; b < N * F.max_list * 2; b += 32 * 128)
+        asm volatile("prefetch.global.L1 [%0];" :: "l"((const char*)rows + b));
+    // slot of each list entry: 0 for the micro-image itself, else 1 + the first entry
+    // that names it
+    int uj[kFuseMaxList / 32], slot[kFuseMaxList / 32];
 #pragma unroll
     for (int ch = 0; ch < kFuseMaxList / 32; ++ch) {
+        uj[ch] = -1;
+        slot[ch] = 0;
         const int j = ch * 32 + lane;
-        uj[ch] = (j < nl) ? F.lists[(size_t)v * F.max_list + j] : -1;
-        cj[ch] = uj[ch] >= 0 ? F.centers[uj[ch]] : make_float2(0.f, 0.f);
+        if (ch < nch && j < nl) {
+            uj[ch] = list[j];
+            slot[ch] = 1 + j;
+            if (uj[ch] == v) slot[ch] = 0;
+            else
+                for (int i = 0; i < j; ++i)
+                    if (list[i] == uj[ch]) { slot[ch] = 1 + i; break; }
+        }
     }
-    for (int idx = 0; idx < ppv; ++idx) {
-        if (F.mask[(size_t)v * ppv + idx] == 1) continue;
-        const float4 pl = F.plane[(size_t)v * ppv + idx];
-        if (pl.w < F.min_ref_disp) continue;
-        const float vdr = virtual_depth(F.mla_base, pl.w);
-        if (!valid_vd(vdr)) continue;
-        const int r = idx / m, c = idx - r * m;
-        const float3 P = virtual_3d(vdr, c, r, cm, cr);
-        float3 sp = P, sn = make_float3(pl.x, pl.y, pl.z), sc = colour(F, v, idx);
-        int num = 0;
-        bool ok[kFuseMaxList / 32];
-        int usi[kFuseMaxList / 32];
+    __syncwarp();
+    // the masks that the micro-images before this one leave
+    for (int t = 0; t <= nl; ++t) {
+        int u = v;
+        if (t) {
+            const int ch = (t - 1) >> 5, src = (t - 1) & 31;
+            int a = -1, b = 0;
 #pragma unroll
-        for (int ch = 0; ch < kFuseMaxList / 32; ++ch) {
-            ok[ch] = false;
-            usi[ch] = 0;
-            if (ch >= nch) continue;                  // uniform
-            const int u = uj[ch];
-            float3 Ps = make_float3(0.f, 0.f, 0.f), Ns = Ps, Cs = Ps;
-            if (u >= 0) {
-                const float2 q = back_project(P, cj[ch], cm);
-                const int src_r = trunc_x86(__fadd_rn(q.y, 0.5f)), src_c = trunc_x86(__fadd_rn(q.x, 0.5f));
-                if (src_c >= 0 && src_c < m && src_r >= 0 && src_r < m) {
-                    const int si = src_r * m + src_c;
-                    if (F.mask[(size_t)u * ppv + si] != 1) {
-                        const float4 ps = F.plane[(size_t)u * ppv + si];
-                        if (!(ps.w <= 0.0f)) {
-                            const float vds = virtual_depth(F.mla_base, ps.w);
-                            if (valid_vd(vds)) {
-                                Ps = virtual_3d(vds, src_c, src_r, cm, cj[ch]);
-                                const float2 rq = back_project(Ps, cr, cm);
-                                const float ex = __fsub_rn((float)c, rq.x), ey = __fsub_rn((float)r, rq.y);
-                                const float err = __fsqrt_rn(__fadd_rn(__fmul_rn(ex, ex), __fmul_rn(ey, ey)));
-                                const float den = vdr < 1.0e-6f ? 1.0e-6f : vdr;
-                                const float rel = __fdiv_rn(fabsf(__fsub_rn(vds, vdr)), den);
-                                if (err < F.max_reproj_px && rel < F.max_rel_vd) {
-                                    ok[ch] = true;
-                                    usi[ch] = si;
-                                    Ns = make_float3(ps.x, ps.y, ps.z);
-                                    Cs = colour(F, u, si);
-                                }
-                            }
-                        }
-                    }
+            for (int c = 0; c < kFuseMaxList / 32; ++c)
+                if (c == ch) { a = uj[c]; b = slot[c]; }
+            u = __shfl_sync(kFull, a, src);
+            if (u < 0 || __shfl_sync(kFull, b, src) != t) continue;
+        }
+        const int r0 = X.rev_start[u], r1 = X.rev_start[u + 1];
+        for (int e = r0 * mw + lane; e < r1 * mw; e += 32) {
+            const int2 wj = X.rev[e / mw];
+            if (wj.x >= v) continue;
+            const int word = e % mw;
+            const uint32_t bits = __ldcg(X.marks + ((size_t)wj.x * F.max_list + wj.y) * mw + word);
+            if (bits) atomicOr(taken + t * mw + word, bits);
+        }
+    }
+    __syncwarp();
+    const uint32_t* maybe = X.maybe + (size_t)v * mw;
+    for (int wd = 0; wd < mw; ++wd) {
+        uint32_t todo = maybe[wd], accepted = 0u;
+        while (todo) {
+            const int b = __ffs(todo) - 1, idx = wd * 32 + b;
+            todo &= todo - 1;
+            if ((taken[wd] >> b) & 1u) continue;         // used by an earlier point
+            int si[kFuseMaxList / 32];
+            uint32_t bits[kFuseMaxList / 32];
+            int num = 0;
+#pragma unroll
+            for (int ch = 0; ch < kFuseMaxList / 32; ++ch) {
+                bits[ch] = 0u;
+                if (ch >= nch) continue;
+                const int j = ch * 32 + lane;
+                si[ch] = j < nl ? rows[(size_t)idx * F.max_list + j] : kFuseNone;
+                const bool ok = si[ch] != kFuseNone && !((taken[slot[ch] * mw + (si[ch] >> 5)] >> (si[ch] & 31)) & 1u);
+                bits[ch] = __ballot_sync(kFull, ok);
+                num += __popc(bits[ch]);
+            }
+            if (num < F.min_consistent) continue;
+            accepted |= 1u << b;
+            __syncwarp();
+#pragma unroll
+            for (int ch = 0; ch < kFuseMaxList / 32; ++ch) {
+                if (ch >= nch) continue;
+                if ((bits[ch] >> lane) & 1u) {
+                    atomicOr(taken + slot[ch] * mw + (si[ch] >> 5), 1u << (si[ch] & 31));
+                    atomicOr(fresh + (ch * 32 + lane) * mw + (si[ch] >> 5), 1u << (si[ch] & 31));
+                }
+                if (lane == 0) X.chosen[((size_t)v * N + idx) * X.chosen_words + ch] = bits[ch];
+            }
+            __syncwarp();
+        }
+        if (lane == 0) X.accepted[(size_t)v * mw + wd] = accepted;
+    }
+    __syncwarp();
+    for (int e = lane; e < nl * mw; e += 32) {
+        uint32_t* g = X.marks + (size_t)v * F.max_list * mw + e;
+        if (__ldcg(g) != fresh[e]) {
+            __stcg(g, fresh[e]);
+            atomicMin(changed_at + list[e / mw], v);
+        }
+    }
+    __syncwarp();
+}
+
+}  // namespace
+
+__global__ void __launch_bounds__(256) pm_fuse_resolve_kernel(FuseFrame F, FuseWork X, int* err)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5, mw = X.mask_words;
+    uint32_t* taken = (uint32_t*)smem + (size_t)warp * (1 + 2 * F.max_list) * mw;
+    uint32_t* fresh = taken + (1 + F.max_list) * mw;
+    unsigned int arrived = 0;
+    // X.ctl: 0 barrier; 1, 2, 3 list lengths of rounds 1, 2, 3 mod 3.  X.changed + (round
+    // mod 3) V: the first micro-image that changed what it masks in each, per round.
+    for (int round = 1; round <= F.V + 2; ++round) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) X.ctl[1 + (round + 1) % 3] = 0u;
+        const int* last = X.changed + (size_t)((round + 2) % 3) * F.V;
+        int* next = X.changed + (size_t)((round + 1) % 3) * F.V;
+        for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < F.V; v += gridDim.x * blockDim.x) {
+            __stcg(next + v, 0x7fffffff);
+            if (!X.is_ref[v]) continue;
+            bool dirty = round == 1;
+            if (!dirty) {
+                dirty = __ldcg(last + v) < v;
+                const int nl = min(F.list_counts[v], F.max_list);
+                for (int j = 0; j < nl && !dirty; ++j) {
+                    const int u = F.lists[(size_t)v * F.max_list + j];
+                    dirty = u >= 0 && __ldcg(last + u) < v;
                 }
             }
-            // the consistent entries of this chunk, summed in list order
-            unsigned bits = __ballot_sync(kFull, ok[ch]);
+            if (dirty) X.list[atomicAdd(X.ctl + 1 + round % 3, 1u)] = v;
+        }
+        if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
+        const int n_list = (int)__ldcg(X.ctl + 1 + round % 3);
+        if (n_list == 0) return;
+        for (int i = blockIdx.x * warps + warp; i < n_list; i += gridDim.x * warps)
+            walk_view(F, X, __ldcg(X.list + i), taken, fresh, X.changed + (size_t)(round % 3) * F.V);
+        if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, 1);       // map order has no cycles: not reached
+}
+
+__global__ void __launch_bounds__(256) pm_fuse_points_kernel(FuseFrame F, FuseWork X)
+{
+    const size_t n = (size_t)F.V * F.ppv;
+    const int m = F.m;
+    const float cm = __fadd_rn(__fmul_rn((float)(m - 1), 0.5f), 1.0f);
+    for (size_t seq = (size_t)blockIdx.x * blockDim.x + threadIdx.x; seq < n; seq += (size_t)gridDim.x * blockDim.x) {
+        const int v = (int)(seq / F.ppv), idx = (int)(seq - (size_t)v * F.ppv);
+        if (!X.is_ref[v] || !((X.accepted[(size_t)v * X.mask_words + (idx >> 5)] >> (idx & 31)) & 1u)) continue;
+        const float4 pl = F.plane[seq];
+        const float vdr = virtual_depth(F.mla_base, pl.w);
+        const int r = idx / m, c = idx - r * m;
+        float3 sp = virtual_3d(vdr, c, r, cm, F.centers[v]);
+        float3 sn = make_float3(pl.x, pl.y, pl.z), sc = colour(F, v, idx);
+        int num = 0;
+        const int nch = (min(F.list_counts[v], F.max_list) + 31) >> 5;
+        for (int ch = 0; ch < nch; ++ch) {
+            uint32_t bits = X.chosen[seq * X.chosen_words + ch];
             num += __popc(bits);
             while (bits) {
-                const int b = __ffs(bits) - 1;
+                const int j = ch * 32 + __ffs(bits) - 1;
                 bits &= bits - 1;
-                sp.x = __fadd_rn(sp.x, __shfl_sync(kFull, Ps.x, b));
-                sp.y = __fadd_rn(sp.y, __shfl_sync(kFull, Ps.y, b));
-                sp.z = __fadd_rn(sp.z, __shfl_sync(kFull, Ps.z, b));
-                sn.x = __fadd_rn(sn.x, __shfl_sync(kFull, Ns.x, b));
-                sn.y = __fadd_rn(sn.y, __shfl_sync(kFull, Ns.y, b));
-                sn.z = __fadd_rn(sn.z, __shfl_sync(kFull, Ns.z, b));
-                sc.x = __fadd_rn(sc.x, __shfl_sync(kFull, Cs.x, b));
-                sc.y = __fadd_rn(sc.y, __shfl_sync(kFull, Cs.y, b));
-                sc.z = __fadd_rn(sc.z, __shfl_sync(kFull, Cs.z, b));
+                const int u = F.lists[(size_t)v * F.max_list + j], si = X.pair_si[seq * F.max_list + j];
+                const float4 ps = F.plane[(size_t)u * F.ppv + si];
+                const int sr = si / m, scol = si - sr * m;
+                const float3 Ps = virtual_3d(virtual_depth(F.mla_base, ps.w), scol, sr, cm, F.centers[u]);
+                const float3 Cs = colour(F, u, si);
+                sp.x = __fadd_rn(sp.x, Ps.x); sp.y = __fadd_rn(sp.y, Ps.y); sp.z = __fadd_rn(sp.z, Ps.z);
+                sn.x = __fadd_rn(sn.x, ps.x); sn.y = __fadd_rn(sn.y, ps.y); sn.z = __fadd_rn(sn.z, ps.z);
+                sc.x = __fadd_rn(sc.x, Cs.x); sc.y = __fadd_rn(sc.y, Cs.y); sc.z = __fadd_rn(sc.z, Cs.z);
             }
         }
-        if (num >= F.min_consistent) {
-            // cv::Vec3f /= float multiplies by the float reciprocal
-            const float ia = __fdiv_rn(1.0f, __fadd_rn((float)num, 1.0f));
-            sp = make_float3(__fmul_rn(sp.x, ia), __fmul_rn(sp.y, ia), __fmul_rn(sp.z, ia));
-            sn = make_float3(__fmul_rn(sn.x, ia), __fmul_rn(sn.y, ia), __fmul_rn(sn.z, ia));
-            sc = make_float3(__fmul_rn(sc.x, ia), __fmul_rn(sc.y, ia), __fmul_rn(sc.z, ia));
-            const int vx = round_x86(sp.x), vy = round_x86(sp.y);
-            if (lane == 0 && vy >= 0 && vy < F.raw_h && vx >= 0 && vx < F.raw_w) {
-                const size_t seq = (size_t)v * ppv + idx;
-                float* rec = F.rec + seq * 10;
-                rec[0] = sp.x; rec[1] = sp.y; rec[2] = sp.z;
-                rec[3] = sn.x; rec[4] = sn.y; rec[5] = sn.z;
-                rec[6] = sc.x; rec[7] = sc.y; rec[8] = sc.z;
-                rec[9] = (float)num;
-                F.has_rec[seq] = 1u;
-                atomicMax(&F.winner[(size_t)vy * F.raw_w + vx], (unsigned int)seq + 1u);
-            }
-#pragma unroll
-            for (int ch = 0; ch < kFuseMaxList / 32; ++ch)
-                if (ok[ch]) F.mask[(size_t)uj[ch] * ppv + usi[ch]] = 1;
+        // cv::Vec3f /= float multiplies by the float reciprocal
+        const float ia = __fdiv_rn(1.0f, __fadd_rn((float)num, 1.0f));
+        sp = make_float3(__fmul_rn(sp.x, ia), __fmul_rn(sp.y, ia), __fmul_rn(sp.z, ia));
+        sn = make_float3(__fmul_rn(sn.x, ia), __fmul_rn(sn.y, ia), __fmul_rn(sn.z, ia));
+        sc = make_float3(__fmul_rn(sc.x, ia), __fmul_rn(sc.y, ia), __fmul_rn(sc.z, ia));
+        const int vx = round_x86(sp.x), vy = round_x86(sp.y);
+        if (vy >= 0 && vy < F.raw_h && vx >= 0 && vx < F.raw_w) {
+            float* rec = F.rec + seq * 10;
+            rec[0] = sp.x; rec[1] = sp.y; rec[2] = sp.z;
+            rec[3] = sn.x; rec[4] = sn.y; rec[5] = sn.z;
+            rec[6] = sc.x; rec[7] = sc.y; rec[8] = sc.z;
+            rec[9] = (float)num;
+            F.has_rec[seq] = 1u;
+            atomicMax(&F.winner[(size_t)vy * F.raw_w + vx], (unsigned int)seq + 1u);
         }
-        __syncwarp();                                 // this pixel's masks before the next pixel reads them
     }
 }
 
@@ -238,10 +478,63 @@ __global__ void __launch_bounds__(kFuseScanBlock) pm_fuse_compact_kernel(FuseFra
     }
 }
 
-cudaError_t launch_fuse_step(const FuseFrame& F, const int* views, int n, cudaStream_t st)
+size_t fuse_work(const FuseFrame& F, unsigned char* buf, FuseWork& X)
 {
-    if (n <= 0) return cudaSuccess;
-    pm_fuse_step_kernel<<<(n + 3) / 4, 128, 0, st>>>(F, views, n);
+    size_t o = 0;
+    auto take = [&](size_t bytes) { const size_t at = o; o += (bytes + 255) & ~(size_t)255; return buf + at; };
+    const size_t V = (size_t)F.V, px = V * F.ppv, L = (size_t)F.max_list;
+    X.mask_words = (F.ppv + 31) / 32;
+    X.chosen_words = (F.max_list + 31) / 32;
+    X.zeroed = buf;
+    X.ctl = (unsigned int*)take(16);
+    X.rev_start = (int*)take(sizeof(int) * (V + 1));
+    X.marks = (uint32_t*)take(sizeof(uint32_t) * V * L * X.mask_words);
+    X.zeroed_bytes = o;
+    X.changed = (int*)take(sizeof(int) * 3 * V);
+    X.rev_fill = (int*)take(sizeof(int) * (V + 1));
+    X.rev = (int2*)take(sizeof(int2) * V * L);
+    X.list = (int*)take(sizeof(int) * V);
+    X.maybe = (uint32_t*)take(sizeof(uint32_t) * V * X.mask_words);
+    X.accepted = (uint32_t*)take(sizeof(uint32_t) * V * X.mask_words);
+    X.chosen = (uint32_t*)take(sizeof(uint32_t) * px * X.chosen_words);
+    X.pair_si = (uint16_t*)take(sizeof(uint16_t) * px * L);
+    return o;
+}
+
+cudaError_t launch_fuse(const FuseFrame& F, const FuseWork& X, int* err, cudaStream_t st)
+{
+    int dev = 0, sms = 0, per_sm = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaError_t e = cudaMemsetAsync(X.zeroed, 0, X.zeroed_bytes, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(X.changed, 0x7f, sizeof(int) * 3 * (size_t)F.V, st);
+    if (e != cudaSuccess) return e;
+    const int flat = (int)std::min<size_t>(((size_t)F.V * F.max_list + 255) / 256, (size_t)sms * 8);
+    pm_fuse_pairs_kernel<<<F.V, std::min(256, (F.ppv + 31) & ~31), (F.max_list + 1) * 12 + 16, st>>>(F, X);
+    pm_fuse_rev_count_kernel<<<flat, 256, 0, st>>>(F, X);
+    pm_fuse_rev_scan_kernel<<<1, 1024, 0, st>>>(F, X);
+    pm_fuse_rev_fill_kernel<<<flat, 256, 0, st>>>(F, X);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    const size_t per_warp = (size_t)(1 + 2 * F.max_list) * X.mask_words * 4;
+    const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)96 * 1024 / per_warp));
+    const int smem = (int)(per_warp * warps);
+    e = cudaFuncSetAttribute(pm_fuse_resolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pm_fuse_resolve_kernel, 32 * warps, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)std::max(1, std::min((F.V + warps - 1) / warps, sms * std::min(per_sm, 4))));
+    lc.blockDim = dim3((unsigned)(32 * warps));
+    lc.dynamicSmemBytes = (size_t)smem;
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    if ((e = cudaLaunchKernelEx(&lc, pm_fuse_resolve_kernel, F, X, err)) != cudaSuccess) return e;
+    const size_t px = (size_t)F.V * F.ppv;
+    pm_fuse_points_kernel<<<(int)std::min<size_t>((px + 255) / 256, (size_t)sms * 16), 256, 0, st>>>(F, X);
     return cudaGetLastError();
 }
 

@@ -19,14 +19,35 @@ struct FuseFrame {
     float mla_base, min_ref_disp, max_reproj_px, max_rel_vd;
     int min_consistent;
     int raw_w, raw_h;
-    uint8_t* mask;                // [V * ppv], zero at the start
     unsigned int* winner;         // [raw_h * raw_w]: 1 + sequence number of the last point there, 0 = none
     float* rec;                   // [V * ppv][10]: point, normal, colour, consistent count
     unsigned int* has_rec;        // [V * ppv]: 1 where a point inside the raw frame was recorded
 };
 
-// One wavefront step: the reference micro-images views[0..n), one warp each.
-cudaError_t launch_fuse_step(const FuseFrame& F, const int* views, int n, cudaStream_t st);
+constexpr unsigned kFuseNone = 0xFFFFu;           // no consistent pixel
+
+// Work area of the walk (see fuse_kernels.cu).
+struct FuseWork {
+    const uint8_t* is_ref;        // [V] reference micro-images
+    int mask_words, chosen_words; // 32-bit words per micro-image mask, per pixel's list mask
+    unsigned char* zeroed;        // the part that starts at zero: ctl, rev_start, marks
+    size_t zeroed_bytes;
+    unsigned int* ctl;
+    int* rev_start;               // [V + 1] offsets into rev
+    int* rev_fill;
+    int2* rev;                    // [V * max_list] (reference micro-image, list entry) naming a micro-image
+    uint32_t* marks;              // [V][max_list][mask_words] pixels of the entry that the micro-image masks
+    int* changed;                 // [3][V]
+    int* list;                    // [V] micro-images of the round
+    uint32_t* maybe;              // [V][mask_words] pixels that can become points
+    uint32_t* accepted;           // [V][mask_words] pixels that did
+    uint32_t* chosen;             // [V * ppv][chosen_words] list entries of the point
+    uint16_t* pair_si;            // [V * ppv][max_list] consistent pixel of each entry, or kFuseNone
+};
+// Lays the work area out in buf and returns its bytes.
+size_t fuse_work(const FuseFrame& F, unsigned char* buf, FuseWork& X);
+// Tests, walk and points (six launches); err gets flag 1 when a device wait gave up.
+cudaError_t launch_fuse(const FuseFrame& F, const FuseWork& X, int* err, cudaStream_t st);
 // The maps from the winning points (outputs zeroed where no point landed).
 cudaError_t launch_fuse_maps(const FuseFrame& F, float* vd_map, uint8_t* conf, uint8_t* aif, cudaStream_t st);
 // Points in sequence order: counts per block of 1024 sequence numbers, then the

@@ -2095,42 +2095,6 @@ pfd_status pfd_refocus(pfd_ctx* ctx, int frame_id, const float* slice_vd, int n_
     return out ? check_device_error(ctx) : PFD_OK;
 }
 
-// Wavefront steps of the fusion: a reference micro-image runs one step after
-// the last step that touched any micro-image it touches (itself and its list
-// entries), so two micro-images that share one keep the reference's order and
-// micro-images of one step touch disjoint sets.
-static void fuse_schedule(int V, const int* lists, const int* counts, int max_list, const uint8_t* is_ref,
-                          std::vector<int>& order, std::vector<int>& step_start)
-{
-    std::vector<int> last(V, 0), step(V, 0);
-    int nsteps = 0;
-    for (int v = 0; v < V; ++v) {
-        if (!is_ref[v]) continue;
-        const int nl = std::min(counts[v], max_list);
-        int s = last[v];
-        for (int j = 0; j < nl; ++j) {
-            const int u = lists[(size_t)v * max_list + j];
-            if (u >= 0) s = std::max(s, last[u]);
-        }
-        step[v] = ++s;
-        last[v] = s;
-        for (int j = 0; j < nl; ++j) {
-            const int u = lists[(size_t)v * max_list + j];
-            if (u >= 0) last[u] = s;
-        }
-        nsteps = std::max(nsteps, s);
-    }
-    std::vector<int> cnt((size_t)nsteps + 2, 0);
-    for (int v = 0; v < V; ++v)
-        if (is_ref[v]) cnt[(size_t)step[v]]++;
-    step_start.assign((size_t)nsteps + 1, 0);
-    for (int s = 1; s <= nsteps; ++s) step_start[s] = step_start[s - 1] + cnt[(size_t)s];
-    order.assign((size_t)step_start[nsteps], 0);
-    std::vector<int> fill(step_start.begin(), step_start.end());
-    for (int v = 0; v < V; ++v)                       // ascending view order inside a step
-        if (is_ref[v]) order[(size_t)fill[(size_t)step[v] - 1]++] = v;
-}
-
 pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_params* p, const int* lists,
                                   const int* list_counts, int max_list, const uint8_t* is_ref, const uint8_t* bgr,
                                   float* vd_map, uint8_t* conf, uint8_t* aif, float* points, long long* n_points)
@@ -2157,8 +2121,6 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
         }
     }
     DeviceGuard g(ctx->device);
-    std::vector<int> order, step_start;
-    fuse_schedule(V, lists, list_counts, max_list, is_ref, order, step_start);
     const size_t ppv = (size_t)f->mi_w * f->mi_h, px = (size_t)V * ppv, npix = (size_t)f->W * f->H;
     const size_t nb = (px + pfd::kFuseScanBlock - 1) / pfd::kFuseScanBlock;
     cudaStream_t s = ctx->stream;
@@ -2173,15 +2135,14 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
             return e;
         }
     } S{ s, {} };
-    int *d_lists = nullptr, *d_counts = nullptr, *d_order = nullptr;
-    uint8_t *d_bgr = nullptr, *d_mask = nullptr, *d_conf = nullptr, *d_aif = nullptr;
+    int *d_lists = nullptr, *d_counts = nullptr;
+    uint8_t *d_bgr = nullptr, *d_ref = nullptr, *d_work = nullptr, *d_conf = nullptr, *d_aif = nullptr;
     unsigned int *d_winner = nullptr, *d_has = nullptr, *d_bcount = nullptr;
     float *d_rec = nullptr, *d_vd = nullptr, *d_points = nullptr;
     CU(S.get((void**)&d_lists, sizeof(int) * (size_t)V * max_list));
     CU(S.get((void**)&d_counts, sizeof(int) * (size_t)V));
-    CU(S.get((void**)&d_order, sizeof(int) * std::max<size_t>(order.size(), 1)));
+    CU(S.get((void**)&d_ref, (size_t)V));
     if (bgr) CU(S.get((void**)&d_bgr, px * 3));
-    CU(S.get((void**)&d_mask, px));
     CU(S.get((void**)&d_winner, sizeof(unsigned int) * npix));
     CU(S.get((void**)&d_has, sizeof(unsigned int) * px));
     CU(S.get((void**)&d_rec, sizeof(float) * 10 * px));
@@ -2190,10 +2151,8 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
     CU(S.get((void**)&d_aif, npix * 3));
     CU(cudaMemcpyAsync(d_lists, lists, sizeof(int) * (size_t)V * max_list, cudaMemcpyHostToDevice, s));
     CU(cudaMemcpyAsync(d_counts, list_counts, sizeof(int) * (size_t)V, cudaMemcpyHostToDevice, s));
-    if (!order.empty())
-        CU(cudaMemcpyAsync(d_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice, s));
+    CU(cudaMemcpyAsync(d_ref, is_ref, (size_t)V, cudaMemcpyHostToDevice, s));
     if (bgr) CU(cudaMemcpyAsync(d_bgr, bgr, px * 3, cudaMemcpyHostToDevice, s));
-    CU(cudaMemsetAsync(d_mask, 0, px, s));
     CU(cudaMemsetAsync(d_winner, 0, sizeof(unsigned int) * npix, s));
     CU(cudaMemsetAsync(d_has, 0, sizeof(unsigned int) * px, s));
     pfd::FuseFrame F;
@@ -2203,12 +2162,13 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
     F.mla_base = p->mla_base; F.min_ref_disp = p->min_ref_disp; F.max_reproj_px = p->max_reproj_px;
     F.max_rel_vd = p->max_rel_vd; F.min_consistent = p->min_consistent;
     F.raw_w = f->W; F.raw_h = f->H;
-    F.mask = d_mask; F.winner = d_winner; F.rec = d_rec; F.has_rec = d_has;
-    for (size_t k = 0; k + 1 < step_start.size(); ++k) {
-        const int a = step_start[k], b = step_start[k + 1];
-        CU(pfd::launch_fuse_step(F, d_order + a, b - a, s));
-        ctx->launches += 1;
-    }
+    F.winner = d_winner; F.rec = d_rec; F.has_rec = d_has;
+    pfd::FuseWork X;
+    CU(S.get((void**)&d_work, pfd::fuse_work(F, nullptr, X)));
+    pfd::fuse_work(F, d_work, X);
+    X.is_ref = d_ref;
+    CU(pfd::launch_fuse(F, X, ctx->d_err, s));
+    ctx->launches += 6;
     CU(pfd::launch_fuse_maps(F, d_vd, d_conf, d_aif, s));
     ctx->launches += 1;
     if (vd_map) CU(cudaMemcpyAsync(vd_map, d_vd, sizeof(float) * npix, cudaMemcpyDeviceToHost, s));
