@@ -2087,10 +2087,13 @@ pfd_status pfd_refocus(pfd_ctx* ctx, int frame_id, const float* slice_vd, int n_
     R.cell_ids = f->d_cells + (size_t)f->grid_w * f->grid_h + 1;
     R.grid_w = f->grid_w; R.grid_h = f->grid_h;
     R.grid_x0 = f->grid_x0; R.grid_y0 = f->grid_y0; R.cell = f->grid_cell;
-    if (pfd::refocus_smem_bytes(R) > 227 * 1024) return fail(ctx, PFD_EINVAL, "refocus: micro-image too large");
     CU(cudaMemcpyAsync(f->d_slice_vd, slice_vd, sizeof(float) * n_slices, cudaMemcpyHostToDevice, ctx->stream));
-    CU(pfd::launch_refocus(R, f->d_slice_vd, n_slices, f->W, f->H, out_w, out_h, f->d_stack, ctx->d_err, ctx->stream));
-    ctx->launches += 1;
+    cudaError_t e;
+    AsyncBuf quads(ctx->stream, pfd::refocus_quads_bytes(R), e);
+    if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, PFD_ENOMEM, "refocus: packed micro-images"); }
+    CU(pfd::launch_refocus(R, (uint32_t*)quads.p, f->d_slice_vd, n_slices, f->W, f->H, out_w, out_h, f->d_stack, ctx->d_err,
+                           ctx->stream));
+    ctx->launches += 2;
     if (out) CU(cudaMemcpyAsync(out, f->d_stack, need, cudaMemcpyDeviceToHost, ctx->stream));
     return out ? check_device_error(ctx) : PFD_OK;
 }

@@ -21,8 +21,9 @@ struct RefocusFrame {
 constexpr int kMaxRefocusCand = 2048;             // lenses that may reach one 64 x 16 output tile
 #define PFD_DEVERR_REFOCUS_LENSES 0x2             // a tile saw more than kMaxRefocusCand lenses
 
-int refocus_smem_bytes(const RefocusFrame& F);
-cudaError_t launch_refocus(const RefocusFrame& F, const float* slice_vd, int n_slices, int raw_w, int raw_h, int out_w,
-                           int out_h, float* out, int* err, cudaStream_t st);
+// Bytes of the packed micro-images a render lays out for itself.
+size_t refocus_quads_bytes(const RefocusFrame& F);
+cudaError_t launch_refocus(const RefocusFrame& F, uint32_t* quads, const float* slice_vd, int n_slices, int raw_w,
+                           int raw_h, int out_w, int out_h, float* out, int* err, cudaStream_t st);
 
 }  // namespace pfd
