@@ -151,7 +151,7 @@ struct Frame {
     // neighbour selection: the rings of the frame's lens grid, kept for the next call
     std::shared_ptr<RingPlan> rings;
     int2* d_pairs = nullptr;                   // rings->pairs on the device
-    int* d_sims = nullptr;                     // their similarities
+    uint16_t* d_sims = nullptr;                // their similarities (counts of a window's pixels)
     size_t n_pairs_alloc = 0;                  // entries d_pairs and d_sims hold
     // CUDA graphs of the enqueue-only PatchMatch and filter (pfd_set_graphs)
     FrameGraph pm_graph, filter_graph;
@@ -2211,35 +2211,39 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
 // d_out: the plan's pairs already on the device and room for their
 // similarities, or NULL to use temporary buffers.  out_ids [n][max_nb],
 // out_counts [n].
-static pfd_status select_lists(pfd_ctx* ctx, const RingPlan& rp, const int2* d_pairs, int* d_out,
+static pfd_status select_lists(pfd_ctx* ctx, const RingPlan& rp, const int2* d_pairs, uint16_t* d_out,
                                const uint8_t* d_img, int tile_stride, int mi_w, int mi_h, const float2* d_c,
                                int max_nb, int* out_ids, int* out_counts)
 {
     const int n_views = rp.G.V;
     cudaStream_t s = ctx->stream;
     const size_t np = rp.pairs.size();
-    std::vector<int> sims(np);
+    const std::unique_ptr<uint16_t[]> sims(new (std::nothrow) uint16_t[np + 1]);     // not zeroed: all of it is copied
+    if (!sims) return fail(ctx, PFD_ENOMEM, "select_neighbors: %zu similarities", np);
     int2* tp = nullptr;
-    int* to = nullptr;
+    uint16_t* to = nullptr;
     cudaError_t e = cudaSuccess;
     if (!d_pairs) {
         e = cudaMallocAsync((void**)&tp, sizeof(int2) * std::max<size_t>(np, 1), s);
-        if (e == cudaSuccess) e = cudaMallocAsync((void**)&to, sizeof(int) * std::max<size_t>(np, 1), s);
+        if (e == cudaSuccess) e = cudaMallocAsync((void**)&to, sizeof(uint16_t) * std::max<size_t>(np, 1), s);
         if (e == cudaSuccess && np)
             e = cudaMemcpyAsync(tp, rp.pairs.data(), sizeof(int2) * np, cudaMemcpyHostToDevice, s);
         d_pairs = tp;
         d_out = to;
     }
-    if (e == cudaSuccess) e = pfd::launch_similarity(d_img, tile_stride, mi_w, mi_h, d_c, d_pairs, (int)np, d_out, s);
-    if (e == cudaSuccess && np) e = cudaMemcpyAsync(sims.data(), d_out, sizeof(int) * np, cudaMemcpyDeviceToHost, s);
-    for (void* q : { (void*)tp, (void*)to })
+    void* rows = nullptr;
+    if (e == cudaSuccess) e = cudaMallocAsync(&rows, pfd::similarity_row_bytes(mi_w) * (size_t)n_views * mi_h, s);
+    if (e == cudaSuccess)
+        e = pfd::launch_similarity(d_img, tile_stride, mi_w, mi_h, n_views, rows, d_c, d_pairs, (int)np, d_out, s);
+    if (e == cudaSuccess && np) e = cudaMemcpyAsync(sims.get(), d_out, sizeof(uint16_t) * np, cudaMemcpyDeviceToHost, s);
+    for (void* q : { (void*)tp, (void*)to, rows })
         if (q) cudaFreeAsync(q, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return fail(ctx, PFD_ECUDA, "select_neighbors: %s", cudaGetErrorString(e));
     }
-    ctx->launches += 1;
+    ctx->launches += 2;
     pfd::parallel_views(n_views, [&](int a, int b) {
         std::vector<int> list;
         for (int v = a; v < b; ++v) {
@@ -2307,15 +2311,15 @@ pfd_status pfd_frame_select_neighbors(pfd_ctx* ctx, int frame_id, int mla_u_size
         if (!rp->build(f->h_centers.data(), f->h_keys.data(), f->V, mla_u_size, mla_v_size, pitch))
             return fail(ctx, PFD_EINVAL, "frame_select_neighbors: a tile key lies outside the grid or is repeated");
         if (f->d_pairs) { frame_free_one(ctx, *f, f->d_pairs, sizeof(int2) * f->n_pairs_alloc); f->d_pairs = nullptr; }
-        if (f->d_sims) { frame_free_one(ctx, *f, f->d_sims, sizeof(int) * f->n_pairs_alloc); f->d_sims = nullptr; }
+        if (f->d_sims) { frame_free_one(ctx, *f, f->d_sims, sizeof(uint16_t) * f->n_pairs_alloc); f->d_sims = nullptr; }
         const size_t np = std::max<size_t>(rp->pairs.size(), 1);
         f->n_pairs_alloc = np;
         void* p = nullptr;
         pfd_status st = frame_alloc(ctx, *f, &p, sizeof(int2) * np);
         if (st != PFD_OK) return st;
         f->d_pairs = (int2*)p;
-        if ((st = frame_alloc(ctx, *f, &p, sizeof(int) * np)) != PFD_OK) return st;
-        f->d_sims = (int*)p;
+        if ((st = frame_alloc(ctx, *f, &p, sizeof(uint16_t) * np)) != PFD_OK) return st;
+        f->d_sims = (uint16_t*)p;
         if (!rp->pairs.empty())
             CU(cudaMemcpyAsync(f->d_pairs, rp->pairs.data(), sizeof(int2) * rp->pairs.size(), cudaMemcpyHostToDevice,
                                ctx->stream));
