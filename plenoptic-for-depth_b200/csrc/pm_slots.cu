@@ -26,8 +26,13 @@
 // Bound by instruction issue: a warp-tap is about 40 instructions (3 loads, 18
 // FP32 operations, 6 integer products, 11 logical operations); packed pairs
 // (f32x2) halve the issue slots of the coordinates, measured 5% of the sweep.
-// Half-sweep, warp per pixel -> slots: 41 -> 28.1 ms (2048x1536, 12 neighbours,
-// 15x15), 8.0 -> 4.1 ms (1024x768, 6, 11x11), 27 -> 16.5 ms (2048x1536, ACMM, 5x5).
+// The scalar code is bound by latency: what it took from a round was mostly chains of
+// shuffles and loops that every lane ran.  So a plane, view, draw or candidate is one
+// lane's wherever its order does not matter, the ordered sums read shared memory, the
+// weight tables are filled by all warps and the finished pixels written by one.  Every
+// lane on the loops -> one lane each: 28.7 -> 27.3 ms, 4.1 -> 3.6, 16.7 -> 10.6.
+// Half-sweep, warp per pixel -> slots: 41 -> 27.3 ms (2048x1536, 12 neighbours,
+// 15x15), 8.0 -> 3.6 ms (1024x768, 6, 11x11), 27 -> 10.6 ms (2048x1536, ACMM, 5x5).
 #include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -61,6 +66,7 @@ struct __align__(16) SlotState {
     uint32_t slots;          // row of propagation slot s in bits [4s, 4s + 4)
     uint32_t tsel;           // selected views
     float best_cost;
+    float best_d;            // disparity of the best plane at the pixel
     int best_min;            // view of the lowest cost of the best plane
     int best_row;            // 0: the current plane is still the best
     int row_lo, row_hi;      // request: rows
@@ -70,10 +76,17 @@ struct __align__(16) SlotState {
     int n, hs;               // walk over the proposals: next one, its speculative row
     uint32_t flags;          // candidate flags (bits 0-7), kFlag*
 };
+// A finished pixel's new state on its way to memory (xy -1: none).
+struct __align__(16) SlotOut {
+    float4 plane;
+    float cost, d;
+    uint32_t sel;
+    int xy_view;             // x | y << 8 | (view of disp + 1) << 16, or -1
+};
 constexpr uint32_t kFlagChanged = 0x100u, kFlagPartial = 0x200u, kFlagSkip3 = 0x400u;
 
 // Where a slot's pixel stands: what the evaluation in flight is for.
-enum Stage : int { kIdle = 0, kNew, kProp, kSpec, kWalk, kRedo, kComplete, kWaits = 16 };
+enum Stage : int { kIdle = 0, kNew, kProp, kSpec, kWalk, kRedo, kComplete, kWaits = 16, kFresh = 32 };
 
 // Hypotheses one slot can hold: 9 propagation rows, or every selected view's
 // proposal, the 5 refinement candidates and one rebuilt proposal.
@@ -87,7 +100,7 @@ enum Ctl : int { kCtlItem = 0, kCtlPixel, kCtlTasks, kCtlPass, kCtlWords = 8 };
 struct SlotPlan {
     int off_ctl, off_Q, off_QB, off_R, off_RB, off_geo, off_ok, off_as, off_ac, off_pc, off_ps, off_bins, off_id, off_order;
     int off_stage, off_wtab, off_plane, off_dp, off_cost, off_bvec, off_wgt, off_wres, off_wmin, off_aux, off_sel, off_state,
-        off_stages;
+        off_out, off_stages;
     int rs, tx, ty, tab_n, rows, nbins, total;
 
     __host__ __device__ static int a16(int v) { return (v + 15) & ~15; }
@@ -129,6 +142,7 @@ struct SlotPlan {
         p.off_aux = o;   o += a16(slots * K * 2);
         p.off_sel = o;   o += a16(slots * K);
         p.off_state = o; o += slots * (int)sizeof(SlotState);
+        p.off_out = o;   o += slots * (int)sizeof(SlotOut);
         p.off_stages = o; o += 64 * 4;
         p.off_id = o;    o += a16(cap * 2);
         p.off_order = o; o += a16(cap * 2);
@@ -186,6 +200,15 @@ __device__ __forceinline__ float div255(float sb)
     const float r = 0x1.010102p-8f;                      // 1 / 255 rounded
     const float q = __fmul_rn(sb, r);
     return __fmaf_rn(__fmaf_rn(-q, 255.0f, sb), r, q);
+}
+
+// a / -0.18f, correctly rounded: the product with the rounded reciprocal and one fused
+// correction (Markstein); for a 0 or in the normal range.
+__device__ __forceinline__ float div_m018(float a)
+{
+    constexpr float v = -0.18f, y = 1.0f / -0.18f;
+    const float q = __fmul_rn(a, y);
+    return __fmaf_rn(__fmaf_rn(-q, v, a), y, q);
 }
 
 // The six moment sums of one NCC (and the blur sums).
@@ -564,6 +587,7 @@ struct View {
 // A slot's arrays.
 struct Slot {
     SlotState* st;
+    SlotOut* out;
     float* wtab;             // [tab_n] bilateral weights of the pixel's window, x outer
     float4* plane;           // [rows]
     float4* dp;              // [rows] disparity plane and the disparity at the pixel
@@ -584,6 +608,7 @@ __device__ __forceinline__ void weigh_rows(const Half& hf, const Slot& S, int K,
     const int n = nsel >= 0 ? nsel : nc;
     for (int h = lo + hf.hl; h < hi; h += 16) {
         WeightedCost wc;
+#pragma unroll 4
         for (int i = 0; i < n; ++i) {
             const int k = nsel >= 0 ? S.sel[i] : i;
             wc.add(k, S.cost[h * K + k], S.wgt[k]);
@@ -629,12 +654,12 @@ __device__ __forceinline__ void plane_rows(const Half& hf, const Slot& S, int lo
     }
 }
 
-// Takes pixel g: its weight table, the propagation candidates (AdaptMIPMFrame.cu:
-// 589-795) and the request for their costs.  Lane a < 8 works on direction a (up,
-// down, left, right; near on even lanes, far on odd ones).  Row 0 holds the
-// current plane, then one row per distinct candidate plane: a cost vector depends
-// only on the pixel and the plane.  The current plane's vector is the stored one
-// when that store is valid.
+// Takes pixel g: the propagation candidates (AdaptMIPMFrame.cu:589-795) and the
+// request for their costs (its weight table is made with the request's list).  Lane
+// a < 8 works on direction a (up, down, left, right; near on even lanes, far on odd
+// ones).  Row 0 holds the current plane, then one row per distinct candidate plane: a
+// cost vector depends only on the pixel and the plane.  The current plane's vector is
+// the stored one when that store is valid.
 __device__ __forceinline__ void begin_pixel(const Half& hf, const Slot& S, const View& V, const PmParams& P,
                                             const StateDev& prev, int g, int phase)
 {
@@ -643,15 +668,12 @@ __device__ __forceinline__ void begin_pixel(const Half& hf, const Slot& S, const
     nth_pixel(g, phase, W, x, y);
     const int center = y * W + x;
     const size_t idx = V.vbase + center;
-    {
-        const PixWin pw = slot_window(P, x, y);
-        const float rc = V.R[x * V.rs + y];
-        const int n = pw.nX * pw.nY;
-        const uint32_t magic = pw.nY > 1 ? 0xFFFFFFFFu / (uint32_t)pw.nY + 1u : 0u;
-        for (int t = hl; t < n; t += 16) {
-            const int ix = pw.nY > 1 ? (int)__umulhi((uint32_t)t, magic) : t, iy = t - ix * pw.nY;
-            S.wtab[t] = tap_weight(V.R, V.rs, V.a_s, V.a_c, P, pw, ix, iy, rc);
-        }
+    const float4 cur = prev.plane[idx];
+    const bool use_cvec = P.cvec_ok != 0;
+    float cv[2] = { 0.0f, 0.0f };
+    if (use_cvec) {
+        if (hl < V.nc) cv[0] = P.cvec[idx * P.K + hl];
+        if (hl + 16 < V.nc) cv[1] = P.cvec[idx * P.K + hl + 16];
     }
     const int a = hl & 7, dir = a >> 1;
     const bool vert = dir < 2, neg = (dir & 1) == 0;
@@ -679,16 +701,18 @@ __device__ __forceinline__ void begin_pixel(const Half& hf, const Slot& S, const
         const int s = pos;
         if (D > 3) take(cm, s + su);
     }
-    const float4 cur = prev.plane[idx];
     float4 q = cur;
     if (own) q = prev.plane[V.vbase + pos];
     const uint32_t flags = hf.ballot(D > 0) & 0xFFu, owns = hf.ballot(own) & 0xFFu;
+    // the first earlier lane with the same plane; the planes side by side in the dp rows,
+    // which are not in use yet
+    if (hl < 8) S.dp[hl] = q;
+    hf.sync();
     const bool eqcur = same_bits(q, cur);
     int match = -1;
-    for (int t = 0; t < 7; ++t) {
-        const float4 o = make_float4(hf.shfl(q.x, t), hf.shfl(q.y, t), hf.shfl(q.z, t), hf.shfl(q.w, t));
-        if (match < 0 && t < a && ((owns >> t) & 1u) && same_bits(o, q)) match = t;
-    }
+#pragma unroll
+    for (int t = 6; t >= 0; --t)
+        if (t < a && ((owns >> t) & 1u) && same_bits(S.dp[t], q)) match = t;
     const bool lead = own && hl < 8 && !eqcur && match < 0;
     const uint32_t leads = hf.ballot(lead);
     int row = lead ? 1 + __popc(hf.below(leads)) : 0;
@@ -698,9 +722,10 @@ __device__ __forceinline__ void begin_pixel(const Half& hf, const Slot& S, const
     if (!own) row = (D > 0) ? nrow : 0;
     if (lead) S.plane[row] = q;
     const uint32_t slots = __reduce_or_sync(hf.mask, hl < 8 ? (uint32_t)row << (4 * hl) : 0u);
-    const bool use_cvec = P.cvec_ok != 0;
-    if (use_cvec)
-        for (int k = hl; k < V.nc; k += 16) S.cost[k] = P.cvec[idx * P.K + k];
+    if (use_cvec) {
+        if (hl < V.nc) S.cost[hl] = cv[0];
+        if (hl + 16 < V.nc) S.cost[hl + 16] = cv[1];
+    }
     if (hl == 0) {
         S.plane[0] = cur;
         S.st->xy = x | (y << 8);
@@ -709,7 +734,44 @@ __device__ __forceinline__ void begin_pixel(const Half& hf, const Slot& S, const
         request(*S.st, use_cvec ? 1 : 0, 1 + __popc(leads), 0ull, -1);
     }
     hf.sync();
-    plane_rows(hf, S, use_cvec ? 1 : 0, 1 + __popc(leads), x, y);
+    plane_rows(hf, S, 0, 1 + __popc(leads), x, y);
+}
+
+// BuildCrossViewPlaneProposal (AdaptMIPMFrame.cu:350-398): the sample position (x | y
+// << 8) of pixel (x, y) at disparity d in neighbour gk, or -1; and the plane from the
+// neighbour's plane hn there.
+__device__ __forceinline__ int proposal_at(const NbGeo& gk, int x, int y, int W, int H, float d)
+{
+    const float2 qf = geo_anchor(gk, x, y, d);
+    const float fqx = floorf(__fadd_rn(qf.x, 0.5f)), fqy = floorf(__fadd_rn(qf.y, 0.5f));
+    if (!(fqx >= 0.0f && fqx < (float)W && fqy >= 0.0f && fqy < (float)H)) return -1;
+    return (int)fqx | ((int)fqy << 8);
+}
+
+__device__ __forceinline__ float4 proposal_from(const NbGeo& gk, float4 hn, int q, int x, int y)
+{
+    const float3 dpn = disparity_plane(q & 0xFF, q >> 8, hn);
+    float denom = __fmaf_rn(dpn.y, gk.by, __fmaf_rn(dpn.x, gk.bx, 1.0f));
+    denom = safe_denom(denom);
+    return encode_plane(x, y, __fdiv_rn(dpn.x, denom), __fdiv_rn(dpn.y, denom), __fdiv_rn(dpn.z, denom));
+}
+
+// The five candidates of PlaneHypothesisRefinement_Frame (AdaptMIPMFrame.cu:400-471)
+// for the best plane, from the draws already taken (c0: the random plane, rn: the
+// random normal, u1-u3: the perturbation, u4: the depth perturbation), those from
+// `from` on into rows r0 + i, one lane each.  Returns whether candidate 3 equals the
+// best plane.  The caller synchronises before the rows are read.
+__device__ __forceinline__ bool refine_rows(const Half& hf, const Slot& S, int x, int y, float4 best, float4 c0, float4 rn,
+                                            float u1, float u2, float u3, float u4, float pert, int r0, int from)
+{
+    const float4 pn = perturbed_normal_u(x, y, best, u1, u2, u3, pert);
+    const float dmin_p = __fmul_rn(__fsub_rn(1.0f, 0.02f), best.w), dmax_p = __fmul_rn(__fadd_rn(1.0f, 0.02f), best.w);
+    const int i = hf.hl;
+    float4 c = i == 0 ? c0 : (i == 1 ? rn : (i == 2 ? pn : best));
+    if (i == 4) c.w = __fmaf_rn(u4, __fsub_rn(dmax_p, dmin_p), dmin_p);
+    if (i > 0) c.w = to_disparity(x, y, disparity_plane(x, y, c));
+    if (i >= from && i < 5) S.plane[r0 + i] = c;
+    return __float_as_uint(hf.shfl(c.w, 3)) == __float_as_uint(best.w);
 }
 
 // After the propagation costs: view-selection priors and sampling (AdaptMIPMFrame.cu:
@@ -727,55 +789,68 @@ __device__ __forceinline__ void after_propagation(const Half& hf, const Slot& S,
     HalfDraws g(hf, P.seed, sweep_id, (uint32_t)(V.vbase + center));
     const int dpos[4] = { (y > 0) ? center - W : -1, (y < H - 1) ? center + W : -1, (x > 0) ? center - 1 : -1,
                           (x < W - 1) ? center + 1 : -1 };
-    float pr[2] = { 0.0f, 0.0f };
+    // one view per lane (two above 16 views)
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
         const int i = hl + 16 * half;
+        if (16 * half >= nc) break;
         if (i >= nc) continue;
         float prior = 0.0f;
-        for (int ii = 0; ii < 4; ++ii) {
-            if (dpos[ii] < 0) continue;
-            prior = __fadd_rn(prior, ((V.ps[dpos[ii]] >> i) & 1u) ? 0.9f : 0.1f);
-        }
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii)
+            if (dpos[ii] >= 0) prior = __fadd_rn(prior, ((V.ps[dpos[ii]] >> i) & 1u) ? 0.9f : 0.1f);
+        // the terms side by side, then their sum in order (a term that does not count is
+        // +0, which leaves the sum as it is)
         float count = 0.0f, tmpw = 0.0f, p = 0.0f;
         int count_false = 0;
+#pragma unroll
         for (int j = 0; j < 8; ++j) {
-            if (!((flags >> j) & 1u)) continue;
+            const bool there = (flags >> j) & 1u;
             const float c = S.cost[(int)((slots >> (4 * j)) & 15u) * K + i];
-            if (c < thr) {
-                tmpw = __fadd_rn(tmpw, pfd_expf(__fdiv_rn(__fmul_rn(c, c), -0.18f)));
-                count = __fadd_rn(count, 1.0f);
-            }
-            if (c > 1.2f) count_false++;
+            const bool low = there && c < thr;
+            const float e = pfd_expf_nonpos(div_m018(__fmul_rn(c, c)));
+            tmpw = __fadd_rn(tmpw, low ? e : 0.0f);
+            count = __fadd_rn(count, low ? 1.0f : 0.0f);
+            count_false += there && c > 1.2f;
         }
         if (count > 2.0f && count_false < 3) p = __fdiv_rn(tmpw, count);
         else if (count_false < 3) p = p_default;
-        pr[half] = __fmul_rn(p, prior);
+        S.wgt[i] = __fmul_rn(p, prior);
     }
-    // the sums over views run in view order, as the reference's loops do
-    float psum = 0.0f;
-    for (int i = 0; i < nc; ++i) psum = __fadd_rn(psum, hf.shfl(i < 16 ? pr[0] : pr[1], i & 15));
+    hf.sync();
+    // the sums over views run in view order, as the reference's loops do;
     // TransformPDFToCDF (CudaUtil.cu:491-507) and the 15 draws, one per lane: a draw's
-    // view is the first whose CDF exceeds it
+    // view is the first whose CDF exceeds it (a CDF of NaN, all probabilities 0, exceeds
+    // nothing)
+    float psum = 0.0f;
+#pragma unroll 4
+    for (int i = 0; i < nc; ++i) psum = __fadd_rn(psum, S.wgt[i]);
+    const float inv = __fdiv_rn(1.0f, psum);
+    const float rp = __fsub_rn(g.d0, 1.1920928955078125e-07f);
+    float cum = 0.0f;
+    int id = 0;
+    bool over = false;
+#pragma unroll 4
+    for (int i = 0; i < nc; ++i) {
+        cum = __fmaf_rn(S.wgt[i], inv, cum);
+        over |= cum > rp;
+        id += !over;
+    }
+    hf.sync();                                           // the probabilities are read before they are replaced
+    // draws per view, 4 bits each (at most 15), added up over the lanes
     uint32_t tsel = 0;
     {
-        const float inv = __fdiv_rn(1.0f, psum);
-        const float rp = __fsub_rn(g.d0, 1.1920928955078125e-07f);
-        bool open = hl < 15;
-        float cum = 0.0f;
-        int c0 = 0, c1 = 0;                              // draws of this lane's views hl and 16 + hl
-        for (int i = 0; i < nc; ++i) {
-            cum = __fmaf_rn(hf.shfl(i < 16 ? pr[0] : pr[1], i & 15), inv, cum);
-            const bool hit = open && cum > rp;
-            open = open && !hit;
-            const uint32_t hits = hf.ballot(hit);
-            if (hits) tsel |= 1u << i;
-            if (hl == (i & 15)) { if (i < 16) c0 = __popc(hits); else c1 = __popc(hits); }
+        const uint32_t one = hl < 15 && id < nc ? 1u << (4 * (id & 7)) : 0u;
+        uint32_t n0 = __reduce_add_sync(hf.mask, (id >> 3) == 0 ? one : 0u);
+        uint32_t n1 = __reduce_add_sync(hf.mask, (id >> 3) == 1 ? one : 0u), n2 = 0u, n3 = 0u;
+        if (nc > 16) {
+            n2 = __reduce_add_sync(hf.mask, (id >> 3) == 2 ? one : 0u);
+            n3 = __reduce_add_sync(hf.mask, (id >> 3) == 3 ? one : 0u);
         }
-        if (tsel == 0) {
-            tsel = nc < 32 ? (1u << nc) - 1u : ~0u;
-            c0 = c1 = 1;
-        }
+        if ((n0 | n1 | n2 | n3) == 0u) n0 = n1 = n2 = n3 = 0x11111111u;        // no draw hit: every view once
+        const int c0 = (int)(((hl < 8 ? n0 : n1) >> (4 * (hl & 7))) & 15u), c1 = (int)(((hl < 8 ? n2 : n3) >> (4 * (hl & 7))) & 15u);
+        tsel = hf.ballot(hl < nc && c0 > 0);
+        if (nc > 16) tsel |= hf.ballot(16 + hl < nc && c1 > 0) << 16;
         if (hl < nc) {
             S.wgt[hl] = (float)c0;
             if ((tsel >> hl) & 1u) S.sel[__popc(tsel & ((1u << hl) - 1u))] = (uint8_t)hl;
@@ -786,52 +861,82 @@ __device__ __forceinline__ void after_propagation(const Half& hf, const Slot& S,
         }
         hf.sync();
     }
-    g.n = 15;
     const int nh = st.row_hi;
     weigh_rows(hf, S, K, 0, nh, nc, -1);
     // current plane, then the candidates in slot order
     float best_cost = S.wres[0];
     int best_row = 0;
+#pragma unroll
     for (int s = 0; s < 8; ++s) {
-        if (!((flags >> s) & 1u)) continue;
         const int r = (int)((slots >> (4 * s)) & 15u);
         const float c = S.wres[r];
-        if (c < best_cost) { best_cost = c; best_row = r; }
+        if (((flags >> s) & 1u) && c < best_cost) { best_cost = c; best_row = r; }
     }
     const int best_min = S.wmin[best_row];
     const float4 best_plane = S.plane[best_row];
+    const float best_d = S.dp[best_row].w;
     for (int k = hl; k < nc; k += 16) S.bvec[k] = S.cost[best_row * K + k];
-    (void)g.uniform();                                   // depth_rand: drawn, never used
-    const float4 rn = random_normal(g);
-    const float u1 = g.uniform(), u2 = g.uniform(), u3 = g.uniform();
-    const float u4 = g.uniform();
-    const float4 c0 = random_plane(g, P.depth_min, P.depth_max);
+    // the refinement's draws: 15 (depth_rand: drawn, never used), a normal by rejection
+    // from pairs of draws 16 on, four uniforms, a depth, another normal.  Lanes 0-7 try
+    // the pairs from even draws and lanes 8-14 those from odd draws side by side; the
+    // first normal is the first accepted even pair, the second the first accepted odd
+    // pair after the five draws between.
+    float4 rn, c0;
+    float u1, u2, u3, u4;
+    {
+        const int first = hl < 8 ? 2 * hl : 2 * hl - 15;
+        const float q1 = __fmaf_rn(2.0f, hf.shfl(g.d1, first & 15), -1.0f);
+        const float q2 = __fmaf_rn(2.0f, hf.shfl(g.d1, (first + 1) & 15), -1.0f);
+        const float ss = __fmaf_rn(q2, q2, __fmul_rn(q1, q1));
+        const uint32_t good = hf.ballot(hl < 15 && ss < 1.0f);
+        const int a1 = __ffs(good & 0xFFu) - 1;
+        const uint32_t odd = a1 >= 0 ? (good >> 8) & ~((1u << (a1 + 3)) - 1u) : 0u;
+        if (odd) {
+            const float sq = __fsqrt_rn(__fsub_rn(1.0f, ss));
+            const float4 n = normalize3(make_float4(__fmul_rn(__fmul_rn(2.0f, q1), sq), __fmul_rn(__fmul_rn(2.0f, q2), sq),
+                                                    __fmaf_rn(-2.0f, ss, 1.0f), 0.0f));
+            const int b1 = 7 + __ffs(odd), at = 2 * a1 + 2;
+            rn = make_float4(hf.shfl(n.x, a1), hf.shfl(n.y, a1), hf.shfl(n.z, a1), 0.0f);
+            u1 = hf.shfl(g.d1, at);
+            u2 = hf.shfl(g.d1, at + 1);
+            u3 = hf.shfl(g.d1, at + 2);
+            u4 = hf.shfl(g.d1, at + 3);
+            const float depth = __fmaf_rn(hf.shfl(g.d1, at + 4), __fsub_rn(P.depth_max, P.depth_min), P.depth_min);
+            c0 = make_float4(hf.shfl(n.x, b1), hf.shfl(n.y, b1), hf.shfl(n.z, b1), depth);
+        } else {                                         // more than 16 draws: one after another
+            g.n = 16;
+            rn = random_normal(g);
+            u1 = g.uniform();
+            u2 = g.uniform();
+            u3 = g.uniform();
+            u4 = g.uniform();
+            c0 = random_plane(g, P.depth_min, P.depth_max);
+        }
+    }
     hf.sync();                                           // every lane has read the rows before they are reused
     const int nsel = __popc(tsel);
     int nact = 0;
     for (int n0 = 0; n0 < nsel; n0 += 16) {
         const int n = n0 + hl;
-        int q = -1, k = -1, nvid = -1;
+        int q = -1, k = 0, nvid = -1;
         if (n < nsel) {
             k = S.sel[n];
             nvid = F.nb_ids[V.vid * K + k];
-            if (nvid >= 0) q = proposal_pos(V.geo[k], x, y, W, H, best_plane);
+            if (nvid >= 0) q = proposal_at(V.geo[k], x, y, W, H, best_d);
         }
         const uint32_t act = hf.ballot(q >= 0);
         if (q >= 0)
             S.plane[nact + __popc(hf.below(act))] =
-                proposal_plane(V.geo[k], prev.plane + (size_t)nvid * P.ppv, q, x, y, W);
+                proposal_from(V.geo[k], prev.plane[(size_t)nvid * P.ppv + (q >> 8) * W + (q & 0xFF)], q, x, y);
         if (n < nsel) S.aux[n] = (int16_t)q;
         nact += __popc(act);
     }
-    float4 cand[5];
-    refine_candidates(x, y, best_plane, c0, rn, u1, u2, u3, u4, P.pert_pi, cand);
     // the candidate equal to the best plane has the best cost and cannot win
-    const bool skip3 = __float_as_uint(cand[3].w) == __float_as_uint(best_plane.w);
+    const bool skip3 = refine_rows(hf, S, x, y, best_plane, c0, rn, u1, u2, u3, u4, P.pert_pi, nact, 0);
     if (hl == 0) {
-        for (int i = 0; i < 5; ++i) S.plane[nact + i] = cand[i];
         st.best_plane = best_plane;
         st.best_cost = best_cost;
+        st.best_d = best_d;
         st.best_min = best_min;
         st.best_row = best_row;
         st.c0 = c0;
@@ -860,31 +965,50 @@ __device__ __forceinline__ int after_speculation(const Half& hf, const Slot& S, 
     const int x = st.xy & 0xFF, y = st.xy >> 8;
     const int nsel = __popc(st.tsel), r0 = st.r0;
     weigh_rows(hf, S, K, st.row_lo, st.row_hi, nc, nsel);
-    float best_cost = st.best_cost;
+    float best_cost = st.best_cost, best_d = st.best_d;
     float4 best_plane = st.best_plane;
     int best_min = st.best_min, n = st.n, hs = st.hs;
     uint32_t flags = st.flags;
     hf.sync();
+    if (stage == kSpec) {
+        // nothing changes before the first proposal that wins: the lanes look for it side
+        // by side
+        for (int n0 = 0; n0 < nsel; n0 += 16) {
+            const bool act = n0 + hl < nsel && S.aux[n0 + hl] >= 0;
+            const uint32_t acts = hf.ballot(act);
+            const uint32_t wins = hf.ballot(act && S.wres[hs + __popc(hf.below(acts))] < best_cost);
+            if (wins) {
+                const int w = __ffs(wins) - 1;
+                n = n0 + w;
+                hs += __popc(acts & ((1u << w) - 1u));
+                break;
+            }
+            hs += __popc(acts);
+            n = nsel;
+        }
+    }
     if (stage != kRedo) {
         bool resumed = stage == kWalk;
         for (; n < nsel; ++n) {
             const int spec_q = S.aux[n];
-            int q = spec_q, k = -1, nvid = -1;
+            int q = spec_q, k = 0, nvid = -1;
             if (flags & kFlagChanged) {
                 k = S.sel[n];
                 nvid = F.nb_ids[V.vid * K + k];
-                q = (nvid >= 0) ? proposal_pos(V.geo[k], x, y, W, H, best_plane) : -1;
+                q = (nvid >= 0) ? proposal_at(V.geo[k], x, y, W, H, best_d) : -1;
             }
             if (q >= 0) {
                 const int row = (spec_q >= 0) ? hs : r0 + 5;
                 if (q != spec_q && !resumed) {
                     // the best plane moved the sample position: rebuild this proposal in its
                     // own row (or the spare row after the refinement candidates)
-                    const float4 proxy = proposal_plane(V.geo[k], prev.plane + (size_t)nvid * P.ppv, q, x, y, W);
+                    const float4 proxy =
+                        proposal_from(V.geo[k], prev.plane[(size_t)nvid * P.ppv + (q >> 8) * W + (q & 0xFF)], q, x, y);
                     if (hl == 0) {
                         S.plane[row] = proxy;
                         st.best_plane = best_plane;
                         st.best_cost = best_cost;
+                        st.best_d = best_d;
                         st.best_min = best_min;
                         st.n = n;
                         st.hs = hs;
@@ -899,6 +1023,7 @@ __device__ __forceinline__ int after_speculation(const Half& hf, const Slot& S, 
                 if (c < best_cost) {
                     best_cost = c;
                     best_plane = S.plane[row];
+                    best_d = S.dp[row].w;
                     best_min = S.wmin[row];
                     flags |= kFlagChanged | kFlagPartial;
                 }
@@ -908,15 +1033,14 @@ __device__ __forceinline__ int after_speculation(const Half& hf, const Slot& S, 
         }
         if (flags & kFlagChanged) {
             // candidates 2-4 follow the best plane: rebuild and evaluate them again
-            float4 cand[5];
-            refine_candidates(x, y, best_plane, st.c0, st.rn, st.u.x, st.u.y, st.u.z, st.u.w, P.pert_pi, cand);
-            const bool skip3 = __float_as_uint(cand[3].w) == __float_as_uint(best_plane.w);
-            flags = (flags & ~kFlagSkip3) | (skip3 ? kFlagSkip3 : 0u);
             hf.sync();                                   // proposal rows may be read above
+            const bool skip3 = refine_rows(hf, S, x, y, best_plane, st.c0, st.rn, st.u.x, st.u.y, st.u.z, st.u.w, P.pert_pi,
+                                           r0, 2);
+            flags = (flags & ~kFlagSkip3) | (skip3 ? kFlagSkip3 : 0u);
             if (hl == 0) {
-                for (int i = 2; i < 5; ++i) S.plane[r0 + i] = cand[i];
                 st.best_plane = best_plane;
                 st.best_cost = best_cost;
+                st.best_d = best_d;
                 st.best_min = best_min;
                 st.flags = flags;
                 request(st, r0 + 2, r0 + 5, skip3 ? (1ull << (r0 + 3)) : 0ull, nsel);
@@ -926,13 +1050,17 @@ __device__ __forceinline__ int after_speculation(const Half& hf, const Slot& S, 
             return kRedo;
         }
     }
-    for (int i = 0; i < 5; ++i) {
-        if (i == 3 && (flags & kFlagSkip3)) continue;
-        const float c = S.wres[r0 + i];
-        if (c < best_cost) {
-            best_cost = c;
-            best_plane = S.plane[r0 + i];
-            best_min = S.wmin[r0 + i];
+    {
+        int won = -1;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const float c = S.wres[r0 + i];
+            if (!(i == 3 && (flags & kFlagSkip3)) && c < best_cost) { best_cost = c; won = i; }
+        }
+        if (won >= 0) {
+            best_plane = S.plane[r0 + won];
+            best_d = S.dp[r0 + won].w;
+            best_min = S.wmin[r0 + won];
             flags |= kFlagPartial;
         }
     }
@@ -943,6 +1071,7 @@ __device__ __forceinline__ int after_speculation(const Half& hf, const Slot& S, 
     if (hl == 0) {
         st.best_plane = best_plane;
         st.best_cost = best_cost;
+        st.best_d = best_d;
         st.best_min = best_min;
         st.flags = flags;
         if (flags & kFlagPartial) {
@@ -956,69 +1085,82 @@ __device__ __forceinline__ int after_speculation(const Half& hf, const Slot& S, 
     return kComplete;
 }
 
-// Writes the pixel's new state.  completed: row 0 holds the winner's cost vector
-// (a proposal or refinement candidate won); otherwise bvec does.
+// The pixel's new state into the slot's out record.  completed: row 0 holds the
+// winner's cost vector (a proposal or refinement candidate won); otherwise bvec does.
 __device__ __forceinline__ void finish_pixel(const Half& hf, const Slot& S, const View& V, const PmParams& P,
-                                             const StateDev& next, bool completed)
+                                             bool completed)
 {
     const int K = P.K, nc = V.nc, hl = hf.hl, W = P.W;
     SlotState& st = *S.st;
     const int x = st.xy & 0xFF, y = st.xy >> 8;
     const size_t idx = V.vbase + y * W + x;
-    int best_min = st.best_min, best_row = st.best_row;
-    const float* vec = S.bvec;
-    if (completed) {
-        weigh_rows(hf, S, K, 0, 1, nc, -1);
-        best_min = S.wmin[0];
-        best_row = -1;
-        vec = S.cost;
-    }
+    const float* vec = completed ? S.cost : S.bvec;
+    const float v0 = hl < nc ? vec[hl] : 2.0f, v1 = 16 + hl < nc ? vec[16 + hl] : 2.0f;
     // the stored vector of the new current plane (unchanged when the current
     // plane stays and its stored vector was used)
-    if (P.cvec && !(best_row == 0 && P.cvec_ok))
-        for (int k = hl; k < nc; k += 16) P.cvec[idx * K + k] = vec[k];
-    if (hl == 0) {
-        const float4 best_plane = st.best_plane;
-        uint32_t sel_out = st.tsel;
-        float cost_out = st.best_cost;
-        int disp_view = best_min;
-        if (P.acmm) {
-            // ACMM write-back (AdaptMIPMFrameACMM.cu:880-900, RecomputeSupportCostDisp_Frame
-            // :259-280): the final plane's vector over every view gives the stored cost
-            // (mean of the top-k), the selected views (the top-k mask) and the disp of the
-            // lowest-cost view; DetailRestorer_FrameACMM does nothing without a warm start
-            disp_view = -1;
-            int valid = 0;
-            for (int i = 0; i < nc; ++i)
-                if (vec[i] < 2.0f) {
-                    ++valid;
-                    if (disp_view < 0 || vec[i] < vec[disp_view]) disp_view = i;
-                }
-            cost_out = 2.0f;
-            sel_out = 0;
-            if (valid > 0) {
-                const int kk = min(valid, P.top_k);
-                float* tmp = S.cost + K;                 // row 1: free by now
-                for (int i = 0; i < nc; ++i) tmp[i] = vec[i];
-                for (int i = 0; i < kk; ++i)
-                    for (int j = i + 1; j < nc; ++j)
-                        if (tmp[j] < tmp[i]) { const float t = tmp[i]; tmp[i] = tmp[j]; tmp[j] = t; }
-                float m = 0.0f;
-                for (int i = 0; i < kk; ++i) m = __fadd_rn(m, tmp[i]);
-                cost_out = __fdiv_rn(m, (float)kk);
-                for (int i = 0; i < nc; ++i)
-                    if (vec[i] <= tmp[kk - 1]) sel_out |= 1u << i;
+    if (P.cvec && (completed || st.best_row != 0 || !P.cvec_ok)) {
+        if (hl < nc) P.cvec[idx * K + hl] = v0;
+        if (16 + hl < nc) P.cvec[idx * K + 16 + hl] = v1;
+    }
+    uint32_t sel_out = st.tsel;
+    float cost_out = st.best_cost;
+    int disp_view = st.best_min;
+    if (completed || P.acmm) {
+        // the first view of the lowest cost, among the costs below 2 (-1: none)
+        uint32_t low = min(v0 < 2.0f ? __float_as_uint(v0) : 0x40000000u, v1 < 2.0f ? __float_as_uint(v1) : 0x40000000u);
+        low = __reduce_min_sync(hf.mask, low);           // costs are >= 0: their bits order as they do
+        const uint32_t at = hf.ballot(__float_as_uint(v0) == low) | (hf.ballot(__float_as_uint(v1) == low) << 16);
+        disp_view = low < 0x40000000u ? __ffs(at) - 1 : -1;
+    }
+    if (P.acmm) {
+        // ACMM write-back (AdaptMIPMFrameACMM.cu:880-900, RecomputeSupportCostDisp_Frame
+        // :259-280): the final plane's vector over every view gives the stored cost
+        // (mean of the top-k), the selected views (the top-k mask) and the disp of the
+        // lowest-cost view; DetailRestorer_FrameACMM does nothing without a warm start
+        const int valid = __popc(hf.ballot(hl < nc && v0 < 2.0f)) + __popc(hf.ballot(16 + hl < nc && v1 < 2.0f));
+        cost_out = 2.0f;
+        sel_out = 0;
+        if (valid > 0) {
+            // the k smallest in ascending order: the lowest left, every time
+            const int kk = min(valid, P.top_k);
+            uint32_t b0 = hl < nc ? __float_as_uint(v0) : 0xffffffffu, b1 = 16 + hl < nc ? __float_as_uint(v1) : 0xffffffffu;
+            float m = 0.0f;
+            uint32_t low = 0u;
+            for (int i = 0; i < kk; ++i) {
+                low = __reduce_min_sync(hf.mask, min(b0, b1));
+                m = __fadd_rn(m, __uint_as_float(low));
+                const int lane = __ffs(hf.ballot(b0 == low || b1 == low)) - 1;
+                if (hl == lane) { if (b0 == low) b0 = 0xffffffffu; else b1 = 0xffffffffu; }
             }
+            cost_out = __fdiv_rn(m, (float)kk);
+            const float thr = __uint_as_float(low);
+            sel_out = hf.ballot(hl < nc && v0 <= thr) | (hf.ballot(16 + hl < nc && v1 <= thr) << 16);
         }
-        float4 best_disp = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (disp_view >= 0)
-            best_disp = geo_disp(V.geo[disp_view], x, y, to_disparity(x, y, disparity_plane(x, y, best_plane)));
-        next.plane[idx] = best_plane;
-        next.cost[idx] = cost_out;
-        next.disp[idx] = best_disp;
-        next.sel[idx] = sel_out;
+    }
+    if (hl == 0) {
+        S.out->plane = st.best_plane;
+        S.out->cost = cost_out;
+        S.out->d = st.best_d;
+        S.out->sel = sel_out;
+        S.out->xy_view = x | (y << 8) | ((disp_view + 1) << 16);
     }
     hf.sync();
+}
+
+// Writes a finished pixel's state (one lane per slot) and clears the record.
+__device__ __forceinline__ void write_out(SlotOut& o, const View& V, const PmParams& P, const StateDev& next)
+{
+    const int xv = o.xy_view;
+    if (xv < 0) return;
+    const int x = xv & 0xFF, y = (xv >> 8) & 0xFF, view = (xv >> 16) - 1;
+    const size_t idx = V.vbase + y * P.W + x;
+    float4 disp = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (view >= 0) disp = geo_disp(V.geo[view], x, y, o.d);
+    next.plane[idx] = o.plane;
+    next.cost[idx] = o.cost;
+    next.disp[idx] = disp;
+    next.sel[idx] = o.sel;
+    o.xy_view = -1;
 }
 
 }  // namespace
@@ -1063,6 +1205,7 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
     auto slot_at = [&](int s) {
         Slot S;
         S.st = (SlotState*)(smem + L.off_state) + s;
+        S.out = (SlotOut*)(smem + L.off_out) + s;
         S.wtab = (float*)(smem + L.off_wtab) + s * L.tab_n;
         S.plane = (float4*)(smem + L.off_plane) + s * L.rows;
         S.dp = (float4*)(smem + L.off_dp) + s * L.rows;
@@ -1157,7 +1300,11 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
         expand_tiles<BLUR>(D, P, nc);
         __syncthreads();
         // stage of every slot; a slot whose request did not fit the list keeps it (kWaits set)
-        if (tid < 32) { stages[tid] = tid < n_slots ? kNew : kIdle; next_stages[tid] = kIdle; }
+        if (tid < 32) {
+            stages[tid] = tid < n_slots ? kNew : kIdle;
+            next_stages[tid] = kIdle;
+            if (tid < n_slots) slot_at(tid).out->xy_view = -1;
+        }
         __syncthreads();
 
         for (;;) {
@@ -1187,11 +1334,11 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
                         stage = kSpec;
                     } else {
                         if (stage == kComplete) {
-                            finish_pixel(hf, S, V, P, next, true);
+                            finish_pixel(hf, S, V, P, true);
                             stage = kNew;
                         } else if (stage != kNew) {
                             stage = after_speculation(hf, S, V, F, P, prev, stage);
-                            if (stage == kNew) finish_pixel(hf, S, V, P, next, false);
+                            if (stage == kNew) finish_pixel(hf, S, V, P, false);
                         }
                         if (stage == kNew) {
                             int g = 0;
@@ -1199,7 +1346,7 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
                             g = hf.shfl(g, 0);
                             if (g < g_hi) {
                                 begin_pixel(hf, S, V, P, prev, g, phase);
-                                stage = kProp;
+                                stage = kProp | kFresh;
                             } else {
                                 stage = kIdle;
                             }
@@ -1214,13 +1361,36 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
             // ---- the requests' NCCs into the list, 32 (row, view) pairs per warp at a time.
             // Slots whose pairs do not fit the list wait for the next round.
             {
-                const int stage = next_stages[lane];
+                const int entered = next_stages[lane], stage = entered & ~kFresh;
                 int pairs = 0;
                 if (stage != kIdle) {
                     const SlotState& st = *slot_at(lane).st;
                     pairs = (st.row_hi - st.row_lo) * (st.n_views >= 0 ? st.n_views : nc);
                 }
+                if (warp == WARPS - 1 && lane < n_slots) write_out(*slot_at(lane).out, V, P, next);
                 if (!__any_sync(kFullMask, stage != kIdle)) break;       // the same in every warp
+                // weight tables of the pixels just taken, 32 taps per warp at a time
+                {
+                    const int chunks = (L.tab_n + 31) >> 5;
+                    uint32_t left = __ballot_sync(kFullMask, (entered & kFresh) != 0);
+                    for (int i = 0; left; left &= left - 1, ++i) {
+                        const int slot = __ffs(left) - 1, xy = slot_at(slot).st->xy, x = xy & 0xFF, y = xy >> 8;
+                        // chunk c of the i-th such slot belongs to warp (i chunks + c) mod WARPS
+                        const int u = (warp + WARPS - (i * chunks) % WARPS) % WARPS;
+                        if (u >= chunks) continue;
+                        const PixWin pw = slot_window(P, x, y);
+                        const float rc = R[x * L.rs + y];
+                        const int n = pw.nX * pw.nY;
+                        const uint32_t magic = pw.nY > 1 ? 0xFFFFFFFFu / (uint32_t)pw.nY + 1u : 0u;
+                        float* wtab = slot_at(slot).wtab;
+                        for (int c = u; c < chunks; c += WARPS) {
+                            const int t = c * 32 + lane;
+                            if (t >= n) continue;
+                            const int ix = pw.nY > 1 ? (int)__umulhi((uint32_t)t, magic) : t, iy = t - ix * pw.nY;
+                            wtab[t] = tap_weight(R, L.rs, V.a_s, V.a_c, P, pw, ix, iy, rc);
+                        }
+                    }
+                }
                 int upto = pairs;
                 for (int o = 1; o < 32; o <<= 1) {
                     const int t = __shfl_up_sync(kFullMask, upto, o);
