@@ -1395,7 +1395,10 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
         const int iter = s / 2, phase = s % 2;
         std::fill(count.begin(), count.end(), 0);
         items.clear();
-        for (size_t grp = 0; grp < groups.size(); ++grp)
+        for (size_t grp = 0; grp < groups.size(); ++grp) {
+            int views = 0;                             // of the launch: its frames share the CTAs
+            for (int b : groups[grp].members)
+                if (s < 2 * params[b].max_iterations) views += fr[b]->V;
             for (int b : groups[grp].members) {
                 Frame& f = *fr[b];
                 if (s >= 2 * params[b].max_iterations) continue;
@@ -1405,7 +1408,7 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
                 it.P.cost_scratch = ctx->d_scratch;
                 it.P.scratch_floats = ctx->scratch_bytes / sizeof(float);
                 it.P.scratch_stride = stride;
-                if (!groups[grp].tex) pfd::slots_plan(it.P, groups[grp].blur == 1, groups[grp].shape, f.V);
+                if (!groups[grp].tex) pfd::slots_plan(it.P, groups[grp].blur == 1, groups[grp].shape, views);
                 it.P.cvec_ok = cvec_usable(f, params[b], phase, mode);
                 it.P.view_queue = d_queues + (size_t)s * n + items.size();
                 it.prev = f.s[f.cur];
@@ -1417,6 +1420,7 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
                 f.cur ^= 1;
                 cvec_swept(f, params[b], phase, mode);
             }
+        }
         pfd::SweepItem* row = d_items + (size_t)s * n;
         if (cudaMemcpyAsync(row, items.data(), sizeof(pfd::SweepItem) * items.size(), cudaMemcpyHostToDevice,
                             ctx->stream) != cudaSuccess) {
