@@ -15,24 +15,24 @@
 // whose source sample can lie in the neighbour window under the hypothesis; a
 // lane walks its own rectangle from its own origin, x offset outer, y offset
 // inner, so each NCC keeps the reference's accumulation order, and a tap whose
-// sample leaves the window adds exact zeros, which leaves the sums as the
-// reference's skipping does.
+// sample leaves the window adds nothing, as the reference skips it.
 //
 // Why: one pixel's NCCs fill 73% of the lanes of whole warps and the taps inside
 // both windows 41-57% of a warp's tap slots; pooled over the slots and sorted,
 // the lanes are full and 92% of the slots carry a tap of the lane's rectangle
 // (500 warp-taps per pixel instead of 860, 2048x1536, 12 neighbours, 15x15).  The
 // scalar code runs on half warps, the two halves of a warp on the same stage.
-// Bound by instruction issue: a warp-tap is about 40 instructions (3 loads, 18
-// FP32 operations, 6 integer products, 11 logical operations); packed pairs
-// (f32x2) halve the issue slots of the coordinates, measured 5% of the sweep.
+// Bound by instruction issue: a warp-tap is about 36 instructions (3 loads, 16
+// FP32 operations, 6 integer products, 8 logical operations); packed pairs
+// (f32x2) halve the issue slots of the coordinates, measured 3% of the sweep, and
+// predicated sums take the place of selected zeros, 12% (with a blur channel 15%).
 // The scalar code is bound by latency: what it took from a round was mostly chains of
 // shuffles and loops that every lane ran.  So a plane, view, draw or candidate is one
 // lane's wherever its order does not matter, the ordered sums read shared memory, the
 // weight tables are filled by all warps and the finished pixels written by one.  Every
 // lane on the loops -> one lane each: 28.7 -> 27.3 ms, 4.1 -> 3.6, 16.7 -> 10.6.
-// Half-sweep, warp per pixel -> slots: 41 -> 27.3 ms (2048x1536, 12 neighbours,
-// 15x15), 8.0 -> 3.6 ms (1024x768, 6, 11x11), 27 -> 10.6 ms (2048x1536, ACMM, 5x5).
+// Half-sweep, warp per pixel -> slots: 41 -> 23.7 ms (2048x1536, 12 neighbours,
+// 15x15), 8.0 -> 3.3 ms (1024x768, 6, 11x11), 27 -> 9.9 ms (2048x1536, ACMM, 5x5).
 #include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -216,39 +216,54 @@ struct Moments {
     float sr, srr, ss, sss, srs, sw, bsx, bsy;
 };
 
+// Whether a sample position lies in the neighbour window (its bits compare below the
+// window's), for the instructions that follow in the same statement.
+#define PFD_IN_WINDOW(sx, sy, w, h) ".reg .pred v;\n\tsetp.lt.u32 v, " sx ", " w ";\n\tsetp.lt.and.u32 v, " sy ", " h ", v;\n\t"
+
+// q = the word at q where the position is inside; otherwise q is unchanged.
+__device__ __forceinline__ uint32_t lds_if(uint32_t q, float sx, float sy, uint32_t wb, uint32_t hb)
+{
+    asm("{\n\t" PFD_IN_WINDOW("%1", "%2", "%3", "%4") "@v ld.shared.u32 %0, [%0];\n\t}"
+        : "+r"(q) : "r"(__float_as_uint(sx)), "r"(__float_as_uint(sy)), "r"(wb), "r"(hb));
+    return q;
+}
+
 // One tap: sample position (sx, sy) with its texture coordinates (tx, ty), the
 // tap's weight w and reference texel r.  A tap outside the neighbour window
-// (its bits compare above the window's) or with in false adds zeros.
+// (wb 0: always outside) adds nothing: its load and its sums are predicated, two
+// selects per tap less than adding zeros.
 template <bool BLUR, bool SHIFT>
 __device__ __forceinline__ void tap(Moments& M, float sx, float sy, float tx, float ty, float w, float r, float rb,
-                                    float sh, bool in, uint32_t wb, uint32_t hb, uint32_t base, uint32_t kq,
-                                    uint32_t qb_delta)
+                                    float sh, uint32_t wb, uint32_t hb, uint32_t base, uint32_t kq, uint32_t qb_delta)
 {
-    const bool v = in && (__float_as_uint(sx) < wb) && (__float_as_uint(sy) < hb);
     // (a, b, ix, iy) in the four bytes; the entry's address is base + 4 ix + row iy
     const uint32_t p = __byte_perm(__float_as_uint(tx), __float_as_uint(ty), 0x5140);
-    const uint32_t addr = v ? __dp4a(p, kq, base) : base;
+    const uint32_t addr = __dp4a(p, kq, base);
     const uint32_t a = __float_as_uint(tx) & 0xFFu, b = __float_as_uint(ty) & 0xFFu;
     const uint32_t w11 = (a * b + 128u) >> 8;
     const uint32_t hi = w11 * 65535u + b;
     const uint32_t lo = a * 65535u + 256u - hi;
-    const uint32_t q = lds_u32(addr);
+    const uint32_t q = lds_if(addr, sx, sy, wb, hb);
     float s = __fsub_rn(__uint_as_float(__dp2a_lo(lo, q, __dp2a_hi(hi, q, 0x47000000u))), 32768.0f);
     if (SHIFT) { s = __fsub_rn(s, sh); r = __fsub_rn(r, sh); }
-    const float wv = v ? w : 0.0f;
-    const float wr = __fmul_rn(wv, r), ws = __fmul_rn(wv, s);
-    M.sr = __fmaf_rn(wv, r, M.sr);
-    M.srr = __fmaf_rn(wr, r, M.srr);
-    M.ss = __fmaf_rn(wv, s, M.ss);
-    M.sss = __fmaf_rn(ws, s, M.sss);
-    M.srs = __fmaf_rn(wr, s, M.srs);
-    M.sw = __fadd_rn(M.sw, wv);
+    const float wr = __fmul_rn(w, r), ws = __fmul_rn(w, s);
+    asm("{\n\t" PFD_IN_WINDOW("%11", "%12", "%13", "%14")
+        "@v fma.rn.f32 %0, %6, %7, %0;\n\t"
+        "@v fma.rn.f32 %1, %9, %7, %1;\n\t"
+        "@v fma.rn.f32 %2, %6, %8, %2;\n\t"
+        "@v fma.rn.f32 %3, %10, %8, %3;\n\t"
+        "@v fma.rn.f32 %4, %9, %8, %4;\n\t"
+        "@v add.rn.f32 %5, %5, %6;\n\t}"
+        : "+f"(M.sr), "+f"(M.srr), "+f"(M.ss), "+f"(M.sss), "+f"(M.srs), "+f"(M.sw)
+        : "f"(w), "f"(r), "f"(s), "f"(wr), "f"(ws), "r"(__float_as_uint(sx)), "r"(__float_as_uint(sy)), "r"(wb), "r"(hb));
     if (BLUR) {
-        const uint32_t qb = lds_u32(addr + qb_delta);
+        const uint32_t qb = lds_if(addr + qb_delta, sx, sy, wb, hb);
         const float sb = __fsub_rn(__uint_as_float(__dp2a_lo(lo, qb, __dp2a_hi(hi, qb, 0x47000000u))), 32768.0f);
         const float db = div255(sb);
-        M.bsx = __fadd_rn(M.bsx, v ? rb : 0.0f);
-        M.bsy = __fadd_rn(M.bsy, v ? db : 0.0f);
+        asm("{\n\t" PFD_IN_WINDOW("%4", "%5", "%6", "%7")
+            "@v add.rn.f32 %0, %0, %2;\n\t@v add.rn.f32 %1, %1, %3;\n\t}"
+            : "+f"(M.bsx), "+f"(M.bsy)
+            : "f"(rb), "f"(db), "r"(__float_as_uint(sx)), "r"(__float_as_uint(sy)), "r"(wb), "r"(hb));
     }
 }
 
@@ -289,7 +304,7 @@ struct EvalEnv {
 // without an entry), the addresses of its first tap (weight wa, reference texel
 // ra), the weight table's column step wstep in bytes, its first tap position
 // (fx, fy) and the neighbour's quads (base).  All lanes walk the widest and
-// tallest rectangle of the warp; taps past a lane's own rectangle add zeros.
+// tallest rectangle of the warp; taps past a lane's own rectangle add nothing.
 // Two taps per iteration, their coordinates in packed pairs.
 template <bool BLUR, bool SHIFT>
 __device__ __forceinline__ void walk(Moments& M, const EvalEnv& E, float3 dp, float stx, float sty, int nx, int ny,
@@ -309,7 +324,7 @@ __device__ __forceinline__ void walk(Moments& M, const EvalEnv& E, float3 dp, fl
         uint64_t fy2 = fy_start;
         uint32_t wp = wa, rp = ra;
         int iy = 0;
-        for (; iy + 2 <= NYm; iy += 2) {
+        auto pair = [&](uint32_t wb0, uint32_t wb1) {
             const uint64_t d2 = add2_rn(fma2_rn(dpy2, fy2, axr2), dpz2);
             const uint64_t sx2 = fma2_rn(stx2, d2, fx2), sy2 = fma2_rn(sty2, d2, fy2);
             const uint64_t tx2 = fma2_rm(add2_rn(sx2, half2), scale2, magic2);
@@ -322,24 +337,36 @@ __device__ __forceinline__ void walk(Moments& M, const EvalEnv& E, float3 dp, fl
             const float w0 = lds_f32(wp), w1 = lds_f32(wp + 4u);
             const float r0 = lds_f32(rp), r1 = lds_f32(rp + rinc);
             const float b0 = BLUR ? lds_f32(rp + E.RB_delta) : 0.0f, b1 = BLUR ? lds_f32(rp + rinc + E.RB_delta) : 0.0f;
-            tap<BLUR, SHIFT>(M, sx0, sy0, tx0, ty0, w0, r0, b0, sh, true, E.wb, E.hb, base, E.kq, E.QB_delta);
-            tap<BLUR, SHIFT>(M, sx1, sy1, tx1, ty1, w1, r1, b1, sh, true, E.wb, E.hb, base, E.kq, E.QB_delta);
+            tap<BLUR, SHIFT>(M, sx0, sy0, tx0, ty0, w0, r0, b0, sh, wb0, E.hb, base, E.kq, E.QB_delta);
+            tap<BLUR, SHIFT>(M, sx1, sy1, tx1, ty1, w1, r1, b1, sh, wb1, E.hb, base, E.kq, E.QB_delta);
             fy2 = add2_rn(fy2, fy_step);
             wp += 8u;
             rp += 2u * rinc;
-        }
+        };
+        for (; iy + 2 <= NYm; iy += 2) pair(E.wb, E.wb);
+        // rows that some lanes keep: in pairs too (24.3 -> 23.9 ms, 2048x1536, 15x15), except
+        // with a blur channel, where the registers do not suffice (22.0 -> 23.7 ms)
+        if (!BLUR)
+            for (; iy + 2 <= NY; iy += 2) pair(iy < ny ? E.wb : 0u, iy + 1 < ny ? E.wb : 0u);
         float fyr, fyr1;
         unpack2(fy2, fyr, fyr1);
-        for (; iy < NY; ++iy) {
+        auto one = [&]() {
             const float d = __fadd_rn(__fmaf_rn(dp.y, fyr, axr), dp.z);
             const float sx = __fmaf_rn(stx, d, fx), sy = __fmaf_rn(sty, d, fyr);
             const float tx = __int_as_float(tex_coord_bits(sx)), ty = __int_as_float(tex_coord_bits(sy));
             const float b = BLUR ? lds_f32(rp + E.RB_delta) : 0.0f;
-            tap<BLUR, SHIFT>(M, sx, sy, tx, ty, lds_f32(wp), lds_f32(rp), b, sh, iy < ny, E.wb, E.hb, base, E.kq,
+            tap<BLUR, SHIFT>(M, sx, sy, tx, ty, lds_f32(wp), lds_f32(rp), b, sh, iy < ny ? E.wb : 0u, E.hb, base, E.kq,
                              E.QB_delta);
-            fyr = __fadd_rn(fyr, finc);
-            wp += 4u;
-            rp += rinc;
+        };
+        if (!BLUR) {
+            if (iy < NY) one();
+        } else {
+            for (; iy < NY; ++iy) {
+                one();
+                fyr = __fadd_rn(fyr, finc);
+                wp += 4u;
+                rp += rinc;
+            }
         }
         fx = __fadd_rn(fx, finc);
         wa += wstep;
@@ -376,8 +403,9 @@ __device__ __forceinline__ void cut_taps(float smin, float smax, float eps, floa
 
 // The rectangle of taps (first column and row, counts; 0 when empty) an NCC of
 // plane dp against a neighbour with steps (stx, sty) can keep.  The disparity is
-// affine over the window, so its range is at the corners; the second cut uses the
-// range over the first.
+// affine over the window, so its range is at the corners.  (A second cut with the
+// range over the first rectangle costs more than it saves: 24.4 against 24.1 ms,
+// 2048x1536, 15x15; 10.1 against 9.8, ACMM, 5x5.)
 __device__ __forceinline__ uint32_t tap_rect(const PixWin& pw, const PmParams& P, float3 dp, float stx, float sty,
                                              float inv_inc)
 {
@@ -387,14 +415,11 @@ __device__ __forceinline__ uint32_t tap_rect(const PixWin& pw, const PmParams& P
     if (mag * fmaxf(fabsf(stx), fabsf(sty)) < 1e6f) {    // false for NaN: the whole window
         const float ex = 0.01f + 4e-6f * mag * fabsf(stx), ey = 0.01f + 4e-6f * mag * fabsf(sty);
         const float dx = dp.x * finc, dy = dp.y * finc, d0 = dp.z + dp.x * X0 + dp.y * Y0;
-#pragma unroll
-        for (int rep = 0; rep < 2; ++rep) {
-            const float xa = dx * i0, xb = dx * i1, ya = dy * j0, yb = dy * j1;
-            const float dmin = d0 + fminf(xa, xb) + fminf(ya, yb), dmax = d0 + fmaxf(xa, xb) + fmaxf(ya, yb);
-            const float ax = stx * dmin, bx = stx * dmax, ay = sty * dmin, by = sty * dmax;
-            cut_taps(fminf(ax, bx), fmaxf(ax, bx), ex, (float)P.W, X0, inv_inc, i0, i1);
-            cut_taps(fminf(ay, by), fmaxf(ay, by), ey, (float)P.H, Y0, inv_inc, j0, j1);
-        }
+        const float xb = dx * i1, yb = dy * j1;
+        const float dmin = d0 + fminf(0.0f, xb) + fminf(0.0f, yb), dmax = d0 + fmaxf(0.0f, xb) + fmaxf(0.0f, yb);
+        const float ax = stx * dmin, bx = stx * dmax, ay = sty * dmin, by = sty * dmax;
+        cut_taps(fminf(ax, bx), fmaxf(ax, bx), ex, (float)P.W, X0, inv_inc, i0, i1);
+        cut_taps(fminf(ay, by), fmaxf(ay, by), ey, (float)P.H, Y0, inv_inc, j0, j1);
     }
     if (!(i0 <= i1 && j0 <= j1)) return 0u;
     const uint32_t a = (uint32_t)(int)i0, b = (uint32_t)(int)j0, c = (uint32_t)(int)i1, d = (uint32_t)(int)j1;
