@@ -31,8 +31,8 @@
 // lane's wherever its order does not matter, the ordered sums read shared memory, the
 // weight tables are filled by all warps and the finished pixels written by one.  Every
 // lane on the loops -> one lane each: 28.7 -> 27.3 ms, 4.1 -> 3.6, 16.7 -> 10.6.
-// Half-sweep, warp per pixel -> slots: 41 -> 23.7 ms (2048x1536, 12 neighbours,
-// 15x15), 8.0 -> 3.3 ms (1024x768, 6, 11x11), 27 -> 9.9 ms (2048x1536, ACMM, 5x5).
+// Half-sweep, warp per pixel -> slots: 41 -> 23.4 ms (2048x1536, 12 neighbours,
+// 15x15), 8.0 -> 3.2 ms (1024x768, 6, 11x11), 27 -> 9.6 ms (2048x1536, ACMM, 5x5).
 #include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
@@ -534,7 +534,7 @@ __device__ __forceinline__ float tap_weight(const float* R, int rs, const float*
 }
 
 // Bin counts to bin offsets (one warp).
-__device__ __forceinline__ void scan_bins(int* bins, int n, int lane)
+__device__ __forceinline__ int scan_bins(int* bins, int n, int lane)
 {
     const int per = (n + 31) / 32;
     int sum = 0;
@@ -547,11 +547,13 @@ __device__ __forceinline__ void scan_bins(int* bins, int n, int lane)
         const int t = __shfl_up_sync(kFullMask, off, o);
         if (lane >= o) off += t;
     }
+    const int total = __shfl_sync(kFullMask, off, 31);
     off -= sum;
     for (int i = 0; i < per; ++i) {
         const int b = lane * per + i;
         if (b < n) { const int c = bins[b]; bins[b] = off; off += c; }
     }
+    return total;
 }
 
 // ---- half-warp collectives -----------------------------------------------------
@@ -1385,6 +1387,9 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
             __syncthreads();
             // ---- the requests' NCCs into the list, 32 (row, view) pairs per warp at a time.
             // Slots whose pairs do not fit the list wait for the next round.
+            // A pair's place in the list is its index (0xFFFF: nothing to evaluate): no vote
+            // and no shared counter per 32 pairs (1% of a half-sweep).
+            int n_pairs;
             {
                 const int entered = next_stages[lane], stage = entered & ~kFresh;
                 int pairs = 0;
@@ -1422,6 +1427,8 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
                     if (lane >= o) upto += t;
                 }
                 const bool fits = upto <= cap;
+                const int start = upto - pairs;
+                n_pairs = __reduce_max_sync(kFullMask, fits ? upto : 0);
                 if (warp == 0) stages[lane] = fits ? stage : (stage | kWaits);
                 int units = fits ? (pairs + 31) >> 5 : 0, first = units;
                 for (int o = 1; o < 32; o <<= 1) {
@@ -1431,9 +1438,12 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
                 const int n_units = __shfl_sync(kFullMask, first, 31);
                 first -= units;
                 for (int u = warp; u < n_units; u += WARPS) {
+                    __syncwarp();
                     const uint32_t holds = __ballot_sync(kFullMask, units > 0 && first <= u);
                     const int slot = 31 - __clz(holds);
                     const int e = (u - __shfl_sync(kFullMask, first, slot)) * 32 + lane, total = __shfl_sync(kFullMask, pairs, slot);
+                    const int at = __shfl_sync(kFullMask, start, slot) + e;
+                    if (e >= total) continue;
                     const Slot S = slot_at(slot);
                     const SlotState& st = *S.st;
                     const int nv = st.n_views, x = st.xy & 0xFF, y = st.xy >> 8;
@@ -1445,7 +1455,7 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
                     const int h = st.row_lo + hr;
                     int k = e - hr * per;
                     uint32_t rect = 0u;
-                    if (e < total && !((skip >> h) & 1ull)) {
+                    if (!((skip >> h) & 1ull)) {
                         if (nv >= 0) k = S.sel[k];
                         if (okk[k]) {
                             const float4 d = S.dp[h];
@@ -1458,34 +1468,29 @@ __device__ __forceinline__ bool sweep_slots(unsigned char* smem, const FrameDev&
                         // NCC to be evaluated holds its rectangle until its cost is known.
                         S.cost[h * K + k] = rect ? __uint_as_float(rect) : kCostMax;
                     }
-                    const uint32_t m = __ballot_sync(kFullMask, rect != 0u);
-                    if (!m) continue;
-                    int at = 0;
-                    if (lane == 0) at = atomicAdd(&ctl[kCtlTasks], __popc(m));
-                    at = __shfl_sync(kFullMask, at, 0) + __popc(m & ((1u << lane) - 1u));
-                    if (rect) {
-                        t_id[at] = (uint16_t)((slot << 11) | (h << 5) | k);
-                        atomicAdd(&bins[rect_bin(rect, L.tx, L.ty)], 1);
-                    }
+                    t_id[at] = rect ? (uint16_t)((slot << 11) | (h << 5) | k) : (uint16_t)0xFFFFu;
+                    if (rect) atomicAdd(&bins[rect_bin(rect, L.tx, L.ty)], 1);
                 }
             }
             __syncthreads();
             // ---- sort by rectangle: bin offsets, then the order
-            const int n_tasks = ctl[kCtlTasks];
             if (warp == 0) {
-                scan_bins(bins, L.nbins, lane);
-                if (lane == 0) ctl[kCtlPass] = 0;
+                const int n = scan_bins(bins, L.nbins, lane);
+                if (lane == 0) {
+                    ctl[kCtlTasks] = n;
+                    ctl[kCtlPass] = 0;
+                }
             }
             __syncthreads();
-            for (int i = tid; i < n_tasks; i += blockDim.x)
-            {
+            const int n_tasks = ctl[kCtlTasks];
+            for (int i = tid; i < n_pairs; i += blockDim.x) {
                 const int id = t_id[i];
+                if (id == 0xFFFF) continue;
                 const uint32_t rect = ((const uint32_t*)(smem + L.off_cost))[((id >> 11) * L.rows + ((id >> 5) & 63)) * K + (id & 31)];
                 t_order[atomicAdd(&bins[rect_bin(rect, L.tx, L.ty)], 1)] = (uint16_t)id;
             }
             __syncthreads();
             for (int e = tid; e < L.nbins; e += blockDim.x) bins[e] = 0;
-            if (tid == 0) ctl[kCtlTasks] = 0;
             // ---- evaluate, 32 NCCs per warp at a time
             for (;;) {
                 int p = 0;
