@@ -214,14 +214,17 @@ __global__ void __launch_bounds__(kThreads) pm_refocus_kernel(RefocusFrame F, co
 
 size_t refocus_quads_bytes(const RefocusFrame& F) { return sizeof(uint32_t) * (size_t)F.V * F.m * F.mh; }
 
-cudaError_t launch_refocus(const RefocusFrame& F, uint32_t* quads, const float* slice_vd, int n_slices, int raw_w,
+cudaError_t launch_refocus_quads(const RefocusFrame& F, uint32_t* quads, cudaStream_t st)
+{
+    const size_t px = (size_t)F.V * F.m * F.mh;
+    pm_refocus_quads_kernel<<<(unsigned)((px + 1023) / 1024), 256, 0, st>>>(F.gray, F.tile_stride, F.m, F.mh, F.V, quads);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_refocus(const RefocusFrame& F, const uint32_t* quads, const float* slice_vd, int n_slices, int raw_w,
                            int raw_h, int out_w, int out_h, float* out, int* err, cudaStream_t st)
 {
     if (n_slices <= 0) return cudaSuccess;
-    const size_t px = (size_t)F.V * F.m * F.mh;
-    pm_refocus_quads_kernel<<<(unsigned)((px + 1023) / 1024), 256, 0, st>>>(F.gray, F.tile_stride, F.m, F.mh, F.V, quads);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
     const int smem = kMaxRefocusCand * 16;
     const float sx = (float)raw_w / (float)out_w, sy = (float)raw_h / (float)out_h;
     const dim3 grid((out_w + kTileW - 1) / kTileW, (out_h + kTileH - 1) / kTileH, n_slices);

@@ -23,7 +23,9 @@ constexpr int kMaxRefocusCand = 2048;             // lenses that may reach one 6
 
 // Bytes of the packed micro-images a render lays out for itself.
 size_t refocus_quads_bytes(const RefocusFrame& F);
-cudaError_t launch_refocus(const RefocusFrame& F, uint32_t* quads, const float* slice_vd, int n_slices, int raw_w,
+cudaError_t launch_refocus_quads(const RefocusFrame& F, uint32_t* quads, cudaStream_t st);
+// Renders n_slices slices into out from the packed micro-images.
+cudaError_t launch_refocus(const RefocusFrame& F, const uint32_t* quads, const float* slice_vd, int n_slices, int raw_w,
                            int raw_h, int out_w, int out_h, float* out, int* err, cudaStream_t st);
 
 }  // namespace pfd
