@@ -45,9 +45,9 @@ namespace pfd {
 namespace {
 
 // Launch shapes: warps per CTA and CTAs per SM.  Shape 0, the default, is the
-// fastest on the frames without a blur channel (2048x1536, 12 neighbours, 15x15:
-// 28.1 ms, 12x2 30.0, 8x3 33.4, 16x1 34.6); one CTA with all the shared memory
-// (shape 3) where the quads of a blur channel leave two CTAs few slots.
+// fastest where two CTAs fit (2048x1536, 12 neighbours, 15x15: 23.5 ms, 12x2 24.4, 8x3
+// 24.7, 16x1 27.5); one CTA with all the shared memory and registers (shape 3) where
+// the quads of a blur channel leave two CTAs few slots (one_cta_shape).
 template <int S> struct ShapeOf;
 template <> struct ShapeOf<0> { static constexpr int warps = 16, min_ctas = 2; };
 template <> struct ShapeOf<1> { static constexpr int warps = 12, min_ctas = 2; };
@@ -1944,6 +1944,14 @@ static const void* slots_batch_kernel(int shape, bool blur, bool shift)
     }
 }
 
+// A plan of more than half of an SM's shared memory runs one CTA per SM whatever the
+// kernel's registers are bounded for: the default shape then runs the kernel of as many
+// warps with the registers of one CTA (a half-sweep at 1531x1147, 17
+// neighbours, 13x13, blur: 21.7 -> 20.3 ms).  Where two CTAs fit, the default's kernel:
+// 23.5 against 27.5 ms (2048x1536, 12, 15x15).
+static_assert(ShapeOf<0>::warps == ShapeOf<3>::warps && ShapeOf<3>::min_ctas == 1, "shapes of one_cta_shape");
+static int one_cta_shape(int shape, int smem) { return shape == 0 && smem > (228 * 1024) / 2 - 1024 ? 3 : shape; }
+
 static cudaError_t slots_grid(const void* k, int threads, int smem, int* n_ctas)
 {
     int dev = 0, sms = 0, per_sm = 0;
@@ -1960,6 +1968,7 @@ static cudaError_t slots_grid(const void* k, int threads, int smem, int* n_ctas)
 
 cudaError_t slots_sweep_grid(const FrameDev& F, const PmParams& P, int smem, int* n_ctas, int shape)
 {
+    shape = one_cta_shape(shape, smem);
     return slots_grid(slots_kernel(shape, F.blur != nullptr, P.shifted != 0), 32 * slots_shape_warps(shape), smem, n_ctas);
 }
 
@@ -1967,6 +1976,7 @@ cudaError_t launch_slots_sweep(const FrameDev& F, const PmParams& P, const State
                                int phase, int smem, int n_ctas, int* err, cudaStream_t st, int shape)
 {
     if (smem <= 0 || smem > 227 * 1024) return cudaErrorInvalidConfiguration;
+    shape = one_cta_shape(shape, smem);
     const void* k = slots_kernel(shape, F.blur != nullptr, P.shifted != 0);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e == cudaSuccess) e = cudaMemsetAsync(P.view_queue, 0, sizeof(int), st);
@@ -1979,6 +1989,7 @@ cudaError_t launch_slots_sweep(const FrameDev& F, const PmParams& P, const State
 
 cudaError_t slots_batch_grid(int smem, bool blur, bool shift, int* n_ctas, int shape)
 {
+    shape = one_cta_shape(shape, smem);
     return slots_grid(slots_batch_kernel(shape, blur, shift), 32 * slots_shape_warps(shape), smem, n_ctas);
 }
 
@@ -1987,6 +1998,7 @@ cudaError_t launch_slots_batch(const SweepItem* items, int n, bool blur, bool sh
 {
     if (n <= 0) return cudaSuccess;
     if (smem <= 0 || smem > 227 * 1024) return cudaErrorInvalidConfiguration;
+    shape = one_cta_shape(shape, smem);
     const void* k = slots_batch_kernel(shape, blur, shift);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
