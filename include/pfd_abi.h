@@ -256,7 +256,8 @@ pfd_status pfd_set_matcher(pfd_ctx* ctx, int matcher);
  * pfd_patchmatch_batch; no counterpart in the reference, whose sweep is one
  * thread per pixel in 16x16 blocks).  A shape is a number of warps per CTA and
  * the CTAs per SM its registers are sized for; every shape computes the same
- * state bit for bit.  Shape 0 (16 warps, 2 CTAs) is the default.  Texture fetches
+ * state bit for bit.  Shape 0 (16 warps, 2 CTAs; 1 CTA with its registers where a plan
+ * takes more than half of the shared memory) is the default.  Texture fetches
  * and tap counting have one shape of their own.
  * PFD_SHAPE_AUTOTUNE: the engine's autotuner picks the shape per key (window,
  * neighbour count, patch size and tap stride, blur channel, moment mode,
