@@ -1878,12 +1878,12 @@ int slots_shape_warps(int shape) { return kShapeWarps[(shape >= 0 && shape < kSw
 int slots_shape_ctas(int shape) { return kShapeCtas[(shape >= 0 && shape < kSweepShapes) ? shape : 0]; }
 
 // Slots, list capacity and parts of a half-sweep; returns the dynamic shared
-// memory of its plan, or 0 when none fits.  A launch of fewer than two items per
+// memory of its plan, or 0 when none fits.  A launch of fewer than six items per
 // CTA splits its micro-images, so that no CTA is without work and the last ones end
 // together; a part stages the micro-image anew and drains its slots, so larger frames
 // and parts of fewer pixels than slots lose.  Half-sweep at 1, 2, 4 and 8 parts: 182
-// micro-images of 21x21 on 296 CTAs .42, .36, .35, .43 ms; 1672 of 23x23 3.56, 3.56,
-// 3.69, 4.55 ms; 6612 of 23x23 27.4, 28.3, 30.3, 33.7 ms.
+// micro-images of 21x21 on 296 CTAs .38, .31, .30, .37 ms; 1672 of 23x23 (5.6 items per
+// CTA) 3.20, 3.08, 3.14, 3.88 ms; 6612 of 16x16 (22 items) 23.0, 23.7, 25.2, 28.1 ms.
 int slots_plan(PmParams& P, bool blur, int shape, int n_views)
 {
     const int warps = slots_shape_warps(shape);
@@ -1901,7 +1901,7 @@ int slots_plan(PmParams& P, bool blur, int shape, int n_views)
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
             const int n_upd = (P.ppv + 1) / 2;
             P.parts = 1;
-            while ((long long)n_views * P.parts < 2LL * sms * ctas && n_upd / (2 * P.parts) >= s) P.parts *= 2;
+            while ((long long)n_views * P.parts < 6LL * sms * ctas && n_upd / (2 * P.parts) >= s) P.parts *= 2;
             return L.total;
         }
     }

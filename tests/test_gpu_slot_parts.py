@@ -1,5 +1,5 @@
 """Half-sweeps whose micro-images are split between CTAs (pm_slots.cu): view
-counts on both sides of two items per CTA, the smallest frame, an odd number of
+counts around one and two items per CTA, the smallest frame, an odd number of
 pixels, parts near the number of slots, and frames that share a launch.  Every
 state field equals the CPU oracle's bit for bit."""
 import numpy as np
