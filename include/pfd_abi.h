@@ -200,14 +200,16 @@ pfd_status pfd_pm_sweep(pfd_ctx* ctx, int frame_id, const pfd_pm_params* params,
  * For callers that cannot allocate device memory once frames are streaming: an
  * application whose memory pool claimed all free HBM at start-up, or a
  * real-time loop that forbids cudaMalloc/cudaFree because they can synchronise
- * the whole device.  The sweep itself needs no scratch; under tap counting or
- * texture fetches its cost-vector scratch is a fixed 8 MiB array in the
- * library's device image (held by every GPU that loads the library, until
- * exit) instead of a cudaMalloc'd buffer.  Inputs and outputs are the frame's
- * state exactly as for pfd_pm_sweep, and the results are the same bit for bit.
- * Limit (tap counting, texture fetches): the array must hold one CTA's scratch (seven warps, each the cost
- * vectors of one pixel) for every SM: every max_nb up to 32 fits on a 148-SM
- * B200; a device with more SMs than the array holds CTAs gets PFD_EINVAL.
+ * the whole device.  The sweep itself needs no scratch; under tap counting, under
+ * texture fetches, and for a window with a blur channel whose quads fill the shared
+ * memory (25x25 with 32 neighbours, 32x32 from 19), its cost-vector scratch is a
+ * fixed 8 MiB array in the library's device image (held by every GPU that loads
+ * the library, until exit) instead of a buffer allocated on the stream.  Inputs
+ * and outputs are the frame's state exactly as for pfd_pm_sweep, and the results
+ * are the same bit for bit.
+ * Limit (where the array is used): it must hold one CTA's scratch (seven warps,
+ * each the cost vectors of one pixel) for every SM: every max_nb up to 32 fits on
+ * a 148-SM B200; a device with more SMs than the array holds CTAs gets PFD_EINVAL.
  * Every call looks up the array's device address (cudaGetSymbolAddress, a
  * host-side lookup), so the address stays right after a cudaDeviceReset; the
  * first call on a device may also load the library's device code there, so
@@ -257,8 +259,9 @@ pfd_status pfd_set_matcher(pfd_ctx* ctx, int matcher);
  * thread per pixel in 16x16 blocks).  A shape is a number of warps per CTA and
  * the CTAs per SM its registers are sized for; every shape computes the same
  * state bit for bit.  Shape 0 (16 warps, 2 CTAs; 1 CTA with its registers where a plan
- * takes more than half of the shared memory) is the default.  Texture fetches
- * and tap counting have one shape of their own.
+ * takes more than half of the shared memory) is the default.  Texture fetches,
+ * tap counting and blurred windows whose quads fill the shared memory have one
+ * shape of their own.
  * PFD_SHAPE_AUTOTUNE: the engine's autotuner picks the shape per key (window,
  * neighbour count, patch size and tap stride, blur channel, moment mode,
  * matcher) and device: the first half-sweep of a new key runs once in every

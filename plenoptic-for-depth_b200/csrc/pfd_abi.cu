@@ -1044,7 +1044,8 @@ static pfd_status tune_shape(pfd_ctx* ctx, Frame& f, pfd::PmParams P, int iter, 
 
 // The shape the context's next half-sweep of frame f runs: the fixed one, or
 // under PFD_SHAPE_AUTOTUNE the tuned one (tuning on this half-sweep when the
-// key is new).  Tap counting and texture fetches have one shape.
+// key is new).  Tap counting, texture fetches and windows without a slot plan have
+// one shape.
 static pfd_status sweep_shape_for(pfd_ctx* ctx, Frame& f, const pfd::PmParams& P, int iter, int phase, int* shape)
 {
     *shape = 0;
@@ -1059,7 +1060,8 @@ static pfd_status sweep_shape_for(pfd_ctx* ctx, Frame& f, const pfd::PmParams& P
         *shape = c;
         return PFD_OK;
     }
-    if (key.tex) {
+    pfd::PmParams Q = P;
+    if (key.tex || !pfd::slots_plan(Q, f.has_blur, 0, f.V)) {       // the warp-per-pixel kernel: one shape
         std::lock_guard<std::mutex> lock(g_shape_mu);
         g_shape_cache[key] = 0;
         return PFD_OK;
@@ -1096,8 +1098,13 @@ pfd_status pfd_tuned_sweep_shape(pfd_ctx* ctx, int frame_id, const pfd_pm_params
     return PFD_OK;
 }
 
-// Tap counting and texture fetches run the warp-per-pixel kernel.
-static bool uses_warp_sweep(const pfd::FrameDev& F, const pfd::PmParams& P) { return F.tex != nullptr || P.tap_counter; }
+// Tap counting, texture fetches and windows whose slot plan does not fit shared memory
+// run the warp-per-pixel kernel, whose plan is the smaller one (no padding behind the
+// reference texels, no lists); check_sweep_fits refuses what that one cannot hold.
+static bool uses_warp_sweep(const Frame& f, const pfd::FrameDev& F, pfd::PmParams P)
+{
+    return F.tex != nullptr || P.tap_counter || !pfd::slots_plan(P, f.has_blur, 0, f.V);
+}
 
 static pfd_status check_sweep_fits(pfd_ctx* ctx, const Frame& f, const pfd::PmParams& P, const pfd::FrameDev& F)
 {
@@ -1139,8 +1146,9 @@ pfd_status pfd_pm_sweep(pfd_ctx* ctx, int frame_id, const pfd_pm_params* params,
     const pfd::FrameDev F = sweep_dev(ctx, *f);
     if ((st = check_sweep_fits(ctx, *f, P, F)) != PFD_OK) return st;
     P.cvec_ok = !ctx->counting && cvec_usable(*f, *params, phase, cost_mode(ctx));
-    int n_ctas = 0;
-    if (uses_warp_sweep(F, P)) {
+    int n_ctas = 0, shape = 0;
+    if ((st = sweep_shape_for(ctx, *f, P, iter, phase, &shape)) != PFD_OK) return st;
+    if (uses_warp_sweep(*f, F, P)) {
         CU(pfd::sweep_warp_grid(F, P, &n_ctas));
         st = ensure_scratch(ctx, pfd::sweep_warp_scratch_bytes(P, n_ctas));
         if (st != PFD_OK) return st;
@@ -1148,9 +1156,6 @@ pfd_status pfd_pm_sweep(pfd_ctx* ctx, int frame_id, const pfd_pm_params* params,
         P.scratch_floats = ctx->scratch_bytes / sizeof(float);
         CU(pfd::launch_sweep_warp(F, P, f->s[f->cur], f->s[f->cur ^ 1], iter, phase, n_ctas, ctx->d_err, ctx->stream));
     } else {
-        int shape = 0;
-        st = sweep_shape_for(ctx, *f, P, iter, phase, &shape);
-        if (st != PFD_OK) return st;
         st = slots_sweep(ctx, *f, P, F, iter, phase, shape);
         if (st != PFD_OK) return st;
     }
@@ -2736,7 +2741,7 @@ extern "C" pfd_status pfd_pm_sweep_noalloc(pfd_ctx* ctx, int frame_id, const pfd
     const pfd::FrameDev F = sweep_dev(ctx, *f);
     if ((st = check_sweep_fits(ctx, *f, P, F)) != PFD_OK) return st;
     P.cvec_ok = !ctx->counting && cvec_usable(*f, *params, phase, cost_mode(ctx));
-    if (!uses_warp_sweep(F, P)) {                // the slot kernel needs no scratch
+    if (!uses_warp_sweep(*f, F, P)) {                // the slot kernel needs no scratch
         st = slots_sweep(ctx, *f, P, F, iter, phase, 0);
         if (st != PFD_OK) return st;
         ctx->launches += 1;

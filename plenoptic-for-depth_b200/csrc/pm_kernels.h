@@ -49,8 +49,8 @@ cudaError_t slots_batch_grid(int smem, bool blur, bool shift, int* n_ctas, int s
 cudaError_t launch_slots_batch(const SweepItem* items, int n, bool blur, bool shift, int smem, int n_ctas, int* err,
                                cudaStream_t st, int shape);
 
-// The warp-per-pixel half-sweep (pm_sweep.cu) of tap counting (P.tap_counter) and
-// of texture fetches (F.tex): grid, shared memory, and the global scratch it
+// The warp-per-pixel half-sweep (pm_sweep.cu) of tap counting (P.tap_counter), of
+// texture fetches (F.tex), and of blurred windows without a slot plan: grid, shared memory, and the global scratch it
 // needs (P.cost_scratch: per warp, the cost vectors of one pixel).
 cudaError_t sweep_warp_grid(const FrameDev& F, const PmParams& P, int* n_ctas);
 int sweep_warp_smem_bytes(const PmParams& P, bool blur, bool tex);

@@ -1,7 +1,7 @@
 // pm_sweep.cu -- CheckerboardUpdateFrame (MIStereo/AdaptMIPMFrame.cu:520-947)
 // with one warp per updated pixel: the half-sweep of tap-counting calibration
-// runs and of texture fetches (PFD_FETCH_TEXTURE).  The other half-sweeps run in
-// pm_slots.cu.
+// runs, of texture fetches (PFD_FETCH_TEXTURE), and of windows with a blur channel
+// whose quads leave no room for a slot.  The other half-sweeps run in pm_slots.cu.
 //
 // A CTA stages one micro-image and its neighbours at a time; its warps take the
 // updated pixels of that micro-image one by one.  For a pixel, every cost
@@ -18,8 +18,8 @@
 //
 // Cross-view proposals depend on the best plane so far (AdaptMIPMFrame.cu:
 // 907-936), and the refinement candidates on the best plane after them
-// (:400-471).  Texture fetches build both speculatively from the best plane
-// after propagation, evaluate them together and walk them in order; a proposal
+// (:400-471).  Without tap counting both are built speculatively from the best plane
+// after propagation, evaluated together and walked in order; a proposal
 // whose sample position changed because an earlier one won is rebuilt and
 // evaluated again, and so are the refinement candidates that follow the best
 // plane, so the result is the sequential one.  Tap counting evaluates exactly
@@ -27,7 +27,7 @@
 //
 // Texture fetches: the frame's micro-images are layered float textures with the
 // reference's filter settings, and a tap is one tex2DLayered fetch, the
-// reference's own tex2D.  Tap counting stages the neighbours in shared memory
+// reference's own tex2D.  The other forms stage the neighbours in shared memory
 // as 32-bit quads, entry (iy, ix) packing the four texels of a bilinear
 // footprint, T(iy,ix), T(iy,ix+1), T(iy+1,ix), T(iy+1,ix+1), indices clamped to
 // the window, and blends them as the texture unit does (measured, and equal to
@@ -1022,10 +1022,15 @@ static cudaError_t set_smem(const void* k, int smem, bool tex)
     return cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
 }
 
-// The half-sweep kernel of one variant: tap counting (shared-memory fetches) or
-// texture fetches.
-static const void* warp_kernel(bool blur, bool count, bool shift)
+// The half-sweep kernel of one variant: tap counting (shared-memory fetches), texture
+// fetches, or plain shared-memory fetches.  The last only with a blur channel: over all
+// windows, neighbour counts and patches, every plan of this kernel that the slot kernel
+// cannot hold has one (32x32 from 19 neighbours, 25x25 with 32).
+static const void* warp_kernel(bool blur, bool count, bool shift, bool tex)
 {
+    if (!count && !tex)
+        return !blur ? nullptr : (shift ? (const void*)pm_sweep_warp_kernel<true, false, true, false>
+                                        : (const void*)pm_sweep_warp_kernel<true, false, false, false>);
     if (count) {
         if (shift) return blur ? (const void*)pm_sweep_warp_kernel<true, true, true, false>
                                : (const void*)pm_sweep_warp_kernel<false, true, true, false>;
@@ -1060,20 +1065,22 @@ static cudaError_t grid_for(const void* k, int smem, bool tex, int* n_ctas)
 
 cudaError_t sweep_warp_grid(const FrameDev& F, const PmParams& P, int* n_ctas)
 {
-    const bool blur = F.blur != nullptr, count = P.tap_counter != nullptr;
-    return grid_for(warp_kernel(blur, count, P.shifted != 0), sweep_warp_smem_bytes(P, blur, !count), !count, n_ctas);
+    const bool blur = F.blur != nullptr, count = P.tap_counter != nullptr, tex = !count && F.tex != nullptr;
+    const void* k = warp_kernel(blur, count, P.shifted != 0, tex);
+    if (!k) return cudaErrorInvalidConfiguration;
+    return grid_for(k, sweep_warp_smem_bytes(P, blur, tex), tex, n_ctas);
 }
 
 cudaError_t launch_sweep_warp(const FrameDev& F, const PmParams& P, const StateDev& prev, const StateDev& next,
                               int iter, int phase, int n_ctas, int* err, cudaStream_t st)
 {
-    const bool blur = F.blur != nullptr, count = P.tap_counter != nullptr;
-    const int smem = sweep_warp_smem_bytes(P, blur, !count);
-    if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
+    const bool blur = F.blur != nullptr, count = P.tap_counter != nullptr, tex = !count && F.tex != nullptr;
+    const int smem = sweep_warp_smem_bytes(P, blur, tex);
+    const void* k = warp_kernel(blur, count, P.shifted != 0, tex);
+    if (!k || smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     const int grid = std::max(1, std::min(n_ctas, F.V));
-    const void* k = warp_kernel(blur, count, P.shifted != 0);
     cudaError_t e = cudaMemsetAsync(P.view_queue, 0, sizeof(int), st);
-    if (e == cudaSuccess) e = set_smem(k, smem, !count);
+    if (e == cudaSuccess) e = set_smem(k, smem, tex);
     if (e != cudaSuccess) return e;
     FrameDev f = F; PmParams p = P; StateDev a = prev, b = next; int it = iter, ph = phase; int* er = err;
     void* args[] = { &f, &p, &a, &b, &it, &ph, &er };
