@@ -984,30 +984,25 @@ cudaError_t launch_cycle(const CheckFrame& F, const CycleCfg& cfg, const StateDe
     return cudaGetLastError();
 }
 
-// The filter's work area: what filter_work() lays out in a scratch buffer.
-size_t filter_work_bytes(const CheckFrame& F, const FilterCfg& cfg)
+// Room per micro-image of P >= 4 pixels: the idle state holds 16 P bytes in plane (8 P
+// needed), 16 P in disp (4 + 4 ceil(P / 32), and 16 for ctl once: 28 <= 64 at P = 4), 4 P
+// in sel (4); the cost vectors hold 4 K P (2 K P: a pixel has at most one test per
+// neighbour, whatever max_triplet).
+FilterWork filter_work(const CheckFrame& F, const StateDev& idle, float* cvec)
 {
     FilterWork X;
-    return filter_work(F, cfg, nullptr, X);
-}
-
-size_t filter_work(const CheckFrame& F, const FilterCfg& cfg, unsigned char* buf, FilterWork& X)
-{
-    const size_t px = (size_t)F.V * F.W * F.H;
-    size_t o = 0;
-    auto take = [&](size_t bytes) { const size_t at = o; o += (bytes + 255) & ~(size_t)255; return buf + at; };
-    X.total = px;
+    X.total = (size_t)F.V * F.W * F.H;
     X.mask_words = (F.W * F.H + 31) / 32;
-    X.zeroed = buf;
-    X.ctl = (unsigned int*)take(16);
-    X.changed = (int*)take(sizeof(int) * (size_t)F.V);
-    X.mask = (uint32_t*)take(sizeof(uint32_t) * (size_t)F.V * X.mask_words);
-    X.zeroed_bytes = o;
-    X.list = (int*)take(sizeof(int) * (size_t)F.V);
-    X.head = (uint32_t*)take(sizeof(uint32_t) * px);
-    X.disp = (float*)take(sizeof(float) * px);
-    X.ent = (uint16_t*)take(sizeof(uint16_t) * px * (size_t)(cfg.max_triplet > 0 ? cfg.max_triplet : 1));
-    return o;
+    X.head = (uint32_t*)idle.plane;
+    X.disp = (float*)(X.head + X.total);
+    X.ctl = (unsigned int*)idle.disp;
+    X.changed = (int*)(X.ctl + 4);
+    X.mask = (uint32_t*)(X.changed + F.V);
+    X.zeroed = (unsigned char*)X.ctl;
+    X.zeroed_bytes = 16 + 4 * (size_t)F.V * (1 + X.mask_words);
+    X.list = (int*)idle.sel;
+    X.ent = (uint16_t*)cvec;
+    return X;
 }
 
 cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,

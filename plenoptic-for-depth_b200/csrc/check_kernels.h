@@ -72,8 +72,10 @@ int cycle_smem_bytes(const CheckFrame& F);
 cudaError_t launch_cycle(const CheckFrame& F, const CycleCfg& cfg, const StateDev& st, float* geo_err, float* pho_err,
                          uint8_t* texmask, CycleTileRec* recs, unsigned int* hist, cudaStream_t s);
 
-// The filter's work area (see check_kernels.cu): 8 + 2 max_triplet bytes per pixel,
-// and a mask, a stamp and a list entry per micro-image.
+// The filter's work area (see check_kernels.cu), laid into device memory that the frame
+// holds anyway and that nobody reads then: the state buffer that is not the current one
+// (the next half-sweep writes all of it) and the stored cost vectors (a filtered state
+// has none that are valid).
 struct FilterWork {
     size_t total;              // pixels of the frame
     int mask_words;            // 32-bit words of a micro-image's mask
@@ -85,10 +87,9 @@ struct FilterWork {
     int* list;                 // [V] micro-images of the round
     uint32_t* head;            // [total] class and final counts
     float* disp;               // [total] disparity
-    uint16_t* ent;             // [max_triplet][total] tests against earlier neighbours
+    uint16_t* ent;             // [K][total] tests against earlier neighbours
 };
-size_t filter_work_bytes(const CheckFrame& F, const FilterCfg& cfg);
-size_t filter_work(const CheckFrame& F, const FilterCfg& cfg, unsigned char* buf, FilterWork& X);
+FilterWork filter_work(const CheckFrame& F, const StateDev& idle, float* cvec);
 // The whole filter, three launches; err gets flag 1 when a device wait gave up.
 cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,
                           uint8_t* reason, unsigned long long* stats, int* err, cudaStream_t s);

@@ -1646,17 +1646,11 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
         f->d_fstats = (unsigned long long*)p;
     }
     unsigned long long* d_stats = f->d_fstats;
-    // three launches over a work area in the context's scratch; as a wavefront where
-    // a rejected pixel's disparity (-1) counts as usable, or where the budget does not
-    // hold the work area (the same result, 10x slower)
-    pfd::FilterWork X;
-    bool wavefront = !(fc.min_valid_disp >= -1.0f);
-    if (!wavefront && ensure_scratch(ctx, pfd::filter_work_bytes(F, fc)) != PFD_OK) wavefront = true;
-    if (wavefront) {
-        if ((st = build_steps(ctx, *f)) != PFD_OK) return st;
-    } else {
-        pfd::filter_work(F, fc, (unsigned char*)ctx->d_scratch, X);
-    }
+    // three launches; as a wavefront where a rejected pixel's disparity (-1) counts as
+    // usable (the same result, 10x slower)
+    const bool wavefront = !(fc.min_valid_disp >= -1.0f);
+    if (wavefront && (st = build_steps(ctx, *f)) != PFD_OK) return st;
+    const pfd::FilterWork X = pfd::filter_work(F, f->s[f->cur ^ 1], f->d_cvec);
     // enqueue-only calls under pfd_set_graphs: the first call with a key runs as
     // usual, the second is captured, later ones replay the graph (it reads the
     // state buffer the frame's current state was in at capture)
@@ -1667,7 +1661,6 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
         std::vector<unsigned char> key(sizeof(pfd_filter_cfg) + sizeof(float));
         std::memcpy(key.data(), cfg, sizeof(pfd_filter_cfg));
         std::memcpy(key.data() + sizeof(pfd_filter_cfg), &baseline_unit, sizeof(float));
-        if (G.exec && G.scratch_gen != ctx->scratch_gen) G.reset();   // the scratch moved since the capture
         if (G.exec && G.key == key && G.cur == f->cur) {
             CU(cudaGraphLaunch(G.exec, ctx->stream));
             ctx->launches += G.launches;
@@ -1710,7 +1703,6 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
         if (graph) cudaGraphDestroy(graph);
         if (fst != PFD_OK) { G.reset(); return fst; }
         G.launches = ctx->launches - launches0;
-        G.scratch_gen = ctx->scratch_gen;
         CU(cudaGraphLaunch(G.exec, ctx->stream));
         return PFD_OK;
     }
