@@ -16,8 +16,12 @@
 //                           micro-image depends on earlier ones only, so this ends at
 //                           the one solution, the sequential walk's.  A cooperative
 //                           launch; the grid barrier's waits are bounded.
+//   pm_fuse_fold_kernel     between bands (below), what a band masks for the next ones.
 //   pm_fuse_points_kernel   the fused points, one thread per pixel, their neighbours
 //                           summed in list order, so every float is the reference's.
+// The tests take two bytes per pixel and list entry, so a frame with long lists is walked
+// in bands of micro-images, one after the other in map order: a band's walk starts from
+// the masks of the bands before it, which are final.
 // Points that land on the same raw pixel overwrite each other in map order in
 // the reference; here each records its sequence number (micro-image, pixel)
 // with atomicMax and the maps are written from the last one afterwards.
@@ -115,7 +119,7 @@ __device__ __forceinline__ int consistent_pixel(const FuseFrame& F, float3 P, fl
 __global__ void __launch_bounds__(256) pm_fuse_pairs_kernel(FuseFrame F, FuseWork X)
 {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int v = blockIdx.x;
+    const int b = blockIdx.x, v = X.v0 + b;
     if (!X.is_ref[v]) return;
     const int m = F.m, N = F.ppv;
     const int nl = min(F.list_counts[v], F.max_list);
@@ -138,7 +142,7 @@ __global__ void __launch_bounds__(256) pm_fuse_pairs_kernel(FuseFrame F, FuseWor
             const bool own = !(w < F.min_ref_disp) && valid_vd(vdr);
             const int r = idx / m, c = idx - r * m;
             const float3 P = virtual_3d(vdr, c, r, cm, cr);
-            uint16_t* row = X.pair_si + ((size_t)v * N + idx) * F.max_list;
+            uint16_t* row = X.pair_si + ((size_t)b * N + idx) * F.max_list;
             if (own) num = 0;
             for (int j = 0; j < nl; ++j) {
                 int si = -1;
@@ -148,19 +152,19 @@ __global__ void __launch_bounds__(256) pm_fuse_pairs_kernel(FuseFrame F, FuseWor
             }
         }
         const unsigned bits = __ballot_sync(kFull, num >= 0 && num >= F.min_consistent);
-        if ((threadIdx.x & 31) == 0) X.maybe[(size_t)v * X.mask_words + (idx >> 5)] = bits;
+        if ((threadIdx.x & 31) == 0) X.maybe[(size_t)b * X.mask_words + (idx >> 5)] = bits;
     }
 }
 
-// Who masks pixels of a micro-image: the (reference micro-image, list entry) pairs
-// that name it, as lists in X.rev.
+// Who masks pixels of a micro-image: the band's (reference micro-image, list entry)
+// pairs that name it, as lists in X.rev.
 __global__ void pm_fuse_rev_count_kernel(FuseFrame F, FuseWork X)
 {
-    const size_t n = (size_t)F.V * F.max_list;
+    const size_t n = (size_t)(X.v1 - X.v0) * F.max_list, e0 = (size_t)X.v0 * F.max_list;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int w = (int)(e / F.max_list), j = (int)(e - (size_t)w * F.max_list);
+        const int b = (int)(e / F.max_list), w = X.v0 + b, j = (int)(e - (size_t)b * F.max_list);
         if (!X.is_ref[w] || j >= F.list_counts[w]) continue;
-        const int u = F.lists[e];
+        const int u = F.lists[e0 + e];
         if (u >= 0) atomicAdd(X.rev_start + u + 1, 1);
     }
 }
@@ -201,11 +205,11 @@ __global__ void __launch_bounds__(1024) pm_fuse_rev_scan_kernel(FuseFrame F, Fus
 
 __global__ void pm_fuse_rev_fill_kernel(FuseFrame F, FuseWork X)
 {
-    const size_t n = (size_t)F.V * F.max_list;
+    const size_t n = (size_t)(X.v1 - X.v0) * F.max_list, e0 = (size_t)X.v0 * F.max_list;
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-        const int w = (int)(e / F.max_list), j = (int)(e - (size_t)w * F.max_list);
+        const int b = (int)(e / F.max_list), w = X.v0 + b, j = (int)(e - (size_t)b * F.max_list);
         if (!X.is_ref[w] || j >= F.list_counts[w]) continue;
-        const int u = F.lists[e];
+        const int u = F.lists[e0 + e];
         if (u >= 0) X.rev[atomicAdd(X.rev_fill + u, 1)] = make_int2(w, j);
     }
 }
@@ -234,16 +238,21 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int tar
 // One micro-image's walk by one warp.  taken: [1 + nl][mw] masks of the micro-image
 // itself and of its list entries (entries naming the same micro-image share the
 // first one's), fresh: [nl][mw] what this walk masks.  Publishes the difference.
+// LATER: the band is not the frame's first (a kernel of its own, since the places in the
+// band cost the registers that keep the first band's walk from spilling, 2% of it).
+template <bool LATER>
 __device__ __forceinline__ void walk_view(const FuseFrame& F, const FuseWork& X, int v, uint32_t* taken, uint32_t* fresh,
                                           int* changed_at)
 {
+    const int v0 = LATER ? X.v0 : 0;
+    const size_t vb = (size_t)(v - v0);                  // place in the band
     const int lane = threadIdx.x & 31, N = F.ppv, mw = X.mask_words;
     const int nl = min(F.list_counts[v], F.max_list);
     const int nch = (nl + 31) >> 5;
     const int* list = F.lists + (size_t)v * F.max_list;
     for (int e = lane; e < (1 + nl) * mw; e += 32) taken[e] = 0u;
     for (int e = lane; e < nl * mw; e += 32) fresh[e] = 0u;
-    const uint16_t* rows = X.pair_si + (size_t)v * N * F.max_list;
+    const uint16_t* rows = X.pair_si + vb * N * F.max_list;
     for (int b = lane * 128; b < N * F.max_list * 2; b += 32 * 128)
         asm volatile("prefetch.global.L1 [%0];" :: "l"((const char*)rows + b));
     // slot of each list entry: 0 for the micro-image itself, else 1 + the first entry
@@ -276,17 +285,22 @@ __device__ __forceinline__ void walk_view(const FuseFrame& F, const FuseWork& X,
             u = __shfl_sync(kFull, a, src);
             if (u < 0 || __shfl_sync(kFull, b, src) != t) continue;
         }
+        if (LATER)
+            for (int word = lane; word < mw; word += 32) {
+                const uint32_t bits = X.base[(size_t)u * mw + word];
+                if (bits) atomicOr(taken + t * mw + word, bits);
+            }
         const int r0 = X.rev_start[u], r1 = X.rev_start[u + 1];
         for (int e = r0 * mw + lane; e < r1 * mw; e += 32) {
             const int2 wj = X.rev[e / mw];
             if (wj.x >= v) continue;
             const int word = e % mw;
-            const uint32_t bits = __ldcg(X.marks + ((size_t)wj.x * F.max_list + wj.y) * mw + word);
+            const uint32_t bits = __ldcg(X.marks + ((size_t)(wj.x - v0) * F.max_list + wj.y) * mw + word);
             if (bits) atomicOr(taken + t * mw + word, bits);
         }
     }
     __syncwarp();
-    const uint32_t* maybe = X.maybe + (size_t)v * mw;
+    const uint32_t* maybe = X.maybe + vb * mw;
     for (int wd = 0; wd < mw; ++wd) {
         uint32_t todo = maybe[wd], accepted = 0u;
         while (todo) {
@@ -316,15 +330,15 @@ __device__ __forceinline__ void walk_view(const FuseFrame& F, const FuseWork& X,
                     atomicOr(taken + slot[ch] * mw + (si[ch] >> 5), 1u << (si[ch] & 31));
                     atomicOr(fresh + (ch * 32 + lane) * mw + (si[ch] >> 5), 1u << (si[ch] & 31));
                 }
-                if (lane == 0) X.chosen[((size_t)v * N + idx) * X.chosen_words + ch] = bits[ch];
+                if (lane == 0) X.chosen[(vb * N + idx) * X.chosen_words + ch] = bits[ch];
             }
             __syncwarp();
         }
-        if (lane == 0) X.accepted[(size_t)v * mw + wd] = accepted;
+        if (lane == 0) X.accepted[vb * mw + wd] = accepted;
     }
     __syncwarp();
     for (int e = lane; e < nl * mw; e += 32) {
-        uint32_t* g = X.marks + (size_t)v * F.max_list * mw + e;
+        uint32_t* g = X.marks + vb * F.max_list * mw + e;
         if (__ldcg(g) != fresh[e]) {
             __stcg(g, fresh[e]);
             atomicMin(changed_at + list[e / mw], v);
@@ -335,6 +349,7 @@ __device__ __forceinline__ void walk_view(const FuseFrame& F, const FuseWork& X,
 
 }  // namespace
 
+template <bool LATER>
 __global__ void __launch_bounds__(256) pm_fuse_resolve_kernel(FuseFrame F, FuseWork X, int* err)
 {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -350,7 +365,7 @@ __global__ void __launch_bounds__(256) pm_fuse_resolve_kernel(FuseFrame F, FuseW
         int* next = X.changed + (size_t)((round + 1) % 3) * F.V;
         for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < F.V; v += gridDim.x * blockDim.x) {
             __stcg(next + v, 0x7fffffff);
-            if (!X.is_ref[v]) continue;
+            if (v < X.v0 || v >= X.v1 || !X.is_ref[v]) continue;
             bool dirty = round == 1;
             if (!dirty) {
                 dirty = __ldcg(last + v) < v;
@@ -366,7 +381,7 @@ __global__ void __launch_bounds__(256) pm_fuse_resolve_kernel(FuseFrame F, FuseW
         const int n_list = (int)__ldcg(X.ctl + 1 + round % 3);
         if (n_list == 0) return;
         for (int i = blockIdx.x * warps + warp; i < n_list; i += gridDim.x * warps)
-            walk_view(F, X, __ldcg(X.list + i), taken, fresh, X.changed + (size_t)(round % 3) * F.V);
+            walk_view<LATER>(F, X, __ldcg(X.list + i), taken, fresh, X.changed + (size_t)(round % 3) * F.V);
         if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, 1);       // map order has no cycles: not reached
@@ -374,12 +389,13 @@ __global__ void __launch_bounds__(256) pm_fuse_resolve_kernel(FuseFrame F, FuseW
 
 __global__ void __launch_bounds__(256) pm_fuse_points_kernel(FuseFrame F, FuseWork X)
 {
-    const size_t n = (size_t)F.V * F.ppv;
+    const size_t n = (size_t)(X.v1 - X.v0) * F.ppv, first = (size_t)X.v0 * F.ppv;
     const int m = F.m;
     const float cm = __fadd_rn(__fmul_rn((float)(m - 1), 0.5f), 1.0f);
-    for (size_t seq = (size_t)blockIdx.x * blockDim.x + threadIdx.x; seq < n; seq += (size_t)gridDim.x * blockDim.x) {
-        const int v = (int)(seq / F.ppv), idx = (int)(seq - (size_t)v * F.ppv);
-        if (!X.is_ref[v] || !((X.accepted[(size_t)v * X.mask_words + (idx >> 5)] >> (idx & 31)) & 1u)) continue;
+    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (size_t)gridDim.x * blockDim.x) {
+        const size_t seq = first + q;
+        const int b = (int)(q / F.ppv), v = X.v0 + b, idx = (int)(q - (size_t)b * F.ppv);
+        if (!X.is_ref[v] || !((X.accepted[(size_t)b * X.mask_words + (idx >> 5)] >> (idx & 31)) & 1u)) continue;
         const float4 pl = F.plane[seq];
         const float vdr = virtual_depth(F.mla_base, pl.w);
         const int r = idx / m, c = idx - r * m;
@@ -388,12 +404,12 @@ __global__ void __launch_bounds__(256) pm_fuse_points_kernel(FuseFrame F, FuseWo
         int num = 0;
         const int nch = (min(F.list_counts[v], F.max_list) + 31) >> 5;
         for (int ch = 0; ch < nch; ++ch) {
-            uint32_t bits = X.chosen[seq * X.chosen_words + ch];
+            uint32_t bits = X.chosen[q * X.chosen_words + ch];
             num += __popc(bits);
             while (bits) {
                 const int j = ch * 32 + __ffs(bits) - 1;
                 bits &= bits - 1;
-                const int u = F.lists[(size_t)v * F.max_list + j], si = X.pair_si[seq * F.max_list + j];
+                const int u = F.lists[(size_t)v * F.max_list + j], si = X.pair_si[q * F.max_list + j];
                 const float4 ps = F.plane[(size_t)u * F.ppv + si];
                 const int sr = si / m, scol = si - sr * m;
                 const float3 Ps = virtual_3d(virtual_depth(F.mla_base, ps.w), scol, sr, cm, F.centers[u]);
@@ -478,64 +494,102 @@ __global__ void __launch_bounds__(kFuseScanBlock) pm_fuse_compact_kernel(FuseFra
     }
 }
 
-size_t fuse_work(const FuseFrame& F, unsigned char* buf, FuseWork& X)
+// What the band's micro-images mask, for the bands after it.
+__global__ void __launch_bounds__(256) pm_fuse_fold_kernel(FuseFrame F, FuseWork X)
+{
+    const int mw = X.mask_words;
+    const size_t n = (size_t)(X.v1 - X.v0) * F.max_list * mw;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const uint32_t bits = X.marks[i];
+        if (!bits) continue;
+        const size_t e = i / mw;
+        atomicOr(X.base + (size_t)F.lists[(size_t)X.v0 * F.max_list + e] * mw + (i - e * mw), bits);
+    }
+}
+
+size_t fuse_work(const FuseFrame& F, int n, unsigned char* buf, FuseWork& X)
 {
     size_t o = 0;
     auto take = [&](size_t bytes) { const size_t at = o; o += (bytes + 255) & ~(size_t)255; return buf + at; };
-    const size_t V = (size_t)F.V, px = V * F.ppv, L = (size_t)F.max_list;
+    const size_t V = (size_t)F.V, B = (size_t)n, px = B * F.ppv, L = (size_t)F.max_list;
     X.mask_words = (F.ppv + 31) / 32;
     X.chosen_words = (F.max_list + 31) / 32;
     X.zeroed = buf;
     X.ctl = (unsigned int*)take(16);
     X.rev_start = (int*)take(sizeof(int) * (V + 1));
-    X.marks = (uint32_t*)take(sizeof(uint32_t) * V * L * X.mask_words);
+    X.marks = (uint32_t*)take(sizeof(uint32_t) * B * L * X.mask_words);
     X.zeroed_bytes = o;
     X.changed = (int*)take(sizeof(int) * 3 * V);
     X.rev_fill = (int*)take(sizeof(int) * (V + 1));
-    X.rev = (int2*)take(sizeof(int2) * V * L);
-    X.list = (int*)take(sizeof(int) * V);
-    X.maybe = (uint32_t*)take(sizeof(uint32_t) * V * X.mask_words);
-    X.accepted = (uint32_t*)take(sizeof(uint32_t) * V * X.mask_words);
+    X.base = (uint32_t*)take(sizeof(uint32_t) * V * X.mask_words);
+    X.rev = (int2*)take(sizeof(int2) * B * L);
+    X.list = (int*)take(sizeof(int) * B);
+    X.maybe = (uint32_t*)take(sizeof(uint32_t) * B * X.mask_words);
+    X.accepted = (uint32_t*)take(sizeof(uint32_t) * B * X.mask_words);
     X.chosen = (uint32_t*)take(sizeof(uint32_t) * px * X.chosen_words);
     X.pair_si = (uint16_t*)take(sizeof(uint16_t) * px * L);
     return o;
 }
 
-cudaError_t launch_fuse(const FuseFrame& F, const FuseWork& X, int* err, cudaStream_t st)
+int fuse_band(const FuseFrame& F, size_t limit)
+{
+    FuseWork X;
+    const size_t all = fuse_work(F, F.V, nullptr, X), fixed = fuse_work(F, 0, nullptr, X);
+    if (all <= limit) return F.V;
+    const size_t per = (all - fixed + F.V - 1) / F.V;
+    const int most = limit > fixed ? (int)std::min<size_t>(std::max<size_t>((limit - fixed) / per, 1), F.V) : 1;
+    const int bands = (F.V + most - 1) / most;
+    return (F.V + bands - 1) / bands;                    // equal bands
+}
+
+cudaError_t launch_fuse(const FuseFrame& F, FuseWork X, int band, int* err, cudaStream_t st, unsigned long long* launches)
 {
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaMemsetAsync(X.zeroed, 0, X.zeroed_bytes, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(X.changed, 0x7f, sizeof(int) * 3 * (size_t)F.V, st);
-    if (e != cudaSuccess) return e;
-    const int flat = (int)std::min<size_t>(((size_t)F.V * F.max_list + 255) / 256, (size_t)sms * 8);
-    pm_fuse_pairs_kernel<<<F.V, std::min(256, (F.ppv + 31) & ~31), (F.max_list + 1) * 12 + 16, st>>>(F, X);
-    pm_fuse_rev_count_kernel<<<flat, 256, 0, st>>>(F, X);
-    pm_fuse_rev_scan_kernel<<<1, 1024, 0, st>>>(F, X);
-    pm_fuse_rev_fill_kernel<<<flat, 256, 0, st>>>(F, X);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const size_t per_warp = (size_t)(1 + 2 * F.max_list) * X.mask_words * 4;
     const int warps = (int)std::max<size_t>(1, std::min<size_t>(8, (size_t)96 * 1024 / per_warp));
     const int smem = (int)(per_warp * warps);
-    e = cudaFuncSetAttribute(pm_fuse_resolve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pm_fuse_resolve_kernel, 32 * warps, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)std::max(1, std::min((F.V + warps - 1) / warps, sms * std::min(per_sm, 4))));
-    lc.blockDim = dim3((unsigned)(32 * warps));
-    lc.dynamicSmemBytes = (size_t)smem;
-    lc.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeCooperative;
-    at[0].val.cooperative = 1;
-    lc.attrs = at;
-    lc.numAttrs = 1;
-    if ((e = cudaLaunchKernelEx(&lc, pm_fuse_resolve_kernel, F, X, err)) != cudaSuccess) return e;
-    const size_t px = (size_t)F.V * F.ppv;
-    pm_fuse_points_kernel<<<(int)std::min<size_t>((px + 255) / 256, (size_t)sms * 16), 256, 0, st>>>(F, X);
-    return cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    if (band < F.V) e = cudaMemsetAsync(X.base, 0, sizeof(uint32_t) * (size_t)F.V * X.mask_words, st);
+    for (X.v0 = 0; e == cudaSuccess && X.v0 < F.V; X.v0 = X.v1) {
+        X.v1 = std::min(F.V, X.v0 + band);
+        const int n = X.v1 - X.v0;
+        e = cudaMemsetAsync(X.zeroed, 0, X.zeroed_bytes, st);
+        if (e == cudaSuccess) e = cudaMemsetAsync(X.changed, 0x7f, sizeof(int) * 3 * (size_t)F.V, st);
+        if (e != cudaSuccess) return e;
+        const auto resolve = X.v0 ? pm_fuse_resolve_kernel<true> : pm_fuse_resolve_kernel<false>;
+        e = cudaFuncSetAttribute(resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resolve, 32 * warps, smem);
+        if (e != cudaSuccess) return e;
+        if (per_sm < 1) return cudaErrorInvalidConfiguration;
+        const int flat = (int)std::min<size_t>(((size_t)n * F.max_list + 255) / 256, (size_t)sms * 8);
+        pm_fuse_pairs_kernel<<<n, std::min(256, (F.ppv + 31) & ~31), (F.max_list + 1) * 12 + 16, st>>>(F, X);
+        pm_fuse_rev_count_kernel<<<flat, 256, 0, st>>>(F, X);
+        pm_fuse_rev_scan_kernel<<<1, 1024, 0, st>>>(F, X);
+        pm_fuse_rev_fill_kernel<<<flat, 256, 0, st>>>(F, X);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3((unsigned)std::max(1, std::min((n + warps - 1) / warps, sms * std::min(per_sm, 4))));
+        lc.blockDim = dim3((unsigned)(32 * warps));
+        lc.dynamicSmemBytes = (size_t)smem;
+        lc.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+        lc.attrs = at;
+        lc.numAttrs = 1;
+        if ((e = cudaLaunchKernelEx(&lc, resolve, F, X, err)) != cudaSuccess) return e;
+        const size_t px = (size_t)n * F.ppv;
+        pm_fuse_points_kernel<<<(int)std::min<size_t>((px + 255) / 256, (size_t)sms * 16), 256, 0, st>>>(F, X);
+        *launches += 6;
+        if (X.v1 < F.V) {
+            pm_fuse_fold_kernel<<<flat, 256, 0, st>>>(F, X);
+            *launches += 1;
+        }
+        e = cudaGetLastError();
+    }
+    return e;
 }
 
 cudaError_t launch_fuse_maps(const FuseFrame& F, float* vd_map, uint8_t* conf, uint8_t* aif, cudaStream_t st)

@@ -2215,12 +2215,21 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
     F.max_rel_vd = p->max_rel_vd; F.min_consistent = p->min_consistent;
     F.raw_w = f->W; F.raw_h = f->H;
     F.winner = d_winner; F.rec = d_rec; F.has_rec = d_has;
+    // The walk's work area takes up to 256 MB, or as much as the point records (40 bytes per
+    // pixel); in a context with a budget, what the budget has left (4 MB at least); and less
+    // where the device has less.  A band costs the latency of its own walk: a 1536x1159 frame
+    // of 128 list entries takes 51 ms in one band of 277 MB, 131 ms in eight.
+    size_t limit = std::max<size_t>((size_t)256 << 20, sizeof(float) * 10 * px);
+    if (ctx->budget) limit = std::min(limit, std::max<size_t>((size_t)4 << 20, ctx->budget - std::min(ctx->budget, ctx->used)));
     pfd::FuseWork X;
-    CU(S.get((void**)&d_work, pfd::fuse_work(F, nullptr, X)));
-    pfd::fuse_work(F, d_work, X);
+    int band = pfd::fuse_band(F, limit);
+    for (cudaError_t e; (e = S.get((void**)&d_work, pfd::fuse_work(F, band, nullptr, X))) != cudaSuccess; band = (band + 1) / 2) {
+        cudaGetLastError();
+        if (band == 1) return fail(ctx, PFD_ECUDA, "fuse: work area: %s", cudaGetErrorString(e));
+    }
+    pfd::fuse_work(F, band, d_work, X);
     X.is_ref = d_ref;
-    CU(pfd::launch_fuse(F, X, ctx->d_err, s));
-    ctx->launches += 6;
+    CU(pfd::launch_fuse(F, X, band, ctx->d_err, s, &ctx->launches));
     CU(pfd::launch_fuse_maps(F, d_vd, d_conf, d_aif, s));
     ctx->launches += 1;
     if (vd_map) CU(cudaMemcpyAsync(vd_map, d_vd, sizeof(float) * npix, cudaMemcpyDeviceToHost, s));
