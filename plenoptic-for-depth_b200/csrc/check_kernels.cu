@@ -40,6 +40,7 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include "check_kernels.h"
+#include "smem_limit.h"
 
 namespace pfd {
 
@@ -977,7 +978,7 @@ cudaError_t launch_cycle(const CheckFrame& F, const CycleCfg& cfg, const StateDe
     if (F.V <= 0) return cudaSuccess;
     const int N = F.W * F.H;
     const int smem = (1 + F.K) * F.tile_stride + F.K * (int)(sizeof(NbDir) + sizeof(int)) + N * 10;
-    cudaError_t e = cudaFuncSetAttribute(pm_cycle_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_dynamic_smem((const void*)pm_cycle_kernel);
     if (e != cudaSuccess) return e;
     const int threads = N < 256 ? ((N + 31) / 32) * 32 : 256;
     pm_cycle_kernel<<<F.V, threads < 64 ? 64 : threads, smem, s>>>(F, cfg, st, geo_err, pho_err, texmask, recs, hist);
@@ -1014,7 +1015,7 @@ cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const State
     const int smem_b = F.K * X.mask_words * 4 + N * 6;
     cudaError_t e = cudaMemsetAsync(X.zeroed, 0, X.zeroed_bytes, s);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(pm_filter_pairs_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_a);
+        e = allow_dynamic_smem((const void*)pm_filter_pairs_kernel);
     if (e != cudaSuccess) return e;
     const int threads = std::min(256, (N + 31) / 32 * 32);
     pm_filter_pairs_kernel<<<F.V, threads, smem_a, s>>>(F, cfg, st, X);
@@ -1053,7 +1054,7 @@ cudaError_t launch_filter_step(const CheckFrame& F, const FilterCfg& cfg, const 
     if (n_step <= 0) return cudaSuccess;
     const int smem = filter_smem_bytes(F);
     const int threads = F.W * F.H < 256 ? ((F.W * F.H + 31) / 32) * 32 : 256;
-    cudaError_t e = cudaFuncSetAttribute(pm_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_dynamic_smem((const void*)pm_filter_kernel);
     if (e != cudaSuccess) return e;
     pm_filter_kernel<<<n_step, threads, smem, s>>>(F, cfg, st, step_views, n_step, reason, stats);
     return cudaGetLastError();

@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cstdint>
 #include "fuse_kernels.h"
+#include "smem_limit.h"
 
 namespace pfd {
 
@@ -559,7 +560,7 @@ cudaError_t launch_fuse(const FuseFrame& F, FuseWork X, int band, int* err, cuda
         if (e == cudaSuccess) e = cudaMemsetAsync(X.changed, 0x7f, sizeof(int) * 3 * (size_t)F.V, st);
         if (e != cudaSuccess) return e;
         const auto resolve = X.v0 ? pm_fuse_resolve_kernel<true> : pm_fuse_resolve_kernel<false>;
-        e = cudaFuncSetAttribute(resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        e = allow_dynamic_smem((const void*)resolve);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resolve, 32 * warps, smem);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;

@@ -38,6 +38,7 @@
 #include "pm_device.cuh"
 #include "pm_kernels.h"
 #include "pm_sweep_device.cuh"
+#include "smem_limit.h"
 
 namespace pfd {
 
@@ -1015,7 +1016,7 @@ size_t sweep_warp_scratch_bytes(const PmParams& P, int n_ctas)
 // L1 and texture cache.
 static cudaError_t set_smem(const void* k, int smem, bool tex)
 {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_dynamic_smem(k);
     if (e != cudaSuccess || !tex) return e;
     const long need = (long)kMinCtas * (smem + 1024);
     const int pct = (int)std::min<long>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024) + 1);

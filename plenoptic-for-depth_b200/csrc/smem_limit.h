@@ -1,0 +1,18 @@
+// smem_limit.h -- dynamic shared memory above the default 48 KB.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace pfd {
+
+// Lets kernel k be launched with all the shared memory of an SM that one CTA may have.
+// The limit belongs to the kernel, not to a launch: one made for each call's own size
+// would be taken back by another thread's smaller call before this one's launch.
+inline cudaError_t allow_dynamic_smem(const void* k)
+{
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, k);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)a.sharedSizeBytes);
+}
+
+}  // namespace pfd
