@@ -117,12 +117,13 @@ def build_synth(force: bool = False) -> str:
 TEST_OUT = os.path.join(ROOT, "tests", "_build")
 TEX_PROBE = os.path.join(TEST_OUT, "libtexprobe.so")
 FMA_PROBE = os.path.join(TEST_OUT, "libfmaprobe.so")
+FILTER_PROBE = os.path.join(TEST_OUT, "libfilterprobe.so")
 SHIM_PROBE = os.path.join(TEST_OUT, "libshimprobe.so")
 
 
 def build_test_helpers(force: bool = False) -> str:
     """Compile the device probes the tests and bench.py use (the texture
-    probe, the FP32 throughput probe) and the C++ drop-in probe."""
+    probe, the FP32 throughput probe, the filter's last launch) and the C++ drop-in probe."""
     os.makedirs(TEST_OUT, exist_ok=True)
     for name, lib_path in (("tex_probe.cu", TEX_PROBE), ("fma_probe.cu", FMA_PROBE)):
         src = os.path.join(ROOT, "tests", "csrc", name)
@@ -131,6 +132,13 @@ def build_test_helpers(force: bool = False) -> str:
             _run([NVCC, *ARCH, "-O2", "-shared", "-Xcompiler", "-fPIC", "-ccbin", "/usr/bin/g++", src, "-o", tmp])
             os.replace(tmp, lib_path)
     host = build_host()
+    src = os.path.join(ROOT, "tests", "csrc", "filter_probe.cu")
+    if force or _stale(FILTER_PROBE, [src, LIB, __file__]):
+        tmp = FILTER_PROBE + ".tmp"
+        _run([NVCC, *ARCH, "-std=c++17", "-O2", "-shared", "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-ccbin",
+              "/usr/bin/g++", "-I", CSRC, src, "-o", tmp, "-L", OUT, "-l:libpfd.so", "-Xlinker",
+              "-rpath=$ORIGIN/" + os.path.relpath(OUT, TEST_OUT)])
+        os.replace(tmp, FILTER_PROBE)
     src = os.path.join(ROOT, "tests", "csrc", "shim_probe.cpp")
     if force or _stale(SHIM_PROBE, [src, host, __file__] + _deps()):
         tmp = SHIM_PROBE + ".tmp"

@@ -21,7 +21,9 @@
 //                             this ends at the one solution, the sequential walk's.
 //                             A cooperative launch; the grid barrier's waits are
 //                             bounded.
-//   pm_filter_apply_kernel    reasons, counters and the rejected pixels' state.
+//   pm_filter_apply_kernel    reasons, counters and the rejected pixels' state; nothing
+//                             when the masks did not settle (a wait gave up), so that a
+//                             reported timeout leaves the state as it was.
 // A rejected pixel gets disparity -1; where the configuration accepts such a
 // disparity (min_valid_disp < -1) it is not an unusable one, and the filter runs as
 // a wavefront instead (pm_filter_kernel): micro-image (col, row) in step
@@ -40,6 +42,7 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include "check_kernels.h"
+#include "grid_barrier.cuh"
 #include "smem_limit.h"
 
 namespace pfd {
@@ -529,25 +532,6 @@ __device__ __forceinline__ void eval_view(const CheckFrame& F, const FilterCfg& 
     __syncthreads();
 }
 
-// Barrier of the whole (cooperative) grid: bounded wait, records a timeout and gives up.
-__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int target, int* err)
-{
-    __syncthreads();
-    int ok = 1;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        ok = 0;
-        for (unsigned int it = 0; it < (1u << 22); ++it) {
-            if (*(volatile unsigned int*)bar >= target) { ok = 1; break; }
-            if (it > 32) __nanosleep(64);
-        }
-        __threadfence();
-        if (!ok) atomicOr(err, 1);
-    }
-    return __syncthreads_and(ok) != 0;
-}
-
 }  // namespace
 
 __global__ void __launch_bounds__(256) pm_filter_resolve_kernel(CheckFrame F, FilterCfg cfg, FilterWork X, int* err)
@@ -559,7 +543,12 @@ __global__ void __launch_bounds__(256) pm_filter_resolve_kernel(CheckFrame F, Fi
     uint8_t* keep = (uint8_t*)(dv + N);                  // [N]
     uint8_t* why = keep + N;                             // [N]
     unsigned int arrived = 0;
-    // X.ctl: 0 barrier; 1, 2, 3 list lengths of rounds 1, 2, 3 mod 3
+    // X.ctl: 0 barrier; 1, 2, 3 list lengths of rounds 1, 2, 3 mod 3; 4 settled; 5 a wait gave up
+    auto barrier = [&]() {
+        const bool ok = grid_barrier(X.ctl, ++arrived * gridDim.x, err);
+        if (!ok && threadIdx.x == 0) X.ctl[kFilterGaveUp] = 1u;
+        return ok;
+    };
     for (int round = 1; round <= F.V + 2; ++round) {
         // views with an earlier neighbour that changed in the last round (or already in
         // this one); all of them in the first round
@@ -576,9 +565,12 @@ __global__ void __launch_bounds__(256) pm_filter_resolve_kernel(CheckFrame F, Fi
                 }
                 if (dirty) X.list[atomicAdd(X.ctl + 1 + round % 3, 1u)] = v;
             }
-            if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
+            if (!barrier()) return;
             n_list = (int)__ldcg(X.ctl + 1 + round % 3);
-            if (n_list == 0) return;
+            if (n_list == 0) {
+                if (blockIdx.x == 0 && threadIdx.x == 0) X.ctl[kFilterSettled] = 1u;
+                return;
+            }
         }
         for (int i = blockIdx.x; i < n_list; i += gridDim.x) {
             const int v = round > 1 ? __ldcg(X.list + i) : i;
@@ -594,15 +586,16 @@ __global__ void __launch_bounds__(256) pm_filter_resolve_kernel(CheckFrame F, Fi
             }
             if (__syncthreads_or(diff) && threadIdx.x == 0) __stcg(X.changed + v, round);
         }
-        if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
+        if (!barrier()) return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, 1);       // key order has no cycles: not reached
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, PFD_DEVERR_TMA_TIMEOUT);       // key order has no cycles: not reached
 }
 
 __global__ void __launch_bounds__(256) pm_filter_apply_kernel(CheckFrame F, FilterCfg cfg, StateDev st, FilterWork X,
                                                               uint8_t* reason, unsigned long long* stats)
 {
     extern __shared__ __align__(16) unsigned char smem[];
+    if (!X.ctl[kFilterSettled] || X.ctl[kFilterGaveUp]) return;
     const int N = F.W * F.H, v = blockIdx.x;
     uint32_t* nmask = (uint32_t*)smem;
     float* dv = (float*)(nmask + F.K * X.mask_words);
@@ -986,7 +979,7 @@ cudaError_t launch_cycle(const CheckFrame& F, const CycleCfg& cfg, const StateDe
 }
 
 // Room per micro-image of P >= 4 pixels: the idle state holds 16 P bytes in plane (8 P
-// needed), 16 P in disp (4 + 4 ceil(P / 32), and 16 for ctl once: 28 <= 64 at P = 4), 4 P
+// needed), 16 P in disp (4 + 4 ceil(P / 32), and 32 for ctl once: 40 <= 64 at P = 4), 4 P
 // in sel (4); the cost vectors hold 4 K P (2 K P: a pixel has at most one test per
 // neighbour, whatever max_triplet).
 FilterWork filter_work(const CheckFrame& F, const StateDev& idle, float* cvec)
@@ -997,27 +990,36 @@ FilterWork filter_work(const CheckFrame& F, const StateDev& idle, float* cvec)
     X.head = (uint32_t*)idle.plane;
     X.disp = (float*)(X.head + X.total);
     X.ctl = (unsigned int*)idle.disp;
-    X.changed = (int*)(X.ctl + 4);
+    X.changed = (int*)(X.ctl + 8);
     X.mask = (uint32_t*)(X.changed + F.V);
     X.zeroed = (unsigned char*)X.ctl;
-    X.zeroed_bytes = 16 + 4 * (size_t)F.V * (1 + X.mask_words);
+    X.zeroed_bytes = 32 + 4 * (size_t)F.V * (1 + X.mask_words);
     X.list = (int*)idle.sel;
     X.ent = (uint16_t*)cvec;
     return X;
+}
+
+static int filter_threads(const CheckFrame& F) { return std::min(256, (F.W * F.H + 31) / 32 * 32); }
+static int filter_mask_smem(const CheckFrame& F, const FilterWork& X) { return F.K * X.mask_words * 4 + F.W * F.H * 6; }
+
+cudaError_t launch_filter_apply(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,
+                                uint8_t* reason, unsigned long long* stats, cudaStream_t s)
+{
+    pm_filter_apply_kernel<<<F.V, filter_threads(F), filter_mask_smem(F, X), s>>>(F, cfg, st, X, reason, stats);
+    return cudaGetLastError();
 }
 
 cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,
                           uint8_t* reason, unsigned long long* stats, int* err, cudaStream_t s)
 {
     if (F.V <= 0) return cudaSuccess;
-    const int N = F.W * F.H;
     const int smem_a = (1 + F.K) * F.tile_stride + F.K * (int)(sizeof(NbDir) + sizeof(int));
-    const int smem_b = F.K * X.mask_words * 4 + N * 6;
+    const int smem_b = filter_mask_smem(F, X);
     cudaError_t e = cudaMemsetAsync(X.zeroed, 0, X.zeroed_bytes, s);
     if (e == cudaSuccess)
         e = allow_dynamic_smem((const void*)pm_filter_pairs_kernel);
     if (e != cudaSuccess) return e;
-    const int threads = std::min(256, (N + 31) / 32 * 32);
+    const int threads = filter_threads(F);
     pm_filter_pairs_kernel<<<F.V, threads, smem_a, s>>>(F, cfg, st, X);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     int dev = 0, sms = 0, per_sm = 0;
@@ -1038,8 +1040,7 @@ cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const State
     lc.numAttrs = 1;
     e = cudaLaunchKernelEx(&lc, pm_filter_resolve_kernel, F, cfg, X, err);
     if (e != cudaSuccess) return e;
-    pm_filter_apply_kernel<<<F.V, threads, smem_b, s>>>(F, cfg, st, X, reason, stats);
-    return cudaGetLastError();
+    return launch_filter_apply(F, cfg, st, X, reason, stats, s);
 }
 
 int filter_smem_bytes(const CheckFrame& F)

@@ -81,7 +81,7 @@ struct FilterWork {
     int mask_words;            // 32-bit words of a micro-image's mask
     unsigned char* zeroed;     // the part that starts at zero: ctl, changed, mask
     size_t zeroed_bytes;
-    unsigned int* ctl;
+    unsigned int* ctl;         // [8], see kFilterSettled
     int* changed;              // [V] round in which the mask last changed
     uint32_t* mask;            // [V][mask_words] rejected pixels
     int* list;                 // [V] micro-images of the round
@@ -90,9 +90,16 @@ struct FilterWork {
     uint16_t* ent;             // [K][total] tests against earlier neighbours
 };
 FilterWork filter_work(const CheckFrame& F, const StateDev& idle, float* cvec);
-// The whole filter, three launches; err gets flag 1 when a device wait gave up.
+// Words of ctl: the masks are the fixed point; a wait of the resolution gave up.
+constexpr int kFilterSettled = 4, kFilterGaveUp = 5;
+// The whole filter, three launches; err gets PFD_DEVERR_TMA_TIMEOUT when a device wait
+// gave up, and the state is then as it was.
 cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,
                           uint8_t* reason, unsigned long long* stats, int* err, cudaStream_t s);
+
+// Its last launch: reasons, counters and state from the settled masks, else nothing.
+cudaError_t launch_filter_apply(const CheckFrame& F, const FilterCfg& cfg, const StateDev& st, const FilterWork& X,
+                                uint8_t* reason, unsigned long long* stats, cudaStream_t s);
 
 int filter_smem_bytes(const CheckFrame& F);
 // One wavefront step: the views step_views[0..n_step) filtered in parallel.

@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cstdint>
 #include "fuse_kernels.h"
+#include "grid_barrier.cuh"
 #include "smem_limit.h"
 
 namespace pfd {
@@ -217,25 +218,6 @@ __global__ void pm_fuse_rev_fill_kernel(FuseFrame F, FuseWork X)
 
 namespace {
 
-// Barrier of the whole (cooperative) grid: bounded wait, records a timeout and gives up.
-__device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int target, int* err)
-{
-    __syncthreads();
-    int ok = 1;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        ok = 0;
-        for (unsigned int it = 0; it < (1u << 22); ++it) {
-            if (*(volatile unsigned int*)bar >= target) { ok = 1; break; }
-            if (it > 32) __nanosleep(64);
-        }
-        __threadfence();
-        if (!ok) atomicOr(err, 1);
-    }
-    return __syncthreads_and(ok) != 0;
-}
-
 // One micro-image's walk by one warp.  taken: [1 + nl][mw] masks of the micro-image
 // itself and of its list entries (entries naming the same micro-image share the
 // first one's), fresh: [nl][mw] what this walk masks.  Publishes the difference.
@@ -385,7 +367,7 @@ __global__ void __launch_bounds__(256) pm_fuse_resolve_kernel(FuseFrame F, FuseW
             walk_view<LATER>(F, X, __ldcg(X.list + i), taken, fresh, X.changed + (size_t)(round % 3) * F.V);
         if (!grid_barrier(X.ctl, ++arrived * gridDim.x, err)) return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, 1);       // map order has no cycles: not reached
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, PFD_DEVERR_TMA_TIMEOUT);       // map order has no cycles: not reached
 }
 
 __global__ void __launch_bounds__(256) pm_fuse_points_kernel(FuseFrame F, FuseWork X)
