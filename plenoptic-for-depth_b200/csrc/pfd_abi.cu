@@ -131,6 +131,7 @@ struct Frame {
     std::vector<void*> allocs;
     // host copies for scheduling the consistency pass
     std::vector<int> h_keys, h_nb_ids, h_nb_counts;
+    bool keys_dense = false;          // no neighbour lists make the filter's schedule too long (dense_keys)
     uint8_t* d_reason = nullptr;      // filter reject reasons, allocated on first use
     float* d_err = nullptr;           // reprojection-error map, allocated on first use
     int* d_steps = nullptr;           // views grouped by wavefront step
@@ -602,6 +603,21 @@ pfd_status pfd_sync(pfd_ctx* ctx)
     return check_device_error(ctx);
 }
 
+// The filter's schedule (build_steps) may have kMaxFilterSteps steps.  Its column weight
+// is at most one more than the columns' extent, which bounds the steps whatever the
+// neighbour lists are.
+static const long long kMaxFilterSteps = 100000000LL;
+static bool dense_keys(const std::vector<int>& keys)
+{
+    int lo[2] = { INT_MAX, INT_MAX }, hi[2] = { INT_MIN, INT_MIN };
+    for (size_t i = 0; i < keys.size(); ++i) {
+        lo[i & 1] = std::min(lo[i & 1], keys[i]);
+        hi[i & 1] = std::max(hi[i & 1], keys[i]);
+    }
+    const double cols = (double)hi[0] - lo[0], rows = (double)hi[1] - lo[1];
+    return cols + (cols + 1.0) * rows + 1.0 <= (double)kMaxFilterSteps;
+}
+
 pfd_status pfd_frame_create(pfd_ctx* ctx, int* frame_id, int W, int H, const float* centers, const int* tilekeys,
                             int n_views, int mi_w, int mi_h, const int* nb_ids, const int* nb_counts, int max_nb,
                             const uint8_t* blur)
@@ -686,6 +702,7 @@ pfd_status pfd_frame_create(pfd_ctx* ctx, int* frame_id, int W, int H, const flo
         return fail(ctx, st, "frame_create: upload failed");
     }
     f.h_keys.assign(tilekeys, tilekeys + 2 * (size_t)n_views);
+    f.keys_dense = dense_keys(f.h_keys);
     f.h_centers.assign(centers, centers + 2 * (size_t)n_views);
     f.h_nb_ids.assign(nb_ids, nb_ids + (size_t)n_views * max_nb);
     f.h_nb_counts.assign(nb_counts, nb_counts + n_views);
@@ -1598,7 +1615,7 @@ static pfd_status build_steps(pfd_ctx* ctx, Frame& f)
         smax = std::max(smax, step[v]);
     }
     const long long ns = smax - smin + 1;
-    if (ns > 100000000LL) return fail(ctx, PFD_EINVAL, "tile keys too sparse for the filter schedule");
+    if (ns > kMaxFilterSteps) return fail(ctx, PFD_EINVAL, "tile keys too sparse for the filter schedule");
     std::vector<int> counts((size_t)ns + 1, 0), order(V);
     for (int v = 0; v < V; ++v) counts[(size_t)(step[v] - smin) + 1]++;
     for (size_t i = 1; i < counts.size(); ++i) counts[i] += counts[i - 1];
@@ -1649,7 +1666,8 @@ pfd_status pfd_filter(pfd_ctx* ctx, int frame_id, const pfd_filter_cfg* cfg, flo
     // three launches; as a wavefront where a rejected pixel's disparity (-1) counts as
     // usable (the same result, 10x slower)
     const bool wavefront = !(fc.min_valid_disp >= -1.0f);
-    if (wavefront && (st = build_steps(ctx, *f)) != PFD_OK) return st;
+    // keys that the wavefront refuses are refused either way
+    if ((wavefront || !f->keys_dense) && (st = build_steps(ctx, *f)) != PFD_OK) return st;
     const pfd::FilterWork X = pfd::filter_work(F, f->s[f->cur ^ 1], f->d_cvec);
     // enqueue-only calls under pfd_set_graphs: the first call with a key runs as
     // usual, the second is captured, later ones replay the graph (it reads the

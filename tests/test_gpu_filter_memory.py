@@ -114,3 +114,28 @@ def test_sweeps_go_on_after_a_filter(pfd, oracle):
             ctx.filter(fid, pfd.FilterCfg(min_good_neighbors=1), BASE)
             oracle.filter_global(orc, pfd.FilterCfg(min_good_neighbors=1), BASE, st)
             _equal(ctx.download(fid), st)
+
+
+@pytest.mark.parametrize("far,ok", [((0, 200_000_000), False), ((90_000, 1000), True), ((100_000, 100_000), True),
+                                    ((-2**31, 2**31 - 1), True)])
+def test_tile_keys_too_sparse_for_a_schedule_are_refused(pfd, far, ok):
+    """As by the wavefront, whichever form runs: keys whose schedule would have more
+    than 10^8 steps.  The last two pairs' bound says so, their schedules do not: with
+    column weight 1 the far key is in step 200000, or in step -1."""
+    rs = np.random.RandomState(7)
+    cen, keys, gray, ids, cnt = _frame(rs, 3, 1, 16, 16, 2)
+    keys = np.array([[0, 0], [1, 1], far], np.int32)
+    ids[:] = -1
+    ids[0, 0], ids[1, 0], cnt[:] = 1, 0, (1, 1, 0)
+    with pfd.Context(0) as ctx:
+        fid = _create(ctx, (cen, keys, gray, ids, cnt), 16, 16)
+        st = _state(rs, 3, 16, 16, 2)
+        ctx.state_upload(fid, st["plane"], st["cost"], st["disp"], st["sel"])
+        for low in (0.0, -2.0):
+            if ok and low < -1 and far[0] < 100_000:
+                continue                                  # the wavefront of 9 10^7 steps is left out
+            if ok:
+                ctx.filter(fid, pfd.FilterCfg(min_valid_disp=low), BASE)
+            else:
+                with pytest.raises(pfd.PfdError, match="too sparse"):
+                    ctx.filter(fid, pfd.FilterCfg(min_valid_disp=low), BASE)
