@@ -2123,10 +2123,11 @@ pfd_status pfd_refocus(pfd_ctx* ctx, int frame_id, const float* slice_vd, int n_
     R.grid_w = f->grid_w; R.grid_h = f->grid_h;
     R.grid_x0 = f->grid_x0; R.grid_y0 = f->grid_y0; R.cell = f->grid_cell;
     CU(cudaMemcpyAsync(f->d_slice_vd, slice_vd, sizeof(float) * n_slices, cudaMemcpyHostToDevice, ctx->stream));
+    // the packed micro-images (4 bytes per pixel) lie in the state buffer that is not the
+    // current one (16 per pixel in plane): the next half-sweep writes all of it
     cudaError_t e;
-    AsyncBuf quads(ctx->stream, pfd::refocus_quads_bytes(R), e);
-    if (e != cudaSuccess) { cudaGetLastError(); return fail(ctx, PFD_ENOMEM, "refocus: packed micro-images"); }
-    CU(pfd::launch_refocus_quads(R, (uint32_t*)quads.p, ctx->stream));
+    uint32_t* quads = (uint32_t*)f->s[f->cur ^ 1].plane;
+    CU(pfd::launch_refocus_quads(R, quads, ctx->stream));
     ctx->launches += 1;
     // A stack for the host is rendered in up to 8 groups of slices, and the copy of one
     // runs beside the rendering of the next; what is left is the copy and the first group's
@@ -2136,7 +2137,7 @@ pfd_status pfd_refocus(pfd_ctx* ctx, int frame_id, const float* slice_vd, int n_
     const int groups = out ? (int)std::max<size_t>(1, std::min<size_t>(std::min(8, n_slices), need >> 23)) : 1;
     const int per = (n_slices + groups - 1) / groups;
     if (groups == 1) {
-        CU(pfd::launch_refocus(R, (const uint32_t*)quads.p, f->d_slice_vd, n_slices, f->W, f->H, out_w, out_h, f->d_stack,
+        CU(pfd::launch_refocus(R, quads, f->d_slice_vd, n_slices, f->W, f->H, out_w, out_h, f->d_stack,
                                ctx->d_err, ctx->stream));
         ctx->launches += 1;
         if (out) CU(cudaMemcpyAsync(out, f->d_stack, need, cudaMemcpyDeviceToHost, ctx->stream));
@@ -2147,7 +2148,7 @@ pfd_status pfd_refocus(pfd_ctx* ctx, int frame_id, const float* slice_vd, int n_
     e = cudaSuccess;
     // every launch before the first copy: a copy to pageable memory blocks the host
     for (int s0 = 0; s0 < n_slices && e == cudaSuccess; s0 += per) {
-        e = pfd::launch_refocus(R, (const uint32_t*)quads.p, f->d_slice_vd + s0, std::min(per, n_slices - s0), f->W, f->H,
+        e = pfd::launch_refocus(R, quads, f->d_slice_vd + s0, std::min(per, n_slices - s0), f->W, f->H,
                                 out_w, out_h, f->d_stack + s0 * slice, ctx->d_err, ctx->stream);
         ctx->launches += 1;
         if (e == cudaSuccess) e = ev.record(ctx->stream);

@@ -212,8 +212,6 @@ __global__ void __launch_bounds__(kThreads) pm_refocus_kernel(RefocusFrame F, co
     }
 }
 
-size_t refocus_quads_bytes(const RefocusFrame& F) { return sizeof(uint32_t) * (size_t)F.V * F.m * F.mh; }
-
 cudaError_t launch_refocus_quads(const RefocusFrame& F, uint32_t* quads, cudaStream_t st)
 {
     const size_t px = (size_t)F.V * F.m * F.mh;

@@ -21,8 +21,7 @@ struct RefocusFrame {
 constexpr int kMaxRefocusCand = 2048;             // lenses that may reach one 64 x 16 output tile
 #define PFD_DEVERR_REFOCUS_LENSES 0x2             // a tile saw more than kMaxRefocusCand lenses
 
-// Bytes of the packed micro-images a render lays out for itself.
-size_t refocus_quads_bytes(const RefocusFrame& F);
+// The packed micro-images a render lays out for itself: quads[V * m * mh].
 cudaError_t launch_refocus_quads(const RefocusFrame& F, uint32_t* quads, cudaStream_t st);
 // Renders n_slices slices into out from the packed micro-images.
 cudaError_t launch_refocus(const RefocusFrame& F, const uint32_t* quads, const float* slice_vd, int n_slices, int raw_w,
