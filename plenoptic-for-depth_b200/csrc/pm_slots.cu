@@ -1881,10 +1881,16 @@ int slots_shape_ctas(int shape) { return kShapeCtas[(shape >= 0 && shape < kSwee
 // Slots, list capacity and parts of a half-sweep; returns the dynamic shared
 // memory of its plan, or 0 when none fits.  A launch of fewer than six items per
 // CTA splits its micro-images, so that no CTA is without work and the last ones end
-// together; a part stages the micro-image anew and drains its slots, so larger frames
-// and parts of fewer pixels than slots lose.  Half-sweep at 1, 2, 4 and 8 parts: 182
-// micro-images of 21x21 on 296 CTAs .38, .31, .30, .37 ms; 1672 of 23x23 (5.6 items per
-// CTA) 3.20, 3.08, 3.14, 3.88 ms; 6612 of 16x16 (22 items) 23.0, 23.7, 25.2, 28.1 ms.
+// together; a part stages the micro-image anew and drains its slots.  Measured at 1, 2, 4
+// and 8 parts over 63 frames, 0.3 to 22 micro-images per CTA, windows of 10x10 to
+// 20x20, patches of 5x5 to 15x15, with and without blur and ACMM: the rule's choice is
+// 1.1% off the best on average, 2.4% with the line at two items.  Half-sweep, ms (16x16,
+// 12 neighbours, 15x15, 296 CTAs): 195 micro-images 1.19, .92, .93, .98; 1554 (5.3 items)
+// 6.02, 5.85, 6.13, 6.77; 1840 (6.2) 6.84, 6.90, 7.23, 7.98; 6612 23.3, 24.1, 25.5, 28.4.
+// ACMM (5x5) gains 2-5% from two parts also above six items.  No part gets fewer pixels
+// than slots: 10x10 windows (50 pixels, 32 slots) at one and two parts .41 and .43 ms at
+// 2.2 items, .72 and .75 at 4.1; the smallest frames would gain (100 of them, .3 items:
+// .141 and .123 ms).
 int slots_plan(PmParams& P, bool blur, int shape, int n_views)
 {
     const int warps = slots_shape_warps(shape);
