@@ -1293,14 +1293,10 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
     }
     DeviceGuard g(ctx->device);
     {
-        // A frame that fills the sweep's grid often enough gains nothing from sharing a
-        // launch (its last wave is a small part of its work); such frames run as their own
-        // launches, the others share launches.  Six equal frames of 16x16, time of one
-        // shared launch over that of six: 0.98, 0.93, 0.97 at 323 micro-images (6
-        // neighbours, 11x11; 12, 15x15; ACMM, 5x5), 1.00, 0.97, 1.02 at 648, 1.03, 1.00,
-        // 1.04 at 957, 1.03, 1.02, 1.05 at 1254, 1.08, 1.08, 1.09 at 6776, on a grid of 296
-        // CTAs; two frames of 1020 1.06, 1.05, 1.09.  So from three micro-images per CTA on;
-        // the texture kernel's grid (592 CTAs) from four, measured with that kernel.
+        // A frame whose micro-images fill the sweep's grid four times over or more gains
+        // nothing from sharing a launch (its last wave is a small part of its work) and
+        // measured 4-5% slower inside one (2048x1536 and 4080x3068 frames of the mixed
+        // set); such frames run as their own launches, the others share launches.
         std::vector<int> solo, rest;
         for (int b = 0; b < n; ++b) {
             int n_ctas = 0;
@@ -1312,7 +1308,7 @@ pfd_status pfd_patchmatch_batch(pfd_ctx* ctx, const int* frame_ids, int n, const
                 cudaGetLastError();
                 n_ctas = 0;
             }
-            (n_ctas > 0 && fr[b]->V >= (F.tex ? 4 : 3) * n_ctas ? solo : rest).push_back(b);
+            (n_ctas > 0 && fr[b]->V >= 4 * n_ctas ? solo : rest).push_back(b);
         }
         if (!solo.empty()) {
             for (int b : solo) {
