@@ -971,7 +971,7 @@ cudaError_t launch_cycle(const CheckFrame& F, const CycleCfg& cfg, const StateDe
     if (F.V <= 0) return cudaSuccess;
     const int N = F.W * F.H;
     const int smem = (1 + F.K) * F.tile_stride + F.K * (int)(sizeof(NbDir) + sizeof(int)) + N * 10;
-    cudaError_t e = allow_dynamic_smem((const void*)pm_cycle_kernel);
+    cudaError_t e = allow_dynamic_smem((const void*)pm_cycle_kernel, smem);
     if (e != cudaSuccess) return e;
     const int threads = N < 256 ? ((N + 31) / 32) * 32 : 256;
     pm_cycle_kernel<<<F.V, threads < 64 ? 64 : threads, smem, s>>>(F, cfg, st, geo_err, pho_err, texmask, recs, hist);
@@ -1017,7 +1017,7 @@ cudaError_t launch_filter(const CheckFrame& F, const FilterCfg& cfg, const State
     const int smem_b = filter_mask_smem(F, X);
     cudaError_t e = cudaMemsetAsync(X.zeroed, 0, X.zeroed_bytes, s);
     if (e == cudaSuccess)
-        e = allow_dynamic_smem((const void*)pm_filter_pairs_kernel);
+        e = allow_dynamic_smem((const void*)pm_filter_pairs_kernel, smem_a);
     if (e != cudaSuccess) return e;
     const int threads = filter_threads(F);
     pm_filter_pairs_kernel<<<F.V, threads, smem_a, s>>>(F, cfg, st, X);
@@ -1055,7 +1055,7 @@ cudaError_t launch_filter_step(const CheckFrame& F, const FilterCfg& cfg, const 
     if (n_step <= 0) return cudaSuccess;
     const int smem = filter_smem_bytes(F);
     const int threads = F.W * F.H < 256 ? ((F.W * F.H + 31) / 32) * 32 : 256;
-    cudaError_t e = allow_dynamic_smem((const void*)pm_filter_kernel);
+    cudaError_t e = allow_dynamic_smem((const void*)pm_filter_kernel, smem);
     if (e != cudaSuccess) return e;
     pm_filter_kernel<<<n_step, threads, smem, s>>>(F, cfg, st, step_views, n_step, reason, stats);
     return cudaGetLastError();

@@ -542,7 +542,7 @@ cudaError_t launch_fuse(const FuseFrame& F, FuseWork X, int band, int* err, cuda
         if (e == cudaSuccess) e = cudaMemsetAsync(X.changed, 0x7f, sizeof(int) * 3 * (size_t)F.V, st);
         if (e != cudaSuccess) return e;
         const auto resolve = X.v0 ? pm_fuse_resolve_kernel<true> : pm_fuse_resolve_kernel<false>;
-        e = allow_dynamic_smem((const void*)resolve);
+        e = allow_dynamic_smem((const void*)resolve, smem);
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, resolve, 32 * warps, smem);
         if (e != cudaSuccess) return e;
         if (per_sm < 1) return cudaErrorInvalidConfiguration;

@@ -298,7 +298,7 @@ __global__ void __launch_bounds__(256) pm_ncc_kernel(FrameDev F, PmParams P, con
 template <class Kern>
 static cudaError_t launch(Kern k, dim3 grid, dim3 block, int smem, cudaStream_t st, void** args)
 {
-    cudaError_t e = allow_dynamic_smem((const void*)k);
+    cudaError_t e = allow_dynamic_smem((const void*)k, smem);
     if (e != cudaSuccess) return e;
     return cudaLaunchKernel((const void*)k, grid, block, args, (size_t)smem, st);
 }

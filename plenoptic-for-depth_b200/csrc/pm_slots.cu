@@ -1862,7 +1862,7 @@ cudaError_t launch_init(const FrameDev& F, const PmParams& P, const StateDev& ou
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = allow_dynamic_smem(k);
+    cudaError_t e = allow_dynamic_smem(k, smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * kInitWarps, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
@@ -1964,7 +1964,7 @@ static cudaError_t slots_grid(const void* k, int threads, int smem, int* n_ctas)
     int dev = 0, sms = 0, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = allow_dynamic_smem(k);
+    cudaError_t e = allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem);
     if (e != cudaSuccess) return e;
@@ -1985,7 +1985,7 @@ cudaError_t launch_slots_sweep(const FrameDev& F, const PmParams& P, const State
     if (smem <= 0 || smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     shape = one_cta_shape(shape, smem);
     const void* k = slots_kernel(shape, F.blur != nullptr, P.shifted != 0);
-    cudaError_t e = allow_dynamic_smem(k);
+    cudaError_t e = allow_dynamic_smem(k, smem);
     if (e == cudaSuccess) e = cudaMemsetAsync(P.view_queue, 0, sizeof(int), st);
     if (e != cudaSuccess) return e;
     const int grid = std::max(1, (int)std::min<long long>(n_ctas, (long long)F.V * P.parts));
@@ -2007,7 +2007,7 @@ cudaError_t launch_slots_batch(const SweepItem* items, int n, bool blur, bool sh
     if (smem <= 0 || smem > 227 * 1024) return cudaErrorInvalidConfiguration;
     shape = one_cta_shape(shape, smem);
     const void* k = slots_batch_kernel(shape, blur, shift);
-    cudaError_t e = allow_dynamic_smem(k);
+    cudaError_t e = allow_dynamic_smem(k, smem);
     if (e != cudaSuccess) return e;
     const SweepItem* it = items; int nn = n; int* er = err;
     void* args[] = { &it, &nn, &er };

@@ -1016,7 +1016,7 @@ size_t sweep_warp_scratch_bytes(const PmParams& P, int n_ctas)
 // L1 and texture cache.
 static cudaError_t set_smem(const void* k, int smem, bool tex)
 {
-    cudaError_t e = allow_dynamic_smem(k);
+    cudaError_t e = allow_dynamic_smem(k, smem);
     if (e != cudaSuccess || !tex) return e;
     const long need = (long)kMinCtas * (smem + 1024);
     const int pct = (int)std::min<long>(100, (need * 100 + 228 * 1024 - 1) / (228 * 1024) + 1);
