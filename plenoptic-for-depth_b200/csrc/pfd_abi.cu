@@ -2200,58 +2200,52 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
     const size_t ppv = (size_t)f->mi_w * f->mi_h, px = (size_t)V * ppv, npix = (size_t)f->W * f->H;
     const size_t nb = (px + pfd::kFuseScanBlock - 1) / pfd::kFuseScanBlock;
     cudaStream_t s = ctx->stream;
-    // scratch of this call, from the stream-ordered pool
-    struct Scratch {
-        cudaStream_t s;
-        std::vector<void*> ptrs;
-        ~Scratch() { for (void* q : ptrs) cudaFreeAsync(q, s); }
-        cudaError_t get(void** q, size_t bytes) {
-            cudaError_t e = cudaMallocAsync(q, bytes > 0 ? bytes : 1, s);
-            if (e == cudaSuccess) ptrs.push_back(*q);
-            return e;
-        }
-    } S{ s, {} };
-    int *d_lists = nullptr, *d_counts = nullptr;
-    uint8_t *d_bgr = nullptr, *d_ref = nullptr, *d_work = nullptr, *d_conf = nullptr, *d_aif = nullptr;
-    unsigned int *d_winner = nullptr, *d_has = nullptr, *d_bcount = nullptr;
-    float *d_rec = nullptr, *d_vd = nullptr, *d_points = nullptr;
-    CU(S.get((void**)&d_lists, sizeof(int) * (size_t)V * max_list));
-    CU(S.get((void**)&d_counts, sizeof(int) * (size_t)V));
-    CU(S.get((void**)&d_ref, (size_t)V));
-    if (bgr) CU(S.get((void**)&d_bgr, px * 3));
-    CU(S.get((void**)&d_winner, sizeof(unsigned int) * npix));
-    CU(S.get((void**)&d_has, sizeof(unsigned int) * px));
-    CU(S.get((void**)&d_rec, sizeof(float) * 10 * px));
-    CU(S.get((void**)&d_vd, sizeof(float) * npix));
-    CU(S.get((void**)&d_conf, npix));
-    CU(S.get((void**)&d_aif, npix * 3));
+    // scratch of this call, from the stream-ordered pool, in one allocation: a dozen of them
+    // cost up to 0.4 ms of the call where other work has left the pool in pieces
+    size_t size = 0;
+    auto place = [&](size_t bytes) { const size_t at = size; size += (bytes + 255) & ~(size_t)255; return at; };
+    const size_t o_lists = place(sizeof(int) * (size_t)V * max_list), o_counts = place(sizeof(int) * (size_t)V);
+    const size_t o_ref = place((size_t)V), o_bgr = place(bgr ? px * 3 : 0), o_winner = place(sizeof(unsigned int) * npix);
+    const size_t o_has = place(sizeof(unsigned int) * px), o_rec = place(sizeof(float) * 10 * px);
+    const size_t o_vd = place(sizeof(float) * npix), o_conf = place(npix), o_aif = place(npix * 3);
+    const size_t o_bcount = place(sizeof(unsigned int) * nb), o_work = size;
+    pfd::FuseFrame F;
+    F.V = V; F.m = f->mi_w; F.ppv = (int)ppv; F.tile_stride = f->tile_stride;
+    F.max_list = max_list;
+    // The walk's work area takes up to 256 MB, or as much as the point records (40 bytes per
+    // pixel); in a context with a budget, what the budget has left (4 MB at least); and less
+    // where the device has less.  A band costs the latency of its own walk: a 1536x1159 frame
+    // of 128 list entries takes 52 ms in one band of 277 MB, 69 ms in two, 131 ms in eight.
+    size_t limit = std::max<size_t>((size_t)256 << 20, sizeof(float) * 10 * px);
+    if (ctx->budget) limit = std::min(limit, std::max<size_t>((size_t)4 << 20, ctx->budget - std::min(ctx->budget, ctx->used)));
+    pfd::FuseWork X;
+    int band = pfd::fuse_band(F, limit);
+    std::unique_ptr<AsyncBuf> buf;
+    for (cudaError_t e;; band = (band + 1) / 2) {
+        buf.reset(new AsyncBuf(s, o_work + pfd::fuse_work(F, band, nullptr, X), e));
+        if (e == cudaSuccess) break;
+        cudaGetLastError();
+        if (band == 1) return fail(ctx, PFD_ECUDA, "fuse: scratch: %s", cudaGetErrorString(e));
+    }
+    unsigned char* d = (unsigned char*)buf->p;
+    int *d_lists = (int*)(d + o_lists), *d_counts = (int*)(d + o_counts);
+    uint8_t *d_bgr = bgr ? d + o_bgr : nullptr, *d_ref = d + o_ref, *d_conf = d + o_conf, *d_aif = d + o_aif;
+    unsigned int *d_winner = (unsigned int*)(d + o_winner), *d_has = (unsigned int*)(d + o_has);
+    unsigned int* d_bcount = (unsigned int*)(d + o_bcount);
+    float *d_rec = (float*)(d + o_rec), *d_vd = (float*)(d + o_vd);
     CU(cudaMemcpyAsync(d_lists, lists, sizeof(int) * (size_t)V * max_list, cudaMemcpyHostToDevice, s));
     CU(cudaMemcpyAsync(d_counts, list_counts, sizeof(int) * (size_t)V, cudaMemcpyHostToDevice, s));
     CU(cudaMemcpyAsync(d_ref, is_ref, (size_t)V, cudaMemcpyHostToDevice, s));
     if (bgr) CU(cudaMemcpyAsync(d_bgr, bgr, px * 3, cudaMemcpyHostToDevice, s));
     CU(cudaMemsetAsync(d_winner, 0, sizeof(unsigned int) * npix, s));
     CU(cudaMemsetAsync(d_has, 0, sizeof(unsigned int) * px, s));
-    pfd::FuseFrame F;
-    F.V = V; F.m = f->mi_w; F.ppv = (int)ppv; F.tile_stride = f->tile_stride;
     F.gray = f->d_gray; F.bgr = d_bgr; F.centers = f->d_centers; F.plane = f->s[f->cur].plane;
-    F.lists = d_lists; F.list_counts = d_counts; F.max_list = max_list;
+    F.lists = d_lists; F.list_counts = d_counts;
     F.mla_base = p->mla_base; F.min_ref_disp = p->min_ref_disp; F.max_reproj_px = p->max_reproj_px;
     F.max_rel_vd = p->max_rel_vd; F.min_consistent = p->min_consistent;
     F.raw_w = f->W; F.raw_h = f->H;
     F.winner = d_winner; F.rec = d_rec; F.has_rec = d_has;
-    // The walk's work area takes up to 256 MB, or as much as the point records (40 bytes per
-    // pixel); in a context with a budget, what the budget has left (4 MB at least); and less
-    // where the device has less.  A band costs the latency of its own walk: a 1536x1159 frame
-    // of 128 list entries takes 51 ms in one band of 277 MB, 131 ms in eight.
-    size_t limit = std::max<size_t>((size_t)256 << 20, sizeof(float) * 10 * px);
-    if (ctx->budget) limit = std::min(limit, std::max<size_t>((size_t)4 << 20, ctx->budget - std::min(ctx->budget, ctx->used)));
-    pfd::FuseWork X;
-    int band = pfd::fuse_band(F, limit);
-    for (cudaError_t e; (e = S.get((void**)&d_work, pfd::fuse_work(F, band, nullptr, X))) != cudaSuccess; band = (band + 1) / 2) {
-        cudaGetLastError();
-        if (band == 1) return fail(ctx, PFD_ECUDA, "fuse: work area: %s", cudaGetErrorString(e));
-    }
-    pfd::fuse_work(F, band, d_work, X);
+    pfd::fuse_work(F, band, d + o_work, X);
     X.is_ref = d_ref;
     CU(pfd::launch_fuse(F, X, band, ctx->d_err, s, &ctx->launches));
     CU(pfd::launch_fuse_maps(F, d_vd, d_conf, d_aif, s));
@@ -2260,7 +2254,6 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
     if (conf) CU(cudaMemcpyAsync(conf, d_conf, npix, cudaMemcpyDeviceToHost, s));
     if (aif) CU(cudaMemcpyAsync(aif, d_aif, npix * 3, cudaMemcpyDeviceToHost, s));
     if (points || n_points) {
-        CU(S.get((void**)&d_bcount, sizeof(unsigned int) * nb));
         CU(pfd::launch_fuse_count(F, d_bcount, s));
         ctx->launches += 1;
         std::vector<unsigned int> bc(nb);
@@ -2271,7 +2264,10 @@ pfd_status pfd_fuse_virtual_depth(pfd_ctx* ctx, int frame_id, const pfd_fuse_par
         if (n_points) *n_points = (long long)total;
         if (points && total) {
             CU(cudaMemcpyAsync(d_bcount, bc.data(), sizeof(unsigned int) * nb, cudaMemcpyHostToDevice, s));
-            CU(S.get((void**)&d_points, sizeof(float) * 9 * total));
+            cudaError_t e;
+            AsyncBuf pts(s, sizeof(float) * 9 * total, e);
+            CU(e);
+            float* d_points = (float*)pts.p;
             CU(pfd::launch_fuse_compact(F, d_bcount, d_points, s));
             ctx->launches += 1;
             CU(cudaMemcpyAsync(points, d_points, sizeof(float) * 9 * total, cudaMemcpyDeviceToHost, s));
