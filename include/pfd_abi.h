@@ -79,8 +79,10 @@ const char* pfd_last_error(pfd_ctx* ctx);
 void* pfd_stream(pfd_ctx* ctx);
 /* Waits for the context's stream; reports any device-side error flag. */
 pfd_status pfd_sync(pfd_ctx* ctx);
-/* Device memory currently held by the context: its frames and the sweep's
- * cudaMalloc'd cost-vector scratch. */
+/* Device memory currently held by the context: its frames, and the cost-vector
+ * scratch of half-sweeps that count taps, fetch from textures or have a blurred
+ * window without room for the default kernel's slots.  Scratch that a call frees
+ * before it returns (fusion, neighbour selection, depth conversions) is not counted. */
 size_t pfd_bytes_in_use(pfd_ctx* ctx);
 
 /* ---- frames ---------------------------------------------------------------

@@ -177,7 +177,7 @@ struct pfd_ctx {
     int ncc_moments = PFD_NCC_REFERENCE;    // accumulation of the NCC moments (pfd_set_ncc_moments)
     int matcher = PFD_MATCHER_FRAME;        // PatchMatch rules (pfd_set_matcher)
     unsigned long long launches = 0;        // kernels this context has launched
-    float* d_scratch = nullptr;             // sweep candidate costs, per resident CTA
+    float* d_scratch = nullptr;             // candidate costs of the warp-per-pixel sweep, per resident CTA
     size_t scratch_bytes = 0;
     int sweep_shape = 0;                    // launch shape of the half-sweeps, or PFD_SHAPE_AUTOTUNE
     int sweep_fetch = PFD_FETCH_SHARED;     // where the half-sweeps read neighbour samples
@@ -2701,17 +2701,18 @@ pfd_status pfd_download(pfd_ctx* ctx, int frame_id, float* plane, float* cost, f
 
 // ---- PatchMatch sweep without allocation --------------------------------------
 //
-// pfd_pm_sweep takes its candidate-cost scratch from cudaMalloc, grown on the
-// first sweep of a larger grid.  Some callers cannot allocate device memory
-// once frames are streaming: an application whose memory pool claimed all free
-// HBM at start-up (a cudaMalloc then fails, or takes memory the pool counts
-// on), or a real-time camera loop that forbids cudaMalloc/cudaFree because they
-// can synchronise the whole device and stall its other streams.
-// pfd_pm_sweep_noalloc runs the same kernel on a fixed array that is part of
-// the library's device image instead.
+// The slot kernel needs no scratch.  The warp-per-pixel kernel (tap counting, texture
+// fetches, blurred windows without a slot plan) does, and pfd_pm_sweep allocates it on
+// the context's stream, grown on the first sweep of a larger grid.  Some callers cannot
+// allocate device memory once frames are streaming: an application whose memory pool
+// claimed all free HBM at start-up (an allocation then fails, or takes memory the pool
+// counts on), or a real-time camera loop that forbids cudaMalloc/cudaFree because they
+// can synchronise the whole device and stall its other streams.  pfd_pm_sweep_noalloc
+// runs the same kernels, the second on a fixed array that is part of the library's
+// device image.
 
 // 8 MiB, held by every GPU that loads the library until the process exits.
-// Each warp of the sweep keeps the cost vectors of its current pixel here,
+// Each warp of that kernel keeps the cost vectors of its current pixel here,
 // (1.5 h max_nb + 3 h) words rounded up to 32 with h = max_nb + 6, seven warps
 // per CTA; the array must hold at least one CTA per SM, which it does for every
 // max_nb up to 32 on a 148-SM B200 (54.7 KB per CTA at 32 neighbours).  Nothing

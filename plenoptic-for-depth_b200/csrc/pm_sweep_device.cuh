@@ -1,6 +1,8 @@
-// pm_sweep_device.cuh -- device helpers shared by the half-sweep kernels
-// (pm_slots.cu, pm_sweep.cu): bulk-copy staging, the texture unit's integer
-// blend, patch windows, cross-view proposals and refinement candidates.
+// pm_sweep_device.cuh -- device helpers of the half-sweep kernels.  Shared by
+// pm_slots.cu and pm_sweep.cu: bulk-copy staging and patch windows.  Of the
+// warp-per-pixel kernel (pm_sweep.cu) only: the texture unit's blend from quads,
+// cross-view proposals and refinement candidates, whole ones per thread (pm_slots.cu
+// spreads its own over a half warp's lanes).
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
