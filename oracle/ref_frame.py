@@ -46,8 +46,9 @@ def available() -> bool:
 
 def build(reference_tree: str = "/root/reference") -> bool:
     """make -C oracle/ref when the reference tree is present (this container);
-    elsewhere the prebuilt libraries are used.  Returns whether all exist."""
-    if os.path.isdir(reference_tree):
+    elsewhere, and where its folder is empty, the prebuilt libraries are used.
+    Returns whether all exist."""
+    if os.path.isfile(os.path.join(reference_tree, "MIStereo", "CudaUtil.cu")):
         r = subprocess.run(["make", "-s", "-C", os.path.join(ORACLE_DIR, "ref"), "REF=" + reference_tree],
                            capture_output=True, text=True)
         if r.returncode != 0:
